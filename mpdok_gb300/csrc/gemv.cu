@@ -184,6 +184,76 @@ gemv_finalize(const ACC* __restrict__ P, int S, int K, long long m, ACC alpha, A
   }
 }
 
+// FP64 y = alpha A x + beta bsrc of a small matrix in one launch, with the sum
+// of squares of y.  The products and their sums carry their rounding errors
+// along (two-product by FMA, two-sum), so y is the rounded exact result: the
+// residual of a refinement subtracts nearly equal vectors, and its own rounding
+// otherwise sets the residual that can be reached (n = 400, kappa 1e5: the
+// computed residual of the rounded solution is 1.7e-13 of ||b||, the true one
+// 0.7e-13).  Ten FP64 operations per entry instead of one, but a single launch
+// with every entry's load in flight at once.  Eight rows per block; 32 threads
+// per row take every 32nd column.
+constexpr long long GEMV_SMALL = 1LL << 19;  // entries: above, the FP64 pipe makes it slower than the two-pass form
+
+struct DD {
+  double s, c;
+};
+__device__ __forceinline__ DD dd_add(DD a, DD b) {
+  const double t = a.s + b.s, bb = t - a.s;
+  return {t, ((a.s - (t - bb)) + (b.s - bb)) + (a.c + b.c)};
+}
+
+__global__ void __launch_bounds__(GEMV_THREADS)
+gemv_n_small_f64(const double* __restrict__ A, long long lda, int m, int n, const double* __restrict__ x, double alpha,
+                 double beta, const double* bsrc, double* y, double* nrm_parts, unsigned* ticket, double* nrm2,
+                 const int* skip) {
+  __shared__ DD sp[8][8];
+  __shared__ double red[32];
+  if (skip != nullptr && *skip) return;
+  const int rl = threadIdx.x & 7, g = threadIdx.x >> 3, warp = threadIdx.x >> 5;
+  const int row = blockIdx.x * 8 + rl;
+  DD a = {0.0, 0.0};
+  if (row < m) {
+#pragma unroll 4
+    for (int j = g; j < n; j += GEMV_THREADS / 8) {
+      const double av = __ldg(A + row + (long long)j * lda), xv = __ldg(x + j);
+      const double p = av * xv;
+      a = dd_add(a, {p, fma(av, xv, -p)});
+    }
+  }
+  auto across = [&](DD v) {  // over the lanes of one row: 8 and 16 apart
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1)
+      v = dd_add(v, {__shfl_xor_sync(0xffffffffu, v.s, o), __shfl_xor_sync(0xffffffffu, v.c, o)});
+    return v;
+  };
+  a = across(a);
+  if ((threadIdx.x & 31) < 8) sp[warp][rl] = a;
+  __syncthreads();
+  double sq = 0.0;
+  if (warp == 0) {
+    a = across(dd_add(sp[g][rl], sp[g + 4][rl]));
+    if (g == 0 && row < m) {
+      const double b = beta != 0.0 ? bsrc[row] : 0.0;
+      const double p = alpha * a.s, q = beta * b;
+      const DD r = dd_add({q, fma(beta, b, -q)}, {p, fma(alpha, a.s, -p) + alpha * a.c});
+      double v = r.s + r.c;
+      if (!isfinite(v)) {  // infinities do not survive the error terms: the plain sum
+        double t = 0.0;
+        for (int j = 0; j < n; ++j) t = fma(A[row + (long long)j * lda], x[j], t);
+        v = alpha * t;
+        if (beta != 0.0) v = fma(beta, b, v);
+      }
+      y[row] = v;
+      sq = v * v;
+    }
+  }
+  if (nrm2 != nullptr) {
+    const double b = block_sum(sq, red);
+    ordered_grid_sum(b, nrm_parts, ticket, nrm2);
+  }
+}
+
 static unsigned finalize_blocks(long long total) {
   long long b = (total + GEMV_THREADS - 1) / GEMV_THREADS;
   long long cap = (long long)num_sms() * 4;
@@ -282,6 +352,17 @@ int gemv_launch(int a_dtype, bool trans, const void* A, long long lda, long long
     const char* Xk = (const char*)X + (size_t)done * ldx * acc_bytes;
     char* Yk = (char*)Y + (size_t)done * ldy * acc_bytes;
     const char* Bk = Bsrc ? (const char*)Bsrc + (size_t)done * ldb * acc_bytes : nullptr;
+    if (a_dtype == MPDOK_F64 && !trans && K == 1 && red > 0 && m * n <= GEMV_SMALL) {
+      if (nrm2 && zero_ticket) MPDOK_CUDA_TRY(cudaMemsetAsync(ticket, 0, sizeof(unsigned), s));
+      const int pslot = prof_start(MPDOK_PROF_GEMV_F64, s);
+      // (the blocks' norm parts, m / 8 of them, fit the partial-sum buffer of m doubles per split)
+      launch(gemv_n_small_f64, (unsigned)((m + 7) / 8), GEMV_THREADS, 0, s, (const double*)A, lda, (int)m, (int)n,
+             (const double*)Xk, alpha, beta, (const double*)Bk, (double*)Yk, (double*)P, ticket, nrm2, skip);
+      prof_stop(pslot, s, (double)m * (double)n * eb + (double)(m + n) * acc_bytes, skip);
+      MPDOK_LAUNCH_CHECK("gemv small");
+      done += K;
+      continue;
+    }
     if (red == 0) {
       // Empty reduction: y = beta * bsrc.  Use one zero split.
       MPDOK_CUDA_TRY(cudaMemsetAsync(P, 0, (size_t)K * out * acc_bytes, s));
