@@ -34,6 +34,7 @@
 //  * The adjoint contraction recomputes phi and its derivatives from the
 //    coordinates (nothing of size N^2 is stored for the gradient).
 #include "krylov.cuh"
+#include "phi64.cuh"
 
 #include <cmath>
 #include <cstring>
@@ -55,6 +56,7 @@ struct BSys {
   long long offR;   // per-row scratch (n doubles)
   int n, nblk, user, pad;
   double eps, gamma, reg;
+  GaussScale gs;    // of gamma
 };
 
 struct BatchPlan {
@@ -135,63 +137,58 @@ __device__ __forceinline__ DF df_sub(DF a, float bh, float bl) {
   return r;
 }
 
-// phi(r2) and its partial derivatives: g = dphi/d(r2), h = dphi/dgamma.
 template <int KIND>
-__device__ __forceinline__ void phi_derivs(double r2, double gamma, double& phi, double& g, double& h) {
-  if (KIND == MPDOK_KERNEL_GAUSSIAN) {
-    phi = exp(-gamma * r2);
-    g = -gamma * phi;
-    h = -r2 * phi;
-  } else {
-    phi = sqrt(fma(gamma, r2, 1.0));
-    const double ip = 0.5 / phi;
-    g = gamma * ip;
-    h = r2 * ip;
-  }
-}
-
-template <int KIND>
-__device__ __forceinline__ double phi_only(double r2, double gamma) {
-  return KIND == MPDOK_KERNEL_GAUSSIAN ? exp(-gamma * r2) : sqrt(fma(gamma, r2, 1.0));
+__device__ __forceinline__ double phi_only(double r2, const BSys& q, const uint64_t* T) {
+  return KIND == MPDOK_KERNEL_GAUSSIAN ? gauss_phi(r2, q.gs, T) : sqrt(fma(q.gamma, r2, 1.0));
 }
 
 // ------------------------------------------------------------------ assembly
-// One task per (system, 64x64 tile) of the full matrix (both triangles).
+// One task per (system, 64x64 tile on or below the diagonal): the tile as
+// double-float pairs and, through shared memory, its mirror image in FP64 (the
+// two triangles hold the same values, phi being even in x_i - x_j).
 template <int KIND, int D>
 __global__ void __launch_bounds__(BT) k_bassemble(const BSys* __restrict__ sys, const long long* __restrict__ pre,
                                                   int nsys, const double* __restrict__ coords,
                                                   double* __restrict__ A) {
-  __shared__ double sR[BNB * D], sC[BNB * D];
+  __shared__ uint64_t sPhi[KIND == MPDOK_KERNEL_GAUSSIAN ? PHI_TAB : 1];
+  extern __shared__ double sM[];  // [column][row] of the tile, BNB x BPAD
+  if constexpr (KIND == MPDOK_KERNEL_GAUSSIAN) phi_table(sPhi);
   const long long t = blockIdx.x;
   const int s = task_system(pre, nsys + 1, t);
   const BSys q = sys[s];
   const long long u = t - pre[s];
-  const int ti = (int)(u % q.nblk), tj = (int)(u / q.nblk);
+  int ti = (int)((sqrtf(8.f * (float)u + 1.f) - 1.f) * 0.5f);
+  while ((long long)(ti + 1) * (ti + 2) / 2 <= u) ++ti;
+  while ((long long)ti * (ti + 1) / 2 > u) --ti;
+  const int tj = (int)(u - (long long)ti * (ti + 1) / 2);
   const int r0 = ti * BNB, c0 = tj * BNB;
+  const int nr = min(BNB, q.n - r0), nc = min(BNB, q.n - c0);
   const double* X = coords + q.offC;
-  for (int e = threadIdx.x; e < BNB * D; e += BT) {
-    const int i = e / D, d = e % D;
-    sR[e] = (r0 + i < q.n) ? X[(long long)(r0 + i) * D + d] : 0.0;
-    sC[e] = (c0 + i < q.n) ? X[(long long)(c0 + i) * D + d] : 0.0;
-  }
-  __syncthreads();
   double* Ab = A + q.offA;
+  const long long lda = q.n;
   const int row = threadIdx.x & 63;
-  for (int col = threadIdx.x >> 6; col < BNB; col += BT / BNB) {
-    const int i = r0 + row, j = c0 + col;
-    if (i >= q.n || j >= q.n) continue;
+  double x[D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) x[d] = row < nr ? X[(long long)(r0 + row) * D + d] : 0.0;
+  __syncthreads();
+#pragma unroll 2
+  for (int col = threadIdx.x >> 6; col < nc; col += BT / BNB) {
     double r2 = 0.0;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      const double df = sR[row * D + d] - sC[col * D + d];
+      const double df = x[d] - __ldg(X + (long long)(c0 + col) * D + d);
       r2 = fma(df, df, r2);
     }
-    double v = phi_only<KIND>(r2, q.gamma);
+    double v = phi_only<KIND>(r2, q, sPhi);
+    const int i = r0 + row, j = c0 + col;
     if (i == j) v += q.reg;
-    double* slot = Ab + (long long)i + (long long)j * q.n;
-    if (i >= j) st_df(slot, to_df(v));
-    else *slot = v;
+    if (row < nr && i >= j) st_df(Ab + i + (long long)j * lda, to_df(v));
+    sM[col * BPAD + row] = v;
   }
+  __syncthreads();
+  // strict upper triangle: entry (c0 + row, r0 + c) mirrors (r0 + c, c0 + row)
+  for (int c = threadIdx.x >> 6; c < nr; c += BT / BNB)
+    if (row < nc && c0 + row < r0 + c) Ab[(c0 + row) + (long long)(r0 + c) * lda] = sM[row * BPAD + c];
 }
 
 // ------------------------------------------------------------------ level k: diagonal block
@@ -611,20 +608,31 @@ __global__ void k_badd(double* __restrict__ X, const double* __restrict__ D, lon
 }
 
 // ------------------------------------------------------------------ adjoint contraction
-// For L(X) with Lam = A^{-T} dL/dX (A symmetric), per row k of each system:
-//   dL/dc_k = -sum_j w_kj * 2 (c_k - c_j) * g_kj,   w_kj = sum_r (lam_kr x_jr + x_kr lam_jr)
-//   dL/deps partial_k = -2 eps sum_j u_kj * h_kj,   u_kj = sum_r lam_kr x_jr
+// For L(X) with Lam = A^{-T} dL/dX (A symmetric), per row k of each system, with
+// w_kj = sum_r (lam_kr x_jr + x_kr lam_jr), symmetric in k and j:
+//   dL/dc_k = -2 sum_j w_kj g_kj (c_k - c_j)
+//   dL/deps = -2 eps sum_kj u_kj h_kj,  u_kj = sum_r lam_kr x_jr;  h is symmetric
+//             too, so this is sum_k of the partials -eps sum_j w_kj h_kj
 //   dL/dreg partial_k = -sum_r lam_kr x_kr
-// with g = dphi/d(r^2), h = dphi/dgamma, gamma = eps^2, phi recomputed in FP64.
-// Four threads per row split the columns; their partial sums combine by
-// shuffles in a fixed order.
-template <int KIND, int D>
+// with g = dphi/d(r^2), h = dphi/dgamma, gamma = eps^2, phi recomputed in FP64:
+//   Gaussian      g = -gamma phi,        h = -r^2 phi
+//   multiquadric  g = gamma / (2 phi),   h = r^2 / (2 phi)
+// so both are one factor p (phi or 1 / phi) times constants applied once per
+// row.  Bound by the FP64 pipe: 2 D + 2 NR + D + 2 operations per entry besides
+// p; the Gaussian p runs on the integer pipe (phi64.cuh).  NR, the number of
+// right-hand sides rounded up to a power of two, is compiled in: eight columns
+// for a single one were 28 of 46 operations (n = 6000, D = 2, one column:
+// 4.60 ms for all eight with CUDA's exp, 0.95 ms now).  Four threads per row split the columns; their
+// partial sums combine by shuffles in a fixed order.
+template <int KIND, int D, int NR>
 __global__ void __launch_bounds__(BT) k_badjoint(const BSys* __restrict__ sys, const long long* __restrict__ pre,
                                                  int nsys, int nrhs, const double* __restrict__ coords,
                                                  const double* __restrict__ X, const double* __restrict__ Lam,
                                                  double* __restrict__ gC, double* __restrict__ rowscr) {
+  __shared__ uint64_t sPhi[KIND == MPDOK_KERNEL_GAUSSIAN ? PHI_TAB : 1];
   __shared__ double sC[BNB * D];
-  __shared__ double sXj[BMAX_RHS * BNB], sLj[BMAX_RHS * BNB];
+  __shared__ double sXj[NR * BNB], sLj[NR * BNB];
+  if constexpr (KIND == MPDOK_KERNEL_GAUSSIAN) phi_table(sPhi);
   const long long t = blockIdx.x;
   const int s = task_system(pre, nsys + 1, t);
   const BSys q = sys[s];
@@ -634,11 +642,11 @@ __global__ void __launch_bounds__(BT) k_badjoint(const BSys* __restrict__ sys, c
   const int k = r0 + lr;
   const bool live = k < q.n;
   const double* Cb = coords + q.offC;
-  double ck[D], xk[BMAX_RHS], lk[BMAX_RHS];
+  double ck[D], xk[NR], lk[NR];
 #pragma unroll
   for (int d = 0; d < D; ++d) ck[d] = live ? Cb[(long long)k * D + d] : 0.0;
 #pragma unroll
-  for (int rr = 0; rr < BMAX_RHS; ++rr) {
+  for (int rr = 0; rr < NR; ++rr) {
     xk[rr] = (live && rr < nrhs) ? X[q.offX + k + (long long)rr * q.n] : 0.0;
     lk[rr] = (live && rr < nrhs) ? Lam[q.offX + k + (long long)rr * q.n] : 0.0;
   }
@@ -649,7 +657,7 @@ __global__ void __launch_bounds__(BT) k_badjoint(const BSys* __restrict__ sys, c
     const int c0 = c * BNB, nc = min(BNB, q.n - c0);
     __syncthreads();
     for (int e = threadIdx.x; e < BNB * D; e += BT) sC[e] = (e / D < nc) ? Cb[(long long)c0 * D + e] : 0.0;
-    for (int e = threadIdx.x; e < BNB * BMAX_RHS; e += BT) {
+    for (int e = threadIdx.x; e < BNB * NR; e += BT) {
       const int j = e % BNB, rr = e / BNB;
       const bool ok = j < nc && rr < nrhs;
       sXj[e] = ok ? X[q.offX + c0 + j + (long long)rr * q.n] : 0.0;
@@ -657,6 +665,7 @@ __global__ void __launch_bounds__(BT) k_badjoint(const BSys* __restrict__ sys, c
     }
     __syncthreads();
     if (!live) continue;
+#pragma unroll 2
     for (int j = part; j < nc; j += 4) {
       double df[D], r2 = 0.0;
 #pragma unroll
@@ -664,18 +673,18 @@ __global__ void __launch_bounds__(BT) k_badjoint(const BSys* __restrict__ sys, c
         df[d] = ck[d] - sC[j * D + d];
         r2 = fma(df[d], df[d], r2);
       }
-      double phi, g, h;
-      phi_derivs<KIND>(r2, q.gamma, phi, g, h);
-      double u = 0.0, v = 0.0;
+      const double p = KIND == MPDOK_KERNEL_GAUSSIAN ? gauss_phi(r2, q.gs, sPhi)
+                                                     : 1.0 / sqrt(fma(q.gamma, r2, 1.0));
+      double w = 0.0;
 #pragma unroll
-      for (int rr = 0; rr < BMAX_RHS; ++rr) {
-        u = fma(lk[rr], sXj[rr * BNB + j], u);
-        v = fma(xk[rr], sLj[rr * BNB + j], v);
+      for (int rr = 0; rr < NR; ++rr) {
+        w = fma(lk[rr], sXj[rr * BNB + j], w);
+        w = fma(xk[rr], sLj[rr * BNB + j], w);
       }
-      const double wg = -2.0 * (u + v) * g;
+      w *= p;
 #pragma unroll
-      for (int d = 0; d < D; ++d) G[d] = fma(wg, df[d], G[d]);
-      E = fma(-u, h, E);
+      for (int d = 0; d < D; ++d) G[d] = fma(w, df[d], G[d]);
+      E = fma(w, r2, E);
     }
   }
   // combine the four column parts (lanes 4m .. 4m+3) in a fixed order
@@ -686,14 +695,25 @@ __global__ void __launch_bounds__(BT) k_badjoint(const BSys* __restrict__ sys, c
     E += __shfl_xor_sync(0xffffffffu, E, o);
   }
   if (live && part == 0) {
+    const double cg = KIND == MPDOK_KERNEL_GAUSSIAN ? 2.0 * q.gamma : -q.gamma;
+    const double ch = KIND == MPDOK_KERNEL_GAUSSIAN ? q.eps : -0.5 * q.eps;
 #pragma unroll
-    for (int d = 0; d < D; ++d) gC[q.offC + (long long)k * D + d] = G[d];
+    for (int d = 0; d < D; ++d) gC[q.offC + (long long)k * D + d] = cg * G[d];
     double lx = 0.0;
 #pragma unroll
-    for (int rr = 0; rr < BMAX_RHS; ++rr) lx = fma(lk[rr], xk[rr], lx);
-    rowscr[q.offR + 2LL * k] = 2.0 * q.eps * E;
+    for (int rr = 0; rr < NR; ++rr) lx = fma(lk[rr], xk[rr], lx);
+    rowscr[q.offR + 2LL * k] = ch * E;
     rowscr[q.offR + 2LL * k + 1] = -lx;
   }
+}
+
+template <int KIND, int D>
+static void launch_badjoint(unsigned grid, const BSys* sys, const long long* pre, int nsys, int nrhs,
+                            const double* coords, const double* X, const double* Lam, double* gC, double* rowscr,
+                            cudaStream_t s) {
+  auto* kern = nrhs == 1 ? k_badjoint<KIND, D, 1> : nrhs == 2 ? k_badjoint<KIND, D, 2>
+               : nrhs <= 4 ? k_badjoint<KIND, D, 4> : k_badjoint<KIND, D, BMAX_RHS>;
+  launch(kern, dim3(grid), BT, 0, s, sys, pre, nsys, nrhs, coords, X, Lam, gC, rowscr);
 }
 
 // Per system: grad_eps = sum_k partial, grad_reg = sum_k partial (fixed order).
@@ -931,6 +951,8 @@ __global__ void __launch_bounds__(BT) k_bstep_dag(const BSys* __restrict__ sys, 
         tj = (int)(u / nblk);
         double* sR = smem;
         double* sC = smem + BNB * D;
+        uint64_t* sPhi = reinterpret_cast<uint64_t*>(smem + 2 * BNB * D);
+        if constexpr (KIND == MPDOK_KERNEL_GAUSSIAN) phi_table(sPhi);
         const int r0 = ti * BNB, c0 = tj * BNB;
         const double* Xc = coords + q.offC;
         for (int e = tid; e < BNB * D; e += BT) {
@@ -949,7 +971,7 @@ __global__ void __launch_bounds__(BT) k_bstep_dag(const BSys* __restrict__ sys, 
             const double df = sR[row * D + d] - sC[col * D + d];
             r2 = fma(df, df, r2);
           }
-          double v = phi_only<KIND>(r2, q.gamma);
+          double v = phi_only<KIND>(r2, q, sPhi);
           if (i == j) v += q.reg;
           double* slot = Ab + (long long)i + (long long)j * q.n;
           if (i >= j) st_df(slot, to_df(v));
@@ -1288,10 +1310,11 @@ static int batch_factor(BatchPlan* p, cudaStream_t s) {
   // assembly: one task per (system, tile); its prefix follows the row prefix
   const long long* preA = p->d_pre + p->d_preRow_base + (p->nsys + 1);
   long long totalA = 0;
-  for (auto& q : p->sys) totalA += (long long)q.nblk * q.nblk;
+  for (auto& q : p->sys) totalA += (long long)q.nblk * (q.nblk + 1) / 2;
+  const size_t asm_smem = (size_t)BNB * BPAD * sizeof(double);
   if (totalA > 0) {
-    BKIND_DIM_SWITCH(p->kernel, p->dim,
-                     launch(k_bassemble<KK_, DD_>, dim3((unsigned)totalA), BT, 0, s, (const BSys*)p->d_sys, preA,
+    BKIND_DIM_SWITCH(p->kernel, p->dim, MPDOK_TRY(set_smem(k_bassemble<KK_, DD_>, asm_smem));
+                     launch(k_bassemble<KK_, DD_>, dim3((unsigned)totalA), BT, asm_smem, s, (const BSys*)p->d_sys, preA,
                             p->nsys, (const double*)p->coords, p->A));
   }
   const size_t tsm = 2 * (size_t)BNB * BPAD * sizeof(double);
@@ -1638,7 +1661,7 @@ extern "C" int mpdok_batch_create(int nsys, const long long* n, int dim, int nrh
   p->preRow.push_back(0);
   for (int i = 0; i < nsys; ++i) p->preRow.push_back(p->preRow.back() + p->sys[i].nblk);
   std::vector<long long> preA(1, 0);
-  for (int i = 0; i < nsys; ++i) preA.push_back(preA.back() + (long long)p->sys[i].nblk * p->sys[i].nblk);
+  for (int i = 0; i < nsys; ++i) preA.push_back(preA.back() + (long long)p->sys[i].nblk * (p->sys[i].nblk + 1) / 2);
   all.insert(all.end(), p->preT.begin(), p->preT.end());
   p->d_preS_base = (long long)all.size();
   all.insert(all.end(), p->preS.begin(), p->preS.end());
@@ -1705,6 +1728,7 @@ extern "C" int mpdok_batch_load(void* plan, const double* coords, const double* 
     q.eps = eps[q.user];
     q.gamma = eps[q.user] * eps[q.user];
     q.reg = reg[q.user];
+    q.gs = gauss_scale(q.gamma);
   }
   MPDOK_CUDA_TRY(cudaMemcpyAsync(p->d_sys, p->sys.data(), p->sys.size() * sizeof(BSys), cudaMemcpyHostToDevice, s));
   MPDOK_CUDA_TRY(cudaMemcpyAsync(p->coords, coords, (size_t)p->total_c * sizeof(double), cudaMemcpyDeviceToDevice,
@@ -1742,9 +1766,8 @@ extern "C" int mpdok_batch_adjoint(void* plan, const double* X, const double* La
   const long long nt = p->preRow.back();
   if (nt > 0) {
     BKIND_DIM_SWITCH(p->kernel, p->dim,
-                     launch(k_badjoint<KK_, DD_>, dim3((unsigned)nt), BT, 0, s, (const BSys*)p->d_sys,
-                            preRow_dev(p), p->nsys, p->nrhs, (const double*)p->coords, X, Lam, grad_coords,
-                            p->rows));
+                     launch_badjoint<KK_, DD_>((unsigned)nt, p->d_sys, preRow_dev(p), p->nsys, p->nrhs, p->coords, X,
+                                               Lam, grad_coords, p->rows, s));
   }
   launch(k_badj_reduce, dim3(p->nsys), BT, 0, s, (const BSys*)p->d_sys, (const double*)p->rows, grad_eps, grad_reg);
   MPDOK_LAUNCH_CHECK("batch adjoint");
@@ -1773,6 +1796,7 @@ extern "C" int mpdok_rbf_adjoint(const double* coords, long long n, int dim, int
   q.nblk = (int)((n + BNB - 1) / BNB);
   q.eps = eps;
   q.gamma = eps * eps;
+  q.gs = gauss_scale(q.gamma);
   char* w = (char*)work;
   BSys* d_sys = (BSys*)w;
   long long* d_pre = (long long*)(w + 256);
@@ -1781,8 +1805,8 @@ extern "C" int mpdok_rbf_adjoint(const double* coords, long long n, int dim, int
   MPDOK_CUDA_TRY(cudaMemcpyAsync(d_sys, &q, sizeof(BSys), cudaMemcpyHostToDevice, s));
   MPDOK_CUDA_TRY(cudaMemcpyAsync(d_pre, pre, sizeof(pre), cudaMemcpyHostToDevice, s));
   BKIND_DIM_SWITCH(kernel, dim,
-                   launch(k_badjoint<KK_, DD_>, dim3((unsigned)q.nblk), BT, 0, s, (const BSys*)d_sys,
-                          (const long long*)d_pre, 1, nrhs, coords, X, Lam, grad_coords, rows));
+                   launch_badjoint<KK_, DD_>((unsigned)q.nblk, d_sys, d_pre, 1, nrhs, coords, X, Lam, grad_coords, rows,
+                                             s));
   launch(k_badj_reduce, dim3(1), BT, 0, s, (const BSys*)d_sys, (const double*)rows, grad_eps, grad_reg);
   MPDOK_LAUNCH_CHECK("rbf adjoint");
   // the host copies above read stack memory: finish them before returning

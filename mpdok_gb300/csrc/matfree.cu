@@ -19,6 +19,7 @@
 // sqrt, for r = b - K x accurate to FP64 rounding.
 #include "krylov.cuh"
 #include "matfree.cuh"
+#include "phi64.cuh"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -174,48 +175,57 @@ k_matfree_f32(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ C
 }
 
 // FP64 evaluate-and-multiply (residual accuracy).  Column centres staged in
-// shared memory by plain loads; one row per thread.
-template <int KIND>
+// shared memory by plain loads; one row per thread.  Bound by the FP64 pipe: 2 D
+// operations for d^2 and K for the products; the exponential runs on the
+// integer pipe (phi64.cuh).  20000 centres x 16384 rows, D = 2, K = 3: 4.3 ms
+// (16.5 ms with CUDA's exp; the 7 FP64 operations per entry alone take 3.6 ms).
+template <int KIND, int D, int K>
 __global__ void __launch_bounds__(MF_THREADS)
-k_matfree_f64(const double* __restrict__ rows, const double* __restrict__ cols, int dim, long long nrows,
-              long long ncols, long long chunk, double gamma, const double* __restrict__ X, long long ldx, int K,
-              double* __restrict__ P) {
-  __shared__ double sc[MF_BC][3];
-  __shared__ double sx[8][MF_BC];
+k_matfree_f64(const double* __restrict__ rows, const double* __restrict__ cols, long long nrows, long long ncols,
+              long long chunk, GaussScale gs, const double* __restrict__ X, long long ldx, double* __restrict__ P) {
+  __shared__ uint64_t sT[KIND == MPDOK_KERNEL_GAUSSIAN ? PHI_TAB : 1];
+  __shared__ double sc[MF_BC][D];
+  __shared__ double sx[K][MF_BC];
+  if constexpr (KIND == MPDOK_KERNEL_GAUSSIAN) phi_table(sT);
   const int tid = threadIdx.x;
   const long long r = (long long)blockIdx.x * MF_THREADS + tid;
   const int sidx = blockIdx.y;
   const long long cb = (long long)sidx * chunk;
   const long long ce = min(ncols, cb + chunk);
-  double rr[3] = {0.0, 0.0, 0.0};
-  if (r < nrows)
-    for (int d = 0; d < dim; ++d) rr[d] = rows[r * dim + d];
-  double acc[8];
+  double rr[D];
 #pragma unroll
-  for (int kk = 0; kk < 8; ++kk) acc[kk] = 0.0;
+  for (int d = 0; d < D; ++d) rr[d] = r < nrows ? rows[r * D + d] : 0.0;
+  double acc[K];
+#pragma unroll
+  for (int kk = 0; kk < K; ++kk) acc[kk] = 0.0;
   for (long long j0 = cb; j0 < ce; j0 += MF_BC) {
     const int nb = (int)min((long long)MF_BC, ce - j0);
     __syncthreads();
-    for (int t = tid; t < MF_BC * 3; t += MF_THREADS) {
-      const int j = t / 3, d = t % 3;
-      sc[j][d] = (j < nb && d < dim) ? cols[(j0 + j) * dim + d] : 0.0;
-    }
+    for (int t = tid; t < nb * D; t += MF_THREADS) sc[t / D][t % D] = cols[j0 * D + t];
     for (int t = tid; t < K * MF_BC; t += MF_THREADS) {
       const int kk = t / MF_BC, j = t % MF_BC;
       sx[kk][j] = (j < nb) ? X[(j0 + j) + kk * ldx] : 0.0;
     }
     __syncthreads();
     if (r < nrows) {
+#pragma unroll 2
       for (int j = 0; j < nb; ++j) {
-        const double dx = rr[0] - sc[j][0], dy = rr[1] - sc[j][1], dz = rr[2] - sc[j][2];
-        const double d2 = fma(dx, dx, fma(dy, dy, dz * dz));
-        const double v = (KIND == MPDOK_KERNEL_GAUSSIAN) ? exp(-gamma * d2) : sqrt(fma(gamma, d2, 1.0));
+        double d2 = 0.0;
+#pragma unroll
+        for (int d = D - 1; d >= 0; --d) {
+          const double df = rr[d] - sc[j][d];
+          d2 = d == D - 1 ? df * df : fma(df, df, d2);
+        }
+        const double v = (KIND == MPDOK_KERNEL_GAUSSIAN) ? gauss_phi(d2, gs, sT) : sqrt(fma(gs.gamma, d2, 1.0));
+#pragma unroll
         for (int kk = 0; kk < K; ++kk) acc[kk] = fma(v, sx[kk][j], acc[kk]);
       }
     }
   }
-  if (r < nrows)
+  if (r < nrows) {
+#pragma unroll
     for (int kk = 0; kk < K; ++kk) P[((long long)sidx * K + kk) * nrows + r] = acc[kk];
+  }
 }
 
 // y = alpha * sum_s P + beta * y + reg * x_shift ; FP32 or FP64; optional
@@ -329,6 +339,25 @@ static void launch_mf32(const CUtensorMap& mc, const CUtensorMap& mx, const floa
   count_launch();
 }
 
+template <int KIND, int D, int K>
+static void launch_mf64_dk(const MfOperand& op, const MfPlan& p, const double* X, long long ldx, double* P,
+                           cudaStream_t s) {
+  launch(k_matfree_f64<KIND, D, K>, dim3(p.gx, p.S), MF_THREADS, 0, s, op.rows, op.cols, op.nrows, op.ncols, p.chunk,
+         gauss_scale(op.gamma), X, ldx, P);
+}
+
+template <int KIND>
+static void launch_mf64(const MfOperand& op, const MfPlan& p, const double* X, long long ldx, int K, double* P,
+                        cudaStream_t s) {
+  using Fn = void (*)(const MfOperand&, const MfPlan&, const double*, long long, double*, cudaStream_t);
+#define MF64_K(D) {launch_mf64_dk<KIND, D, 1>, launch_mf64_dk<KIND, D, 2>, launch_mf64_dk<KIND, D, 3>, \
+                   launch_mf64_dk<KIND, D, 4>, launch_mf64_dk<KIND, D, 5>, launch_mf64_dk<KIND, D, 6>, \
+                   launch_mf64_dk<KIND, D, 7>, launch_mf64_dk<KIND, D, 8>}
+  static const Fn fn[3][8] = {MF64_K(1), MF64_K(2), MF64_K(3)};
+#undef MF64_K
+  fn[op.dim - 1][K - 1](op, p, X, ldx, P, s);
+}
+
 int matfree_apply(const MfOperand& op, int precision, const void* X, long long ldx, int K, void* Y, long long ldy,
                   double alpha, double beta, const void* Bsrc, long long ldb, void* work, size_t work_bytes,
                   cudaStream_t s, const int* skip) {
@@ -351,13 +380,10 @@ int matfree_apply(const MfOperand& op, int precision, const void* X, long long l
   if (nc == 0) {
     MPDOK_CUDA_TRY(cudaMemsetAsync(P, 0, p.part_bytes, s));
   } else if (f64) {
-    dim3 grid(p.gx, p.S);
     if (op.kernel == MPDOK_KERNEL_GAUSSIAN)
-      launch(k_matfree_f64<MPDOK_KERNEL_GAUSSIAN>, grid, MF_THREADS, 0, s, op.rows, op.cols, op.dim, nr, nc,
-             p.chunk, op.gamma, (const double*)X, ldx, K, (double*)P);
+      launch_mf64<MPDOK_KERNEL_GAUSSIAN>(op, p, (const double*)X, ldx, K, (double*)P, s);
     else
-      launch(k_matfree_f64<MPDOK_KERNEL_MQ>, grid, MF_THREADS, 0, s, op.rows, op.cols, op.dim, nr, nc, p.chunk,
-             op.gamma, (const double*)X, ldx, K, (double*)P);
+      launch_mf64<MPDOK_KERNEL_MQ>(op, p, (const double*)X, ldx, K, (double*)P, s);
   } else {
     MPDOK_ARG_CHECK(aligned16(X) && (ldx * 4) % 16 == 0, "FP32 X must be 16-byte aligned with ldx % 4 == 0");
     float4* rp = (float4*)(w + MF_STATUS + p.part_bytes);
