@@ -248,7 +248,8 @@ MPDOK_API int mpdok_chol_cg_ir(void* plan, const double* A64, long long lda, con
  * Blocked right-looking LU with FP32 panels and a trailing update
  * W22 -= L21 U12 whose operands are rounded to the factor type: BF16 / FP16
  * run on tcgen05 tensor cores (FP32 accumulation in tensor memory), FP32 on
- * CUDA cores (the reference's Sgetrf precision, benchmark_mpdok.ipynb:982-993).
+ * them too, as three BF16 planes per operand with FP32 sums (the reference's
+ * Sgetrf precision, benchmark_mpdok.ipynb:982-993).
  *
  * pivoting = 0: W = D A D (D = diag(1/sqrt|a_ii|), symmetric scaling), no row
  *   exchanges (SPD / diagonally dominant systems, e.g. Gaussian RBF); pivots

@@ -622,7 +622,7 @@ __global__ void k_badd(double* __restrict__ X, const double* __restrict__ D, lon
 // p; the Gaussian p runs on the integer pipe (phi64.cuh).  NR, the number of
 // right-hand sides rounded up to a power of two, is compiled in: eight columns
 // for a single one were 28 of 46 operations (n = 6000, D = 2, one column:
-// 4.60 ms for all eight with CUDA's exp, 0.95 ms now).  Four threads per row split the columns; their
+// 4.60 ms for all eight with CUDA's exp, 1.13 ms now).  Four threads per row split the columns; their
 // partial sums combine by shuffles in a fixed order.
 template <int KIND, int D, int NR>
 __global__ void __launch_bounds__(BT) k_badjoint(const BSys* __restrict__ sys, const long long* __restrict__ pre,

@@ -32,16 +32,46 @@
 namespace mpdok {
 
 constexpr int LNB = 128;          // panel width / TRSV block
-// Super-panel width: K of the far trailing update.  For 16-bit factors the
-// tensor-core update is HBM-bound on its FP32 C tile, and K = 1024 halves that
-// read-modify-write against K = 512 (at K = 2048 the longer inner strips cost
-// more than that saves).  The FP32 factors' CUDA-core update is compute-bound,
-// so there the narrower width, with twice the super-panels to overlap, is
-// faster.
-inline long long super_panel_width(int fdtype) { return fdtype == MPDOK_F32 ? 512 : 2048; }
+// Super-panel width: K of the far trailing update.  A wider one reads and writes
+// the FP32 trailing matrix less often per flop, and spends more on the strips
+// inside the super-panel.  16-bit factors: the update is HBM-bound on its FP32
+// C tile up to K = 2048.  FP32 factors form six products per entry, so the
+// update is bound by the tensor cores from K = 1024 on (n = 32768 / 16384 / 8192:
+// 137.7 / 23.6 / 6.9 ms at 512, 122.9 / 21.8 / 6.7 ms at 1024, 121.9 / 22.5 /
+// 6.7 ms at 2048).
+inline long long super_panel_width(int fdtype) { return fdtype == MPDOK_F32 ? 1024 : 2048; }
 constexpr long long SPIN_LIMIT = 1LL << 24;
 
 static int fsize(int fdtype) { return fdtype == MPDOK_F32 ? 4 : 2; }
+
+// What the trailing updates read: 16-bit factors as they are, FP32 factors as
+// three BF16 planes whose sum is the value (tc_gemm.cuh), `plane` elements apart.
+template <typename F>
+struct Operand {
+  using T = F;
+  static constexpr int PLANES = 1;
+};
+template <>
+struct Operand<float> {
+  using T = __nv_bfloat16;
+  static constexpr int PLANES = 3;
+};
+static int operand_bytes(int fdtype) { return fdtype == MPDOK_F32 ? 6 : 2; }
+
+template <typename F>
+__device__ __forceinline__ void put_operand(typename Operand<F>::T* p, long long plane, float v) {
+  if constexpr (Operand<F>::PLANES == 1) {
+    *p = from_f32<F>(v);
+  } else {
+    // each difference is exact: the rounded part shares the leading bits
+    const __nv_bfloat16 h = __float2bfloat16_rn(v);
+    const float r = v - __bfloat162float(h);
+    const __nv_bfloat16 m = __float2bfloat16_rn(r);
+    p[0] = h;
+    p[plane] = m;
+    p[2 * plane] = __float2bfloat16_rn(r - __bfloat162float(m));
+  }
+}
 
 struct LULayout {
   long long n = 0, ldf = 0;
@@ -102,8 +132,8 @@ static LUWork lu_work_layout(long long n, int fdtype) {
   w.off_W = take((size_t)w.ldw * n * sizeof(float));
   // two operand buffers each: super-panel J + 1 is factored while the far
   // update of super-panel J still reads its own operands (look-ahead)
-  w.off_Lp = take(2 * (size_t)std::max(1LL, n) * super_panel_width(fdtype) * fsize(fdtype));
-  w.off_Up = take(2 * (size_t)std::max(1LL, n) * super_panel_width(fdtype) * fsize(fdtype));
+  w.off_Lp = take(2 * (size_t)std::max(1LL, n) * super_panel_width(fdtype) * operand_bytes(fdtype));
+  w.off_Up = take(2 * (size_t)std::max(1LL, n) * super_panel_width(fdtype) * operand_bytes(fdtype));
   w.off_err = take(64);
   // pivoting: candidate (|value|, row) per CTA and the candidate rows, double
   // buffered by column parity; the row at the panel's current position; the
@@ -622,7 +652,8 @@ k_tri_inv_complete(const float* __restrict__ W, long long ldw, long long n, floa
 template <typename F, int RB>
 __device__ __forceinline__ void trsm_right_body(const float* __restrict__ W, long long ldw, long long j0,
                                                 long long r_begin, long long n, const float* __restrict__ Uinv,
-                                                F* __restrict__ Lp, long long lp_pitch, long long lp_row0, int koff,
+                                                typename Operand<F>::T* __restrict__ Lp, long long plane,
+                                                long long lp_pitch, long long lp_row0, int koff,
                                                 F* __restrict__ LU, long long ldf, int bid) {
   static_assert(RB % 16 == 0 && RB <= 64, "rows per block: a multiple of 16, at most 64");
   constexpr int RU = RB / 8;      // rows per thread
@@ -697,7 +728,7 @@ __device__ __forceinline__ void trsm_right_body(const float* __restrict__ W, lon
   // K-major operand for the trailing GEMM: Lp[row][k]
   for (int idx = tid; idx < RB * LNB; idx += TRSM_THREADS) {
     const int r = idx / LNB, c = idx % LNB;
-    if (r < rows) Lp[(r0 - lp_row0 + r) * lp_pitch + koff + c] = from_f32<F>(Xs[r * XP + c]);
+    if (r < rows) put_operand<F>(Lp + (r0 - lp_row0 + r) * lp_pitch + koff + c, plane, Xs[r * XP + c]);
   }
   // column-major factor
   for (int idx = tid; idx < RB * LNB; idx += TRSM_THREADS) {
@@ -711,7 +742,8 @@ __device__ __forceinline__ void trsm_right_body(const float* __restrict__ W, lon
 template <typename F, int RB>
 __device__ __forceinline__ void trsm_left_body(const float* __restrict__ W, long long ldw, long long j0,
                                                long long c_begin, long long n, const float* __restrict__ Linv,
-                                               F* __restrict__ Up, long long up_pitch, long long up_col0, int koff,
+                                               typename Operand<F>::T* __restrict__ Up, long long plane,
+                                               long long up_pitch, long long up_col0, int koff,
                                                F* __restrict__ LU, long long ldf, int bid) {
   static_assert(RB % 16 == 0 && RB <= 64, "columns per block: a multiple of 16, at most 64");
   constexpr int RS = TRSM_THREADS / RB;  // row stride between a thread's rows
@@ -786,9 +818,9 @@ __device__ __forceinline__ void trsm_left_body(const float* __restrict__ W, long
   for (int idx = tid; idx < LNB * RB; idx += TRSM_THREADS) {
     const int r = idx % LNB, c = idx / LNB;
     if (c < cols) {
-      const F v = from_f32<F>(Xs[r * XP + c]);
-      Up[(c0 - up_col0 + c) * up_pitch + koff + r] = v;
-      LU[(j0 + r) + (c0 + c) * ldf] = v;
+      const float v = Xs[r * XP + c];
+      put_operand<F>(Up + (c0 - up_col0 + c) * up_pitch + koff + r, plane, v);
+      LU[(j0 + r) + (c0 + c) * ldf] = from_f32<F>(v);
     }
   }
 }
@@ -808,110 +840,13 @@ constexpr size_t trsm_pair_smem(int rb) {
 template <typename F, int RB>
 __global__ void __launch_bounds__(TRSM_THREADS)
 k_trsm_pair(const float* __restrict__ W, long long ldw, long long j0, long long begin, long long n,
-            const float* __restrict__ Uinv, const float* __restrict__ Linv, F* __restrict__ Lp, F* __restrict__ Up,
-            long long pitch, long long base0, int koff, F* __restrict__ LU, long long ldf, int nb) {
+            const float* __restrict__ Uinv, const float* __restrict__ Linv, typename Operand<F>::T* __restrict__ Lp,
+            typename Operand<F>::T* __restrict__ Up, long long plane, long long pitch, long long base0, int koff,
+            F* __restrict__ LU, long long ldf, int nb) {
   if ((int)blockIdx.x < nb)
-    trsm_right_body<F, RB>(W, ldw, j0, begin, n, Uinv, Lp, pitch, base0, koff, LU, ldf, (int)blockIdx.x);
+    trsm_right_body<F, RB>(W, ldw, j0, begin, n, Uinv, Lp, plane, pitch, base0, koff, LU, ldf, (int)blockIdx.x);
   else
-    trsm_left_body<F, RB>(W, ldw, j0, begin, n, Linv, Up, pitch, base0, koff, LU, ldf, (int)blockIdx.x - nb);
-}
-
-// CUDA-core trailing update for FP32 factors: C -= A B^T, A (M x K) and B
-// (N x K) K-major FP32 with row pitch ldk.  CTA tile 128 x 128; K in slabs
-// of 16 staged transposed in shared memory, double-buffered (the next slab's
-// global loads sit in registers while the current slab is used, one barrier
-// per slab); thread tile 8 x 8 = rows {4 ty .. +3, 64 + 4 ty .. +3} x columns
-// {4 tx .. +3, 64 + 4 tx .. +3}, read as float4 (conflict-free).  Every
-// output accumulates its products in ascending k, one FMA each.
-constexpr int SG_BK = 16;
-constexpr int SG_P = 128 + 4;
-
-// Eight consecutive K-values of one operand row (zero past M or K).
-__device__ __forceinline__ void sg_load8(const float* __restrict__ X, int row, int rows, int k, int K, long long ldk,
-                                         float (&r)[8]) {
-  const float* p = X + (long long)row * ldk + k;
-  if (row < rows && k + 8 <= K && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-    const float4 u = __ldg(reinterpret_cast<const float4*>(p));
-    const float4 v = __ldg(reinterpret_cast<const float4*>(p) + 1);
-    r[0] = u.x; r[1] = u.y; r[2] = u.z; r[3] = u.w; r[4] = v.x; r[5] = v.y; r[6] = v.z; r[7] = v.w;
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) r[i] = (row < rows && k + i < K) ? __ldg(p + i) : 0.f;
-  }
-}
-
-__global__ void __launch_bounds__(256)
-k_gemm_update_f32(float* __restrict__ C, long long ldc, const float* __restrict__ A, const float* __restrict__ B,
-                  long long ldk, int M, int N, int K) {
-  __shared__ __align__(16) float As[2][SG_BK][SG_P];
-  __shared__ __align__(16) float Bs[2][SG_BK][SG_P];
-  const int tid = threadIdx.x;
-  const int m0 = blockIdx.x * 128, n0 = blockIdx.y * 128;
-  const int ty = tid / 16, tx = tid % 16;
-  const int lr = tid >> 1, lk = (tid & 1) * 8;  // staging: row lr, K-values lk .. lk + 7 of the slab
-  float ra[8], rb[8];
-  auto stage = [&](int buf) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      As[buf][lk + i][lr] = ra[i];
-      Bs[buf][lk + i][lr] = rb[i];
-    }
-  };
-  float acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-  sg_load8(A, m0 + lr, M, lk, K, ldk, ra);
-  sg_load8(B, n0 + lr, N, lk, K, ldk, rb);
-  stage(0);
-  __syncthreads();
-  for (int kb = 0; kb < K; kb += SG_BK) {
-    const int cur = (kb / SG_BK) & 1;
-    const bool more = kb + SG_BK < K;
-    if (more) {
-      sg_load8(A, m0 + lr, M, kb + SG_BK + lk, K, ldk, ra);
-      sg_load8(B, n0 + lr, N, kb + SG_BK + lk, K, ldk, rb);
-    }
-#pragma unroll
-    for (int k = 0; k < SG_BK; ++k) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&As[cur][k][4 * ty]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&As[cur][k][64 + 4 * ty]);
-      const float4 b0 = *reinterpret_cast<const float4*>(&Bs[cur][k][4 * tx]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&Bs[cur][k][64 + 4 * tx]);
-      const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    if (more) stage(cur ^ 1);  // the other buffer was last read before the previous barrier
-    __syncthreads();
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int col = n0 + (j < 4 ? 4 * tx + j : 64 + 4 * tx + j - 4);
-    if (col >= N) continue;
-    float* c = C + (long long)col * ldc;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int row = m0 + h * 64 + 4 * ty;
-      float* cp = c + row;
-      if (row + 4 <= M && (reinterpret_cast<uintptr_t>(cp) & 15) == 0) {
-        float4 v = *reinterpret_cast<float4*>(cp);
-        v.x -= acc[4 * h + 0][j];
-        v.y -= acc[4 * h + 1][j];
-        v.z -= acc[4 * h + 2][j];
-        v.w -= acc[4 * h + 3][j];
-        *reinterpret_cast<float4*>(cp) = v;
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (row + i < M) cp[i] -= acc[4 * h + i][j];
-      }
-    }
-  }
+    trsm_left_body<F, RB>(W, ldw, j0, begin, n, Linv, Up, plane, pitch, base0, koff, LU, ldf, (int)blockIdx.x - nb);
 }
 
 // ------------------------------------------------------------ TRSV (apply)
@@ -1377,7 +1312,7 @@ __global__ void k_scale_out_multi(const float* __restrict__ z, const float* __re
 //   2. k_laswp: the panel's row exchanges applied to every other column of W;
 //   3. k_piv_diag: the 128 x 128 diagonal block's unit-lower / upper inverses;
 //   4. U12 = L11^-1 W12 (the panel solve of the unpivoted path), L21 to the
-//      K-major operand, and W22 -= L21 U12 (tensor cores or CUDA cores);
+//      K-major operand, and W22 -= L21 U12 on the tensor cores;
 // and at the end the strictly lower part of W is rounded into the factor.
 
 // |a_ij| maxima per row over a column chunk (non-negative doubles compare as
@@ -1722,7 +1657,7 @@ k_piv_diag(const float* __restrict__ W, long long ldw, long long j0, int nbk, F*
 template <typename F>
 __global__ void __launch_bounds__(256)
 k_make_lop(const float* __restrict__ W, long long ldw, long long jp, int nb, long long r0, long long n,
-           F* __restrict__ Lp, long long pitch) {
+           typename Operand<F>::T* __restrict__ Lp, long long plane, long long pitch) {
   __shared__ float t[LNB][33];
   const long long rb = r0 + (long long)blockIdx.x * 32;
   for (int e = threadIdx.x; e < 32 * LNB; e += blockDim.x) {
@@ -1732,7 +1667,7 @@ k_make_lop(const float* __restrict__ W, long long ldw, long long jp, int nb, lon
   __syncthreads();
   for (int e = threadIdx.x; e < 32 * LNB; e += blockDim.x) {
     const int k = e % LNB, i = e / LNB;
-    if (rb + i < n && k < nb) Lp[(rb + i - r0) * pitch + k] = from_f32<F>(t[k][i]);
+    if (rb + i < n && k < nb) put_operand<F>(Lp + (rb + i - r0) * pitch + k, plane, t[k][i]);
   }
 }
 
@@ -2089,10 +2024,12 @@ static int lu_factor_t(const double* A, long long lda, long long n, int fdtype, 
   float* d = (float*)(fb + L.off_d);
   LUMeta* meta = (LUMeta*)(fb + L.off_meta);
   float* W = (float*)(wb + w.off_W);
-  F* Lp2 = (F*)(wb + w.off_Lp);
-  F* Up2 = (F*)(wb + w.off_Up);
+  using Op = typename Operand<F>::T;
+  Op* Lp2 = (Op*)(wb + w.off_Lp);
+  Op* Up2 = (Op*)(wb + w.off_Up);
   const long long spw = super_panel_width(fdtype);
-  const size_t opsz = (size_t)std::max(1LL, n) * spw;  // elements of one operand buffer
+  const long long plane = std::max(1LL, n) * spw;               // elements of one operand plane
+  const size_t opsz = (size_t)plane * Operand<F>::PLANES;       // elements of one operand buffer
   int* errw = (int*)(wb + w.off_err);
   MPDOK_CUDA_TRY(cudaMemsetAsync(errw, 0, 64, s));
   MPDOK_CUDA_TRY(cudaMemsetAsync(meta, 0, sizeof(LUMeta), s));
@@ -2108,21 +2045,13 @@ static int lu_factor_t(const double* A, long long lda, long long n, int fdtype, 
   MPDOK_TRY(set_smem(k_trsm_pair<F, 16>, smem_tp16));
   const float tau = 1e-6f;
   // C -= A B^T on one strip: A rows / B rows at the given Lp / Up offsets.
-  auto update = [&](long long crow, long long ccol, long long m, long long nn, const F* Ab, const F* Bb, int K,
+  auto update = [&](long long crow, long long ccol, long long m, long long nn, const Op* Ab, const Op* Bb, int K,
                     cudaStream_t st) -> int {
-    if (m <= 0 || nn <= 0) return MPDOK_OK;
     float* C = W + crow + ccol * w.ldw;
-    if (fdtype == MPDOK_F32) {
-      const int gs = prof_start(MPDOK_PROF_LU_GEMM, st);
-      dim3 gg((unsigned)((m + 127) / 128), (unsigned)((nn + 127) / 128));
-      launch(k_gemm_update_f32, gg, 256, 0, st, C, w.ldw, (const float*)Ab, (const float*)Bb, spw,
-             (int)m, (int)nn, K);
-      prof_stop(gs, st, 2.0 * (double)m * (double)nn * K);
-      prof_stop_bytes(gs, 8.0 * (double)m * (double)nn + 4.0 * (double)K * ((double)m + (double)nn));
-      MPDOK_LAUNCH_CHECK("lu gemm f32");
-      return MPDOK_OK;
-    }
-    return gemm_update(C, w.ldw, Ab, Bb, spw, (int)m, (int)nn, K, fdtype, MPDOK_ENGINE_TENSOR, errw, st);
+    if constexpr (std::is_same<F, float>::value)
+      return gemm_update_split3(C, w.ldw, Ab, Bb, spw, plane, (int)m, (int)nn, K, errw, st);
+    else
+      return gemm_update(C, w.ldw, Ab, Bb, spw, (int)m, (int)nn, K, fdtype, MPDOK_ENGINE_TENSOR, errw, st);
   };
   const bool lookahead = n > spw;
   // the chain first; the panel work below the super-panel next; the far update last
@@ -2147,8 +2076,8 @@ static int lu_factor_t(const double* A, long long lda, long long n, int fdtype, 
       }
       const cudaStream_t cs = streams[st.stream];
       const int buf = (int)((st.J / spw) & 1);
-      F* Lp = Lp2 + (size_t)buf * opsz;
-      F* Up = Up2 + (size_t)buf * opsz;
+      Op* Lp = Lp2 + (size_t)buf * opsz;
+      Op* Up = Up2 + (size_t)buf * opsz;
       switch (st.kind) {
         case LU_DIAG: {
           const int k = (int)(st.jp / LNB);
@@ -2166,11 +2095,11 @@ static int lu_factor_t(const double* A, long long lda, long long n, int fdtype, 
           if (st.rb == 16) {
             const int nb = (int)((st.b - st.a + 15) / 16);
             launch(k_trsm_pair<F, 16>, (unsigned)(2 * nb), TRSM_THREADS, smem_tp16, cs, (const float*)W, w.ldw, st.jp,
-                   st.a, st.b, ui, li, Lp, Up, spw, st.J, koff, LU, L.ldf, nb);
+                   st.a, st.b, ui, li, Lp, Up, plane, spw, st.J, koff, LU, L.ldf, nb);
           } else {
             const int nb = (int)((st.b - st.a + 63) / 64);
             launch(k_trsm_pair<F, 64>, (unsigned)(2 * nb), TRSM_THREADS, smem_tp, cs, (const float*)W, w.ldw, st.jp,
-                   st.a, st.b, ui, li, Lp, Up, spw, st.J, koff, LU, L.ldf, nb);
+                   st.a, st.b, ui, li, Lp, Up, plane, spw, st.J, koff, LU, L.ldf, nb);
           }
           MPDOK_LAUNCH_CHECK("lu panel solve");
           break;
@@ -2269,9 +2198,11 @@ static int lu_factor_piv(const double* A, long long lda, long long n, int fdtype
   int* ipiv = (int*)(fb + L.off_ipiv);
   LUMeta* meta = (LUMeta*)(fb + L.off_meta);
   float* W = (float*)(wb + w.off_W);
-  F* Lp = (F*)(wb + w.off_Lp);
-  F* Up = (F*)(wb + w.off_Up);
+  using Op = typename Operand<F>::T;
+  Op* Lp = (Op*)(wb + w.off_Lp);
+  Op* Up = (Op*)(wb + w.off_Up);
   const long long pitch = super_panel_width(fdtype);
+  const long long plane = n * pitch;
   int* errw = (int*)(wb + w.off_err);  // [0] tensor-core wait, [2] first zero pivot, [3] panel barrier wait
   PivCand* cand = (PivCand*)(wb + w.off_cand);
   float* crow = (float*)(wb + w.off_crow);
@@ -2330,21 +2261,14 @@ static int lu_factor_piv(const double* A, long long lda, long long n, int fdtype
     // U12 = L11^-1 W12 (rows jp .. jp + 128, every column to the right)
     launch(k_trsm_pair<F, 64>, (unsigned)((rest + 63) / 64), TRSM_THREADS, smem_tp, s, (const float*)W, w.ldw, jp,
            r1, n, (const float*)(Uinv + (size_t)k * LNB * LNB), (const float*)(Linv + (size_t)k * LNB * LNB), Lp, Up,
-           pitch, r1, 0, LU, L.ldf, 0);
-    launch(k_make_lop<F>, (unsigned)((rest + 31) / 32), 256, 0, s, (const float*)W, w.ldw, jp, nb, r1, n, Lp, pitch);
+           plane, pitch, r1, 0, LU, L.ldf, 0);
+    launch(k_make_lop<F>, (unsigned)((rest + 31) / 32), 256, 0, s, (const float*)W, w.ldw, jp, nb, r1, n, Lp, plane, pitch);
     MPDOK_LAUNCH_CHECK("pivoted panel solve");
     float* C = W + r1 + r1 * w.ldw;
-    if (fdtype == MPDOK_F32) {
-      const int gs = prof_start(MPDOK_PROF_LU_GEMM, s);
-      dim3 gg((unsigned)((rest + 127) / 128), (unsigned)((rest + 127) / 128));
-      launch(k_gemm_update_f32, gg, 256, 0, s, C, w.ldw, (const float*)Lp, (const float*)Up, pitch, (int)rest,
-             (int)rest, nb);
-      prof_stop(gs, s, 2.0 * (double)rest * (double)rest * nb);
-      prof_stop_bytes(gs, 8.0 * (double)rest * (double)rest + 4.0 * nb * 2.0 * (double)rest);
-      MPDOK_LAUNCH_CHECK("pivoted update f32");
-    } else {
+    if constexpr (std::is_same<F, float>::value)
+      MPDOK_TRY(gemm_update_split3(C, w.ldw, Lp, Up, pitch, plane, (int)rest, (int)rest, nb, errw, s));
+    else
       MPDOK_TRY(gemm_update(C, w.ldw, Lp, Up, pitch, (int)rest, (int)rest, nb, fdtype, MPDOK_ENGINE_TENSOR, errw, s));
-    }
   }
   {
     dim3 g2((unsigned)std::min<long long>((n + 255) / 256, 16), (unsigned)std::min<long long>(n, 65535));

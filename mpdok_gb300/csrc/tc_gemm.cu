@@ -538,6 +538,276 @@ tc_gemm_update_ws(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 
 }  // namespace ws
 
+// ------------------------------------------------------------------------
+// FP32 operands on the BF16 tensor cores: C -= A B^T with A and B each given as
+// three BF16 planes, x = h + m + l exactly (h, m, l the round-to-nearest BF16
+// values of x and of what is left: 3 x 8 bits cover FP32's 24).  Six of the
+// nine plane products are formed, l h + h l + m m + m h + h m + h h; the others
+// are below 2^-26 of |a| |b|.
+//
+// The tensor cores truncate every accumulation to FP32 (one instruction's 16
+// products at a time), so a long K would drift towards zero: by 9e-7 of the sum
+// at K = 512 for terms of one sign, where a chain of FMAs is off by 2.6e-7.
+// Each 16-deep K step is therefore accumulated from zero, its five small
+// products before h h, and then drained and added in round-to-nearest FP32
+// by the epilogue warps, which hold the tile's running sum in registers: one
+// truncation at full size per step.  ||L U - W|| / ||W|| of the factorization
+// against the chain of FMAs that this replaces: n = 5000 8.0e-8 / 14.4e-8
+// (Gaussian), 9.3e-8 / 10.2e-8 (Gaussian, nugget 1e-6), 8.5e-8 / 12.0e-8
+// (pivoted), 5.2e-6 / 11.6e-6 (pivoted, N(0, 1)).  Draining every 32 would be 8%
+// faster at n = 32768 but less exact than the chain in some families.
+//
+// One CTA walks a strip of T tiles of 128 x 256.  Warp 0 issues TMA loads into a
+// ring of eight 24 KB slots (one plane of A and B of one 32-deep K block, 64-byte
+// swizzle; planes in the order h, l, m), warp 1 the MMAs (six per K step, 128 x
+// 256 x 16 each, into two alternating 256-column accumulators), warps 2..17
+// drain (64 columns of a lane quarter each) and, at the end of a tile, add -sum into C with TMA
+// reduce-adds.  A plane is loaded once for the four, four or two products that
+// use it, so a K block moves 72 KB for 12 MMAs: half the bytes per MMA of the
+// plain kernel above, which those bytes bound.  Factorization: n = 32768 516.8
+// -> 122.9 ms, 16384 72.9 -> 21.8 ms, 8192 13.2 -> 6.7 ms (CUDA-core FMAs before).
+namespace split3 {
+
+constexpr int BK3 = 32;
+constexpr int SLOTS = 8;
+constexpr int A_SUB = BM * BK3 * 2;  // 8 KB
+constexpr int B_SUB = BN * BK3 * 2;  // 16 KB
+constexpr int SLOT = A_SUB + B_SUB;
+constexpr int EPI_WARPS3 = 16;
+constexpr int THREADS3 = 32 * (2 + EPI_WARPS3);
+constexpr int COLS = BN * 4 / EPI_WARPS3;  // accumulator columns of one epilogue warp
+constexpr int STG_COLS = 8;                // columns of one staging buffer, two buffers per warp
+constexpr int STG_BUF = 32 * STG_COLS * 4;
+constexpr int STAGING_OFF = SLOTS * SLOT;
+constexpr int BAR_OFF = STAGING_OFF + EPI_WARPS3 * 2 * STG_BUF;
+constexpr int NBAR = 2 * SLOTS + 5;
+constexpr int TOTAL = BAR_OFF + 8 * NBAR + 16;
+constexpr int ALLOC = TOTAL + 1024;
+static_assert(ALLOC <= 232448, "shared memory of one CTA");
+
+// K-major operand, 64-byte swizzle: 8-row atoms 512 bytes apart.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) |
+         ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
+}
+
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+
+__global__ void __launch_bounds__(THREADS3, 1)
+tc_gemm_update_split3(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                      const __grid_constant__ CUtensorMap tmC, int M, int N, int K, int T, int* err) {
+  using namespace ws;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  uint8_t* gbase = smem_raw + (base - raw);
+  const uint32_t bar_full = base + split3::BAR_OFF;
+  const uint32_t bar_empty = bar_full + 8 * SLOTS;
+  const uint32_t bar_accf = bar_empty + 8 * SLOTS;
+  const uint32_t bar_acce = bar_accf + 16;
+  const uint32_t bar_drain = bar_acce + 16;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + split3::BAR_OFF + 8 * split3::NBAR);
+  __shared__ int s_fail;
+  volatile int* fail = &s_fail;
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int m0 = blockIdx.x * BM;
+  const int tile0 = blockIdx.y * T;
+  const int ntiles_n = (N + BN - 1) / BN;
+  const int nt = max(0, min(T, ntiles_n - tile0));
+  const int KB = K / BK3;
+
+  if (threadIdx.x == 0) {
+    s_fail = 0;
+    for (int st = 0; st < SLOTS; ++st) {
+      mbar_init(bar_full + 8 * st, 1);
+      mbar_init(bar_empty + 8 * st, 1);
+    }
+    mbar_init(bar_accf, 1);
+    mbar_init(bar_accf + 8, 1);
+    mbar_init(bar_acce, EPI_WARPS3);
+    mbar_init(bar_acce + 8, EPI_WARPS3);
+    mbar_init(bar_drain, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(ws::TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // producer: planes h, l, m of every (tile, K block)
+      int g = 0;
+      bool ok = true;
+      for (int t = 0; t < nt && ok; ++t) {
+        const int n0 = (tile0 + t) * BN;
+        for (int kb = 0; kb < KB && ok; ++kb) {
+          for (int i = 0; i < 3; ++i, ++g) {
+            const int plane = i == 0 ? 0 : 3 - i;
+            const int st = g % SLOTS, round = g / SLOTS;
+            if (round > 0 && !wait_or_fail(bar_empty + 8 * st, (round - 1) & 1, fail)) {
+              atomicExch(&s_fail, 1);
+              ok = false;
+              break;
+            }
+            const uint32_t sa = base + st * SLOT;
+            mbar_expect_tx(bar_full + 8 * st, (uint32_t)SLOT);
+            tma_load_3d(sa, &tmA, bar_full + 8 * st, kb * BK3, m0, plane);
+            tma_load_3d(sa + split3::A_SUB, &tmB, bar_full + 8 * st, kb * BK3, n0, plane);
+          }
+        }
+      }
+      if (!ok || *fail) {
+        // loads still in flight land in this CTA's shared memory: wait for
+        // each slot's last issued load (bounded) before the CTA may exit
+        for (int st = 0; st < SLOTS && st < g; ++st) {
+          const int last = g - 1 - ((g - 1 - st) % SLOTS);
+          const int round = last / SLOTS;
+          for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(bar_full + 8 * st, round & 1); ++i) {
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = idesc_f16(true, BM, BN);
+      int g = 0, gc = 0;
+      bool ok = true;
+      auto full = [&](int slot_g) {
+        if (!wait_or_fail(bar_full + 8 * (slot_g % SLOTS), (slot_g / SLOTS) & 1, fail)) {
+          atomicExch(&s_fail, 3);
+          return false;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        return true;
+      };
+      auto a_of = [&](int slot_g) { return base + (slot_g % SLOTS) * SLOT; };
+      for (int t = 0; t < nt && ok; ++t) {
+        for (int kb = 0; kb < KB && ok; ++kb, g += 3) {
+          const uint32_t sh = a_of(g), sl = a_of(g + 1), sm = a_of(g + 2);
+          if (!full(g) || !full(g + 1) || !full(g + 2)) {
+            ok = false;
+            break;
+          }
+#pragma unroll
+          for (int k = 0; k < BK3 / 16; ++k, ++gc) {
+            const int a = gc & 1, use = gc >> 1;
+            if (use > 0 && !wait_or_fail(bar_acce + 8 * a, (use - 1) & 1, fail)) {
+              atomicExch(&s_fail, 2);
+              ok = false;
+              break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t dacc = tmem + (uint32_t)(a * BN);
+            auto mul = [&](uint32_t pa, uint32_t pb, uint32_t add) {
+              mma_f16(dacc, smem_desc_sw64(pa + k * 32), smem_desc_sw64(pb + split3::A_SUB + k * 32), idesc, add);
+            };
+            constexpr int LAST = BK3 / 16 - 1;
+            mul(sl, sh, 0u);
+            mul(sh, sl, 1u);
+            if (k == LAST) mma_commit(bar_empty + 8 * ((g + 1) % SLOTS));
+            mul(sm, sm, 1u);
+            mul(sm, sh, 1u);
+            mul(sh, sm, 1u);
+            if (k == LAST) mma_commit(bar_empty + 8 * ((g + 2) % SLOTS));
+            mul(sh, sh, 1u);
+            if (k == LAST) mma_commit(bar_empty + 8 * (g % SLOTS));
+            mma_commit(bar_accf + 8 * a);
+          }
+        }
+      }
+      // every MMA issued here has completed before the tensor memory is released
+      mma_commit(bar_drain);
+      for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(bar_drain, 0); ++i) {
+        if (i > 64) __nanosleep(32);
+      }
+    }
+  } else {
+    // lane quarter q = warp % 4 (rows m0 + 32 q + lane), column group h of COLS
+    const int q = warp & 3, h = (warp - 2) >> 2;
+    const int ew = warp - 2;
+    float* stg = reinterpret_cast<float*>(gbase + split3::STAGING_OFF + ew * 2 * STG_BUF);
+    const uint32_t stg_s = base + split3::STAGING_OFF + ew * 2 * STG_BUF;
+    int nbuf = 0, gc = 0;
+    bool ok = true;
+    for (int t = 0; t < nt && ok; ++t) {
+      const int nbase = (tile0 + t) * BN + h * COLS;
+      float2 sum[COLS / 2];
+#pragma unroll
+      for (int c = 0; c < COLS / 2; ++c) sum[c] = make_float2(0.f, 0.f);
+      for (int kb = 0; kb < K / 16; ++kb, ++gc) {
+        const int a = gc & 1, use = gc >> 1;
+        if (!wait_or_fail(bar_accf + 8 * a, use & 1, fail)) {
+          atomicExch(&s_fail, 4);
+          ok = false;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t tacc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * BN + h * COLS);
+#pragma unroll
+        for (int i = 0; i < COLS / 16; ++i) {
+          float v[16];
+          tmem_ld16(tacc + (uint32_t)(i * 16), v);
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            sum[i * 8 + c] = __fadd2_rn(sum[i * 8 + c], make_float2(v[2 * c], v[2 * c + 1]));
+        }
+        // this warp has read its part of accumulator a: hand it back to the MMA
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_acce + 8 * a);
+      }
+      if (!ok) break;
+#pragma unroll
+      for (int i = 0; i < COLS / STG_COLS; ++i) {
+        // (uniform per warp: chunks past N or M hold nothing to add)
+        if (nbase + i * STG_COLS < N && m0 + q * 32 < M) {
+          const int b = nbuf & 1;
+          ++nbuf;
+          if (lane == 0) bulk_wait_read<1>();  // the buffer's previous reduce has read it
+          __syncwarp();
+          float* buf = stg + b * (STG_BUF / 4);
+#pragma unroll
+          for (int c = 0; c < STG_COLS / 2; ++c) {
+            const float2 v = sum[i * (STG_COLS / 2) + c];
+            buf[2 * c * 32 + lane] = -v.x;
+            buf[(2 * c + 1) * 32 + lane] = -v.y;
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) {
+            tma_reduce_add_2d(&tmC, stg_s + b * STG_BUF, m0 + q * 32, nbase + i * STG_COLS);
+            bulk_commit();
+          }
+        }
+      }
+    }
+    if (lane == 0) bulk_wait<0>();  // every reduce of this warp has completed
+    __syncwarp();
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x == 0 && s_fail != 0 && err) atomicExch(err, 1);
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ws::TMEM_COLS));
+  }
+}
+
+}  // namespace split3
+
 // CUDA-core comparator with the same operand rounding (test use).
 __global__ void simt_gemm_update(const void* A, const void* B, long long ldk, int bf16, float* C, long long ldc,
                                  int M, int N, int K) {
@@ -597,9 +867,31 @@ static int make_map(CUtensorMap* map, const void* ptr, int rows, int K, long lon
   return MPDOK_OK;
 }
 
+// 3-D tensor map over the three BF16 planes of a K-major operand: box 32 x box_rows x 1.
+static int make_map_planes(CUtensorMap* map, const void* ptr, int rows, int K, long long ldk, long long plane,
+                           int box_rows) {
+  auto enc = get_encode();
+  if (!enc) {
+    set_error("cuTensorMapEncodeTiled unavailable from the driver");
+    return MPDOK_ERR_UNSUPPORTED;
+  }
+  cuuint64_t gdim[3] = {(cuuint64_t)K, (cuuint64_t)rows, 3};
+  cuuint64_t gstride[2] = {(cuuint64_t)ldk * 2, (cuuint64_t)plane * 2};
+  cuuint32_t box[3] = {(cuuint32_t)tc::split3::BK3, (cuuint32_t)box_rows, 1};
+  cuuint32_t es[3] = {1, 1, 1};
+  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), gdim, gstride, box, es,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled (planes) failed (%d)", (int)r);
+    return MPDOK_ERR_CUDA;
+  }
+  return MPDOK_OK;
+}
+
 // 2-D tensor map over the FP32 C (rows x columns, column-major, ldc), box 32
-// rows x 16 columns: the target of the epilogue's TMA reduce-adds.
-static int make_map_c(CUtensorMap* map, float* C, int M, int N, long long ldc) {
+// rows x box_cols columns: the target of the epilogue's TMA reduce-adds.
+static int make_map_c(CUtensorMap* map, float* C, int M, int N, long long ldc, int box_cols) {
   auto enc = get_encode();
   if (!enc) {
     set_error("cuTensorMapEncodeTiled unavailable from the driver");
@@ -607,7 +899,7 @@ static int make_map_c(CUtensorMap* map, float* C, int M, int N, long long ldc) {
   }
   cuuint64_t gdim[2] = {(cuuint64_t)M, (cuuint64_t)N};
   cuuint64_t gstride[1] = {(cuuint64_t)ldc * 4};
-  cuuint32_t box[2] = {32, (cuuint32_t)tc::ws::EPI_COLS};
+  cuuint32_t box[2] = {32, (cuuint32_t)box_cols};
   cuuint32_t es[2] = {1, 1};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, C, gdim, gstride, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -648,18 +940,24 @@ static int sm_count() {
   return cnt[dev];
 }
 
+// Tiles per CTA along N for a grid of ntm row blocks: WS_TILES, fewer while the
+// strips would not fill the GPU once (the 128-row block updates of the
+// left-looking panels).
+static int strip_tiles(int ntm, int ntn) {
+  int T = WS_TILES;
+  while (T > 1 && (long long)ntm * ((ntn + T - 1) / T) < sm_count()) T >>= 1;
+  return T;
+}
+
 static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, float* C, long long ldc, int M, int N, int K,
                      int bf16, int* err, cudaStream_t s) {
   if (K >= WS_MIN_K && aligned16(C) && ldc % 4 == 0) {
     CUtensorMap mc;
-    MPDOK_TRY(make_map_c(&mc, C, M, N, ldc));
+    MPDOK_TRY(make_map_c(&mc, C, M, N, ldc, tc::ws::EPI_COLS));
     MPDOK_TRY(set_smem(tc::ws::tc_gemm_update_ws, tc::ws::ALLOC));
     const int ntm = (M + tc::BM - 1) / tc::BM;
     const int ntn = (N + tc::BN - 1) / tc::BN;
-    // fewer tiles per CTA while the strips would not fill the GPU once (the
-    // 128-row block updates of the left-looking panels)
-    int T = WS_TILES;
-    while (T > 1 && (long long)ntm * ((ntn + T - 1) / T) < sm_count()) T >>= 1;
+    const int T = strip_tiles(ntm, ntn);
     dim3 grid(ntm, (ntn + T - 1) / T);
     tc::ws::tc_gemm_update_ws<<<grid, tc::ws::THREADS, tc::ws::ALLOC, s>>>(ma, mb, mc, M, N, K, T, bf16, err);
     count_launch();
@@ -699,6 +997,33 @@ int gemm_update(float* C, long long ldc, const void* A, const void* B, long long
   prof_stop(slot, s, 2.0 * (double)M * (double)N * (double)K);
   // C read and written in FP32, both 16-bit operands read once
   prof_stop_bytes(slot, 8.0 * (double)M * (double)N + 2.0 * (double)K * ((double)M + (double)N));
+  return MPDOK_OK;
+}
+
+// C -= A B^T with FP32 operands as three BF16 planes each (plane p of row r,
+// column k at X[p * plane + r * ldk + k]).
+int gemm_update_split3(float* C, long long ldc, const __nv_bfloat16* A, const __nv_bfloat16* B, long long ldk,
+                       long long plane, int M, int N, int K, int* err, cudaStream_t s) {
+  if (M <= 0 || N <= 0 || K <= 0) return MPDOK_OK;
+  MPDOK_ARG_CHECK(K % tc::split3::BK3 == 0 && ldk >= K, "FP32 update: K must be a multiple of 32 within the pitch");
+  MPDOK_ARG_CHECK(aligned16(C) && ldc % 4 == 0 && ldc >= M, "FP32 update: C must be 16-byte aligned");
+  MPDOK_ARG_CHECK(aligned16(A) && aligned16(B) && ldk % 8 == 0 && plane % 8 == 0,
+                  "FP32 update: operands must be 16-byte aligned");
+  const int slot = prof_start(MPDOK_PROF_LU_GEMM, s);
+  CUtensorMap ma, mb, mc;
+  MPDOK_TRY(make_map_planes(&ma, A, M, K, ldk, plane, tc::BM));
+  MPDOK_TRY(make_map_planes(&mb, B, N, K, ldk, plane, tc::BN));
+  MPDOK_TRY(make_map_c(&mc, C, M, N, ldc, tc::split3::STG_COLS));
+  MPDOK_TRY(set_smem(tc::split3::tc_gemm_update_split3, tc::split3::ALLOC));
+  const int ntm = (M + tc::BM - 1) / tc::BM, ntn = (N + tc::BN - 1) / tc::BN;
+  const int T = strip_tiles(ntm, ntn);
+  dim3 grid(ntm, (ntn + T - 1) / T);
+  tc::split3::tc_gemm_update_split3<<<grid, tc::split3::THREADS3, tc::split3::ALLOC, s>>>(ma, mb, mc, M, N, K, T, err);
+  count_launch();
+  MPDOK_LAUNCH_CHECK("tc_gemm_update_split3");
+  prof_stop(slot, s, 2.0 * (double)M * (double)N * (double)K);
+  // C read and written in FP32, three 16-bit planes of both operands read once
+  prof_stop_bytes(slot, 8.0 * (double)M * (double)N + 6.0 * (double)K * ((double)M + (double)N));
   return MPDOK_OK;
 }
 

@@ -2,8 +2,8 @@
 
 ``LUFactorization(A, dtype)`` factors W = D A D (D = diag(1/sqrt|a_ii|)) with
 128-wide FP32 panels and a tcgen05 trailing update whose operands are rounded
-to BF16 or FP16 (FP32 accumulation).  ``dtype='fp32'`` keeps FP32 operands and
-runs the update on CUDA cores (the reference's Sgetrf precision).
+to BF16 or FP16 (FP32 accumulation).  ``dtype='fp32'`` keeps FP32 operands, each
+as three BF16 planes on the tensor cores (the reference's Sgetrf precision).
 ``pivoting=True`` equilibrates rows and columns by powers of two and pivots by
 rows (P Dr A Dc = L U), the reference's cusolverDnSgetrf semantics.
 
