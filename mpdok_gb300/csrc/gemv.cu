@@ -157,26 +157,43 @@ gemv_t_stage1(const TA* __restrict__ A, long long lda, long long m, long long n,
   }
 }
 
-// y[i,k] = alpha * sum_s P[s,k,i] + beta * bsrc[i,k]; optional sum of y^2.
+// y[i,k] = alpha * sum_s P[s,k,i] + beta * bsrc[i,k]; optional sum of y^2.  Each
+// block sums FIN_ROWS entries, four threads to an entry (every fourth split,
+// eight loads in flight): bound by the latency of the loads, so the splits are
+// spread rather than walked (n = 8192, 76 splits: 5.7 us; 10.2 us with one
+// thread to an entry).  The order of the sum is fixed.
+constexpr int FIN_ROWS = GEMV_THREADS / 4;
 template <typename ACC>
 __global__ void __launch_bounds__(GEMV_THREADS)
 gemv_finalize(const ACC* __restrict__ P, int S, int K, long long m, ACC alpha, ACC beta,
               const ACC* bsrc, long long ldb, ACC* y, long long ldy,
               double* nrm_parts, unsigned* ticket, double* nrm2, const int* skip) {
   __shared__ double red[32];
+  __shared__ ACC part[4][FIN_ROWS];
   if (skip != nullptr && *skip) return;
   const long long total = m * K;
+  const int r = threadIdx.x % FIN_ROWS, q = threadIdx.x / FIN_ROWS;
   double sq = 0.0;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long i = idx % m;
-    const int k = (int)(idx / m);
+  for (long long b0 = (long long)blockIdx.x * FIN_ROWS; b0 < total; b0 += (long long)gridDim.x * FIN_ROWS) {
+    const long long idx = b0 + r;
     ACC sum = ACC(0);
-    for (int s = 0; s < S; ++s) sum += P[((long long)s * K + k) * m + i];
-    ACC v = alpha * sum;
-    if (beta != ACC(0)) v = fma(beta, bsrc[i + k * ldb], v);
-    y[i + k * ldy] = v;
-    sq += (double)v * (double)v;
+    if (idx < total) {
+      const ACC* p = P + idx;  // P is [S][K][m], idx = k m + i
+#pragma unroll 8
+      for (int s = q; s < S; s += 4) sum += p[s * total];
+    }
+    part[q][r] = sum;
+    __syncthreads();
+    if (q == 0 && idx < total) {
+      const long long i = idx % m;
+      const int k = (int)(idx / m);
+      sum = ((sum + part[1][r]) + part[2][r]) + part[3][r];
+      ACC v = alpha * sum;
+      if (beta != ACC(0)) v = fma(beta, bsrc[i + k * ldb], v);
+      y[i + k * ldy] = v;
+      sq += (double)v * (double)v;
+    }
+    __syncthreads();
   }
   if (nrm2 != nullptr) {
     double b = block_sum(sq, red);
@@ -255,7 +272,7 @@ gemv_n_small_f64(const double* __restrict__ A, long long lda, int m, int n, cons
 }
 
 static unsigned finalize_blocks(long long total) {
-  long long b = (total + GEMV_THREADS - 1) / GEMV_THREADS;
+  long long b = (total + FIN_ROWS - 1) / FIN_ROWS;
   long long cap = (long long)num_sms() * 4;
   return (unsigned)std::max(1LL, std::min(b, cap));
 }

@@ -44,140 +44,361 @@ struct ArnState {
   double* y;
 };
 
-// Per-block dot products of V[:, 0..kp1) (rows of this chunk) with sw.
-__device__ __forceinline__ void block_dots(const float* Vc, long long ldv, int kp1, const float* sw, int len,
-                                           double* part_out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int j = warp; j < kp1; j += nw) {
-    const float* v = Vc + (long long)j * ldv;
-    double acc = 0.0;
-    for (int i = lane; i < len; i += 32) acc = fma((double)v[i], (double)sw[i], acc);
-    acc = warp_sum(acc);
-    if (lane == 0) part_out[j] = acc;
-  }
+// ------------------------------------------------------------- Arnoldi step
+// One launch per step: classical Gram-Schmidt (one or two passes) of w against
+// V[:, 0..k], ||w||, the Givens update of the Hessenberg column and
+// V[:, k+1] = w / ||w||.  G co-resident CTAs (a cooperative launch) own R rows
+// each and meet at two or three grid barriers; every CTA then sums the G partial
+// dot products itself, in one fixed order, so the step is reproducible and needs
+// no further hand-off.
+//
+// What bounds it is FP64: a warp's FP64 instruction occupies an SM for 16
+// clocks and dependent ones are about 170 apart.  So the rows are spread over
+// 64 CTAs (128 above n = 16384: more of them shorten the dot products and
+// lengthen the sums of the partials); the dot products of four columns share one
+// shuffle reduction (6 additions instead of 20); FP32 entries are widened by
+// integer operations; and the rotations of the new column, a linear recurrence,
+// run as a warp scan while the CTAs gather at the last barrier.  Taking ||w||
+// from the second pass instead (||w||^2 - ||h2||^2, right to 1e-8) would spare
+// that barrier, but a stagnating restarted solve then leaves the reference's
+// trajectory.  n = 8192, 1 to 50 columns: 26.4 us per step on average, the four
+// kernels that it replaces 50 us and three more launches.
+constexpr int AT = 512;              // threads
+constexpr int A_SUB = 1024;          // rows staged at a time
+constexpr int A_SL = 4;              // row slices of the dot products
+constexpr long long ARN_WAIT = 1LL << 22;
+
+__device__ __forceinline__ void arn_arrive(unsigned* p) {  // releases what the block's last barrier covers
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
+}
+__device__ __forceinline__ unsigned arn_ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
 }
 
-// Ordered column sums of parts[b * kp1 + j] over blocks b, by the last block.
-__device__ __forceinline__ void finish_dots(const double* parts, int nb, int kp1, double* out, double* accum) {
-  for (int j = threadIdx.x; j < kp1; j += blockDim.x) {
-    double s = 0.0;
-    for (int b = 0; b < nb; ++b) s += __ldcg(parts + (long long)b * kp1 + j);
-    out[j] = s;
-    if (accum) accum[j] += s;
-  }
+// (double)f by integer operations for normal numbers.
+__device__ __forceinline__ double widen_f32(float f) {
+  const unsigned u = __float_as_uint(f);
+  if (((u & 0x7f800000u) - 0x00800000u) < 0x7f000000u)
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(u << 29));
+  return (double)f;
 }
 
-// h = V[:, :kp1]^T w  (first Gram-Schmidt pass), stored into `out`.
-__global__ void __launch_bounds__(KT)
-k_dots(const float* __restrict__ V, long long ldv, int kp1, const float* __restrict__ w, long long n, long long ch,
-       double* parts, unsigned* ticket, double* out, const KScal* sc) {
-  extern __shared__ float sw[];
-  if (sc->done) return;
-  const long long r0 = (long long)blockIdx.x * ch;
-  const int len = (int)min(ch, n - r0);
-  for (int t = threadIdx.x; t < len; t += blockDim.x) sw[t] = w[r0 + t];
-  __syncthreads();
-  block_dots(V + r0, ldv, kp1, sw, len, parts + (long long)blockIdx.x * kp1);
-  if (last_block_arrive(ticket)) {
-    finish_dots(parts, gridDim.x, kp1, out, nullptr);
-    if (threadIdx.x == 0) *ticket = 0u;
-  }
-}
+struct ArnStep {
+  const float* V;
+  long long ldv;
+  int kp1;           // columns of V to orthogonalise against
+  float* w;
+  float* vnext;
+  long long n;
+  int R;             // rows per CTA
+  double* parts;     // [G][kp1] dot products of each pass, [G] squares
+  unsigned* bar;     // [3] barrier counters, zero between launches (bar[2]: reset by the next one)
+  double tol_rel;
+  int passes;
+  int* hdone;        // pinned host copy of the done flag after this step, or null
+};
 
-// Arnoldi step finish (one thread): H(k+1,k), previous rotations, new Givens
-// rotation, residual estimate g, stop flags.  mpdok_ooc.py:275-301.
-__device__ void arnoldi_finish(KScal* sc, const ArnState& st, int k, double nrm2, double tol_rel) {
-  double* H = st.H;
-  const long long ldh = st.ldh;
-  const double nrm = sqrt(nrm2);
-  H[(k + 1) + k * ldh] = nrm;
-  const bool bd = !(nrm > 1e-12);
-  for (int j = 0; j < k; ++j) {
-    const double hj = H[j + k * ldh], hj1 = H[(j + 1) + k * ldh];
-    const double tmp = st.cs[j] * hj + st.sn[j] * hj1;
-    H[(j + 1) + k * ldh] = -st.sn[j] * hj + st.cs[j] * hj1;
-    H[j + k * ldh] = tmp;
-  }
-  const double a = H[k + k * ldh], b = H[(k + 1) + k * ldh];
-  const double rho = hypot(a, b);
-  double c = 1.0, s = 0.0;
-  if (rho != 0.0) { c = a / rho; s = b / rho; }
-  st.cs[k] = c;
-  st.sn[k] = s;
-  H[k + k * ldh] = (rho != 0.0) ? rho : a;
-  H[(k + 1) + k * ldh] = 0.0;
-  st.g[k + 1] = -s * st.g[k];
-  st.g[k] = c * st.g[k];
-  sc->m_used = k + 1;
-  sc->aux = nrm;
-  if (!isfinite(nrm) || !isfinite(st.g[k + 1])) {
-    sc->nonfinite = 1;
-    sc->done = 1;
-  } else if (bd) {
-    sc->breakdown = 1;
-    sc->done = 1;
-  } else if (tol_rel > 0.0 && fabs(st.g[k + 1]) / sc->beta < tol_rel) {
-    sc->done = 1;
-  }
-}
-
-// w -= V[:, :kp1] h, then either the second-pass dots (MODE 0) or ||w||^2 and
-// the step finish (MODE 1).
-template <int MODE>
-__global__ void __launch_bounds__(KT)
-k_apply(const float* __restrict__ V, long long ldv, int kp1, float* __restrict__ w, long long n, long long ch,
-        const double* h, double* parts, unsigned* ticket, double* h2out, double* Hcol, KScal* sc, ArnState st,
-        int k, double tol_rel) {
-  extern __shared__ float smem[];
-  float* sh = smem;             // kp1 floats
-  float* sw = smem + KMAX_RESTART + 1;  // ch floats
-  __shared__ double red[32];
-  if (sc->done) return;
-  for (int j = threadIdx.x; j < kp1; j += blockDim.x) sh[j] = (float)h[j];
-  __syncthreads();
-  const long long r0 = (long long)blockIdx.x * ch;
-  const int len = (int)min(ch, n - r0);
-  double sq = 0.0;
-  for (int t = threadIdx.x; t < len; t += blockDim.x) {
-    const float* v = V + r0 + t;
-    float acc = 0.f;
-    for (int j = 0; j < kp1; ++j) acc = fmaf(v[(long long)j * ldv], sh[j], acc);
-    const float nw = w[r0 + t] - acc;
-    w[r0 + t] = nw;
-    if (MODE == 0) sw[t] = nw;
-    else sq = fma((double)nw, (double)nw, sq);
-  }
-  if (MODE == 0) {
-    __syncthreads();
-    block_dots(V + r0, ldv, kp1, sw, len, parts + (long long)blockIdx.x * kp1);
-    if (last_block_arrive(ticket)) {
-      finish_dots(parts, gridDim.x, kp1, h2out, Hcol);
-      if (threadIdx.x == 0) *ticket = 0u;
-    }
-  } else {
-    const double bsum = block_sum(sq, red);
-    if (threadIdx.x == 0) parts[blockIdx.x] = bsum;
-    if (last_block_arrive(ticket)) {
-      if (threadIdx.x < 32) {
-        double s = 0.0;
-        for (unsigned b = threadIdx.x; b < gridDim.x; b += 32) s += __ldcg(parts + b);
-        s = warp_sum(s);
-        if (threadIdx.x == 0) {
-          sc->nrm2 = s;
-          arnoldi_finish(sc, st, k, s, tol_rel);
-          *ticket = 0u;
-        }
+// The previous rotations on the new column h (in place), by one warp: the
+// running entry obeys t_{j+1} = -s_j t_j + c_j h_{j+1}, t_0 = h_0, and row j
+// becomes c_j t_j + s_j h_{j+1} (mpdok_ooc.py:283-287).
+__device__ void arnoldi_rotate(double* h, const double* cs, const double* sn, int k) {
+  const int lane = threadIdx.x & 31;
+  double t0 = h[0];
+  for (int j0 = 0; j0 < k; j0 += 32) {
+    const int j = j0 + lane;
+    const bool ok = j < k;
+    const double c = ok ? cs[j] : 1.0, s = ok ? sn[j] : -1.0, h1 = ok ? h[j + 1] : 0.0;
+    double A = -s, B = ok ? c * h1 : 0.0;  // (lanes past k keep t)
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double a1 = __shfl_up_sync(0xffffffffu, A, o), b1 = __shfl_up_sync(0xffffffffu, B, o);
+      if (lane >= o) {
+        B = fma(A, b1, B);
+        A *= a1;
       }
     }
+    const double tn = fma(A, t0, B);  // t_{j+1}
+    double t = __shfl_up_sync(0xffffffffu, tn, 1);
+    if (lane == 0) t = t0;
+    t0 = __shfl_sync(0xffffffffu, tn, 31);
+    __syncwarp();
+    if (ok) h[j] = c * t + s * h1;
+    __syncwarp();
+  }
+  if (lane == 0) h[k] = t0;
+  __syncwarp();
+}
+
+// H(k+1,k), the new rotation, the residual estimate g and the stop flags
+// (mpdok_ooc.py:275-301) from a = H(k,k) rotated, ||w||^2, ||w|| and
+// 1 / sqrt(a^2 + ||w||^2); returns the done flag.
+__device__ bool arnoldi_finish(KScal* sc, const ArnState& st, int k, double a, double nrm2, double nrm, double rinv,
+                               double gk, double beta, double tol_rel) {
+  const bool bd = !(nrm > 1e-12);
+  const double rho2 = fma(a, a, nrm2);
+  double c = 1.0, s = 0.0, r = a;
+  if (rho2 != 0.0) {
+    c = a * rinv;
+    s = nrm * rinv;
+    r = rho2 * rinv;
+  }
+  const double gk1 = -s * gk;
+  st.cs[k] = c;
+  st.sn[k] = s;
+  st.H[k + k * st.ldh] = r;
+  st.H[(k + 1) + k * st.ldh] = 0.0;
+  st.g[k + 1] = gk1;
+  st.g[k] = c * gk;
+  sc->nrm2 = nrm2;
+  sc->m_used = k + 1;
+  sc->aux = nrm;
+  bool done = true;
+  if (!isfinite(nrm) || !isfinite(gk1)) {
+    sc->nonfinite = 1;
+  } else if (bd) {
+    sc->breakdown = 1;
+  } else {
+    done = tol_rel > 0.0 && fabs(gk1) < tol_rel * beta;
+  }
+  if (done) sc->done = 1;
+  return done;
+}
+
+__global__ void __launch_bounds__(AT, 1) k_arnoldi_step(ArnStep p, ArnState st, KScal* sc) {
+  extern __shared__ double dsm[];
+  const int kp1 = p.kp1, k = kp1 - 1, G = gridDim.x, g = blockIdx.x, tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  const int kq = (kp1 + 3) & ~3;   // columns in groups of four
+  double* sh = dsm;                // [kq] the pass's coefficients
+  double* hc = sh + kq;            // [kq] their sum over the passes: the Hessenberg column
+  double* scs = hc + kq;           // [kq] previous rotations
+  double* ssn = scs + kq;          // [kq]
+  double* sdot = ssn + kq;         // [A_SL][kq] this CTA's dot products
+  double* sw = sdot + A_SL * kq;   // [A_SUB] staged rows of w
+  double* sred = sw + A_SUB;       // [AT] partial sums
+  float* shf = reinterpret_cast<float*>(sred + AT);  // [kq] coefficients in FP32
+  float* spart = shf + kq;                           // [AT] partial sums of the updates
+  __shared__ int s_abort;
+  __shared__ double s_fin[3];
+  if (sc->done) {
+    if (g == 0 && tid == 0 && p.hdone) *p.hdone = 1;
+    return;
+  }
+  if (tid == 0) s_abort = 0;
+  const long long r0 = (long long)g * p.R;
+  const int rows = (int)max(0LL, min((long long)p.R, p.n - r0));
+  double gk = 0.0, beta = 0.0;
+  if (g == 0) {
+    for (int j = tid; j < k; j += AT) {
+      scs[j] = st.cs[j];
+      ssn[j] = st.sn[j];
+    }
+    if (tid == 0) {
+      gk = st.g[k];
+      beta = sc->beta;
+    }
+  }
+
+  auto barrier_arrive = [&](int b) {
+    __syncthreads();
+    if (tid == 0) {
+      // no CTA can be at the last barrier yet: this launch starts with it at zero
+      if (b == 0 && g == 0) p.bar[2] = 0u;
+      arn_arrive(p.bar + b);
+    }
+  };
+  auto barrier_wait = [&](int b) {
+    if (tid == 0) {
+      bool ok = false;
+      for (long long it = 0; it < ARN_WAIT; ++it) {
+        if (arn_ld_acquire(p.bar + b) >= (unsigned)G) { ok = true; break; }
+        if (it > 256) __nanosleep(32);
+      }
+      if (!ok) {
+        s_abort = 1;
+        sc->timeout = 1;
+        sc->done = 1;
+      }
+    }
+    __syncthreads();
+    return s_abort == 0;
+  };
+  // w of rows [s0, s0 + len) is staged in sw: add V^T w to sdot.  A warp takes
+  // four columns of one row slice.
+  auto dots = [&](int s0, int len) {
+    const int groups = kq / 4;
+    const int sl = groups * 4 <= AT / 32 ? 4 : groups * 2 <= AT / 32 ? 2 : 1;
+    for (int t = warp; t < groups * sl; t += AT / 32) {
+      const int q = t % sl, j0 = 4 * (t / sl);
+      const float* v = p.V + r0 + s0 + (long long)j0 * p.ldv;
+      double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+      for (int i = lane + 32 * q; i < len; i += 32 * sl) {
+        const double x = sw[i];
+        double y[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) y[u] = j0 + u < kp1 ? widen_f32(v[(long long)u * p.ldv + i]) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] = fma(y[u], x, acc[u]);
+      }
+      // lanes 0-7 end with column 0, 8-15 with 1, 16-23 with 2, 24-31 with 3
+      const bool up = lane & 16;
+      double b0 = (up ? acc[2] : acc[0]) + __shfl_xor_sync(0xffffffffu, up ? acc[0] : acc[2], 16);
+      double b1 = (up ? acc[3] : acc[1]) + __shfl_xor_sync(0xffffffffu, up ? acc[1] : acc[3], 16);
+      const bool odd = lane & 8;
+      double c = (odd ? b1 : b0) + __shfl_xor_sync(0xffffffffu, odd ? b0 : b1, 8);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+      if ((lane & 7) == 0) sdot[q * kq + j0 + (lane >> 3)] += c;
+    }
+  };
+  auto clear_dots = [&]() {
+    for (int j = tid; j < A_SL * kq; j += AT) sdot[j] = 0.0;
+  };
+  auto publish_dots = [&](double* out) {
+    __syncthreads();
+    for (int j = tid; j < kp1; j += AT)
+      out[(long long)g * kp1 + j] = (sdot[j] + sdot[kq + j]) + (sdot[2 * kq + j] + sdot[3 * kq + j]);
+  };
+  // sh[j] = sum over the CTAs of their dot products: column j by sixteen threads
+  // that take every sixteenth CTA, then pairwise
+  auto sum_dots = [&](const double* in) {
+    constexpr int Q = 16, C = AT / Q;
+    for (int j0 = 0; j0 < kp1; j0 += C) {
+      const int j = j0 + tid % C, q = tid / C;
+      double t = 0.0;
+      if (j < kp1) {
+#pragma unroll 4
+        for (int b = q; b < G; b += Q) t += __ldcg(in + (long long)b * kp1 + j);
+      }
+      sred[tid] = t;
+      __syncthreads();
+      if (q == 0 && j < kp1) {
+        double v[Q];
+#pragma unroll
+        for (int u = 0; u < Q; ++u) v[u] = sred[u * C + tid];
+#pragma unroll
+        for (int o = Q / 2; o > 0; o >>= 1)
+#pragma unroll
+          for (int u = 0; u < o; ++u) v[u] += v[u + o];
+        sh[j] = v[0];
+        shf[j] = (float)v[0];
+      }
+      __syncthreads();
+    }
+  };
+  // w -= V h on rows [s0, s0 + len); cg threads share a row's columns.  The
+  // new w is staged in sw; returns the thread's sum of squares.
+  auto update = [&](int s0, int len) {
+    const int cg = len <= 64 ? 8 : len <= 128 ? 4 : len <= 256 ? 2 : 1;
+    const int rp = AT / cg, r = tid % rp, q = tid / rp;
+    double sq = 0.0;
+    for (int i0 = 0; i0 < len; i0 += rp) {
+      const int i = i0 + r;
+      float acc = 0.f;
+      if (i < len) {
+        const float* v = p.V + r0 + s0 + i;
+#pragma unroll 4
+        for (int j = q; j < kp1; j += cg) acc = fmaf(v[(long long)j * p.ldv], shf[j], acc);
+      }
+      if (cg > 1) {
+        spart[tid] = acc;
+        __syncthreads();
+        if (q == 0)
+          for (int u = 1; u < cg; ++u) acc += spart[u * rp + r];
+      }
+      if (q == 0 && i < len) {
+        float* wp = p.w + r0 + s0 + i;
+        const float nw = *wp - acc;
+        *wp = nw;
+        const double x = (double)nw;
+        sw[i] = x;
+        sq = fma(x, x, sq);
+      }
+      if (cg > 1) __syncthreads();
+    }
+    return sq;
+  };
+
+  double* parts1 = p.parts;
+  double* parts2 = parts1 + (long long)G * kp1;
+  double* sqs = parts2 + (long long)G * kp1;
+  // first pass: h = V^T w
+  clear_dots();
+  for (int s0 = 0; s0 < rows; s0 += A_SUB) {
+    const int len = min(A_SUB, rows - s0);
+    __syncthreads();
+    for (int i = tid; i < len; i += AT) sw[i] = (double)p.w[r0 + s0 + i];
+    __syncthreads();
+    dots(s0, len);
+  }
+  publish_dots(parts1);
+  barrier_arrive(0);
+  if (!barrier_wait(0)) return;
+  sum_dots(parts1);
+  for (int j = tid; j < kp1; j += AT) hc[j] = sh[j];
+  if (p.passes >= 2) {
+    // w -= V h, second pass: h2 = V^T w
+    clear_dots();
+    for (int s0 = 0; s0 < rows; s0 += A_SUB) {
+      const int len = min(A_SUB, rows - s0);
+      __syncthreads();
+      update(s0, len);
+      __syncthreads();
+      dots(s0, len);
+    }
+    publish_dots(parts2);
+    barrier_arrive(1);
+    if (!barrier_wait(1)) return;
+    sum_dots(parts2);
+    for (int j = tid; j < kp1; j += AT) hc[j] += sh[j];
+  }
+  // the last update and ||w||^2
+  double sq = 0.0;
+  for (int s0 = 0; s0 < rows; s0 += A_SUB) {
+    __syncthreads();
+    sq += update(s0, min(A_SUB, rows - s0));
+  }
+  sq = block_sum(sq, sred);
+  if (tid == 0) sqs[g] = sq;
+  barrier_arrive(2);
+  // while the others arrive: the previous rotations of the new column
+  if (g == 0 && warp == 0) arnoldi_rotate(hc, scs, ssn, k);
+  if (!barrier_wait(2)) return;
+  // (everyone has left the first two barriers)
+  if (tid == 0 && g == 0) p.bar[0] = p.bar[1] = 0u;
+  if (warp == 0) {
+    double t = 0.0;
+    for (int b = lane; b < G; b += 32) t += __ldcg(sqs + b);
+    t = warp_sum(t);
+    // lane 0: 1 / sqrt(a^2 + ||w||^2), lane 1: 1 / ||w||, by the same instructions
+    const double a = g == 0 && lane == 0 ? hc[k] : 0.0;
+    const double x = fma(a, a, t);
+    const double rs = x > 0.0 ? rsqrt(x) : 0.0;
+    if (lane < 2) s_fin[1 + lane] = rs;
+    if (lane == 0) s_fin[0] = t;
+  }
+  __syncthreads();
+  const double nrm2 = s_fin[0], ninv = s_fin[2];
+  const double nrm = nrm2 > 0.0 ? nrm2 * ninv : nrm2;
+  if (nrm > 1e-12 && isfinite(nrm)) {
+    const float inv = (float)ninv;
+    for (int i = tid; i < rows; i += AT) p.vnext[r0 + i] = p.w[r0 + i] * inv;
+  }
+  if (g == 0) {
+    for (int j = tid; j < k; j += AT) st.H[j + k * st.ldh] = hc[j];
+    if (tid == 0) {
+      const bool done = arnoldi_finish(sc, st, k, hc[k], nrm2, nrm, s_fin[1], gk, beta, p.tol_rel);
+      if (p.hdone) *p.hdone = done;
+    }
   }
 }
 
-// V[:, k+1] = w * (1 / ||w||)  (mpdok_ooc.py:279).
-__global__ void k_normalize(const float* __restrict__ w, float* __restrict__ vnext, long long n, const KScal* sc) {
-  if (sc->done) return;
-  const float inv = (float)(1.0 / sc->aux);
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    vnext[i] = w[i] * inv;
+static size_t arnoldi_smem(int kp1) {
+  const int kq = (kp1 + 3) & ~3;
+  return (size_t)((4 + A_SL) * kq + A_SUB + AT) * sizeof(double) + (size_t)(kq + AT) * sizeof(float);
 }
 
 // dst = (float) src with ||dst||^2, then the cycle state: beta, g[0], flags.
@@ -221,16 +442,28 @@ __global__ void k_scale_v0(float* __restrict__ v, long long n, const KScal* sc) 
     v[i] *= inv;
 }
 
-// y = H(0:m,0:m)^{-1} g(0:m) by back substitution (mpdok_ooc.py:303-307).
-__global__ void k_backsub(const KScal* sc, ArnState st) {
-  if (threadIdx.x != 0) return;
+// y = H(0:m,0:m)^{-1} g(0:m) by back substitution (mpdok_ooc.py:303-307), one
+// block, column by column; the triangle of up to 64 columns sits in shared
+// memory (m = 50: 48 us; 144 us by one thread walking rows of H in global
+// memory).
+constexpr int BS_M = 64;
+__global__ void __launch_bounds__(KT) k_backsub(const KScal* sc, ArnState st) {
+  __shared__ double sH[BS_M * BS_M];
+  __shared__ double s[KMAX_RESTART];
   const int m = sc->m_used;
-  const long long ldh = st.ldh;
+  const bool staged = m <= BS_M;
+  const double* H = staged ? sH : st.H;
+  const long long ldh = staged ? m : st.ldh;
+  if (staged)
+    for (int e = threadIdx.x; e < m * m; e += KT) sH[e] = st.H[e % m + (long long)(e / m) * st.ldh];
+  for (int l = threadIdx.x; l < m; l += KT) s[l] = st.g[l];
+  __syncthreads();
   for (int j = m - 1; j >= 0; --j) {
-    double s = st.g[j];
-    for (int l = j + 1; l < m; ++l) s -= st.H[j + l * ldh] * st.y[l];
-    const double d = st.H[j + j * ldh];
-    st.y[j] = (d != 0.0) ? s / d : 0.0;
+    const double d = H[j + j * ldh];
+    const double y = (d != 0.0) ? s[j] / d : 0.0;
+    if (threadIdx.x == 0) st.y[j] = y;
+    for (int l = threadIdx.x; l < j; l += KT) s[l] -= H[l + j * ldh] * y;
+    __syncthreads();
   }
 }
 
@@ -579,12 +812,10 @@ KWs krylov_layout(long long n, int m, void* base) {
   ws.n = n;
   ws.m = m;
   ws.ldv = (long long)align_up((size_t)std::max(1LL, n), 64);
-  const long long nsm = num_sms();
-  long long ch = (n + 2 * nsm - 1) / (2 * nsm);
-  ch = (long long)align_up((size_t)std::max(1LL, ch), 256);
-  ch = std::min(std::max(ch, 256LL), 4096LL);
-  ws.ch = ch;
-  ws.nblk = (int)std::max(1LL, (n + ch - 1) / ch);
+  // (at most one CTA per SM, so that a cooperative launch always fits)
+  const long long gmax = std::min<long long>(num_sms(), n <= 16384 ? 64 : 128);
+  ws.ch = std::max(64LL, (long long)align_up((size_t)((n + gmax - 1) / gmax), 8));
+  ws.nblk = (int)std::max(1LL, (n + ws.ch - 1) / ws.ch);
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
   const size_t fv = (size_t)ws.ldv * sizeof(float);
@@ -592,9 +823,8 @@ KWs krylov_layout(long long n, int m, void* base) {
   size_t oV = take(fv * (m + 1)), ow = take(fv), ox = take(fv), ob = take(fv), op = take(fv), oq = take(fv);
   size_t or64 = take(dv), ox64 = take(dv), oe64 = take(dv * 2);
   size_t oH = take(sizeof(double) * (size_t)(m + 1) * m), ocs = take(sizeof(double) * m),
-         osn = take(sizeof(double) * m), og = take(sizeof(double) * (m + 1)), oy = take(sizeof(double) * m),
-         oh2 = take(sizeof(double) * (m + 1));
-  const size_t nparts = (size_t)std::max<long long>(ws.nblk, vec_blocks(n)) * (m + 1) + 64;
+         osn = take(sizeof(double) * m), og = take(sizeof(double) * (m + 1)), oy = take(sizeof(double) * m);
+  const size_t nparts = std::max((size_t)vec_blocks(n), (size_t)ws.nblk * (2 * (size_t)(m + 1) + 1)) + 64;
   size_t oparts = take(sizeof(double) * nparts);
   size_t otk = take(sizeof(unsigned) * 8);
   size_t osc = take(sizeof(KScal));
@@ -607,7 +837,7 @@ KWs krylov_layout(long long n, int m, void* base) {
     ws.p32 = (float*)(b + op); ws.q32 = (float*)(b + oq);
     ws.r64 = (double*)(b + or64); ws.x64t = (double*)(b + ox64); ws.e64 = (double*)(b + oe64);
     ws.H = (double*)(b + oH); ws.cs = (double*)(b + ocs); ws.sn = (double*)(b + osn); ws.g = (double*)(b + og);
-    ws.y = (double*)(b + oy); ws.h2 = (double*)(b + oh2); ws.parts = (double*)(b + oparts);
+    ws.y = (double*)(b + oy); ws.parts = (double*)(b + oparts);
     ws.tickets = (unsigned*)(b + otk); ws.sc = (KScal*)(b + osc); ws.gw = (void*)(b + ogw);
   }
   return ws;
@@ -654,6 +884,10 @@ Residual64 stored_res64(const StoredCtx* c) {
 int read_scal(const KWs& ws, KScal* host, cudaStream_t s) {
   MPDOK_CUDA_TRY(cudaMemcpyAsync(host, ws.sc, sizeof(KScal), cudaMemcpyDeviceToHost, s));
   MPDOK_CUDA_TRY(cudaStreamSynchronize(s));
+  if (host->timeout != 0) {
+    set_error("Arnoldi step: the grid barrier wait ran out");
+    return MPDOK_ERR_TIMEOUT;
+  }
   return MPDOK_OK;
 }
 
@@ -678,7 +912,8 @@ static int cycle_start_from_f32(const KWs& ws, const float* src32, cudaStream_t 
 }
 
 // Host copies of a cycle's done flag, two slots per host thread and device
-// (pinned, so the copy is asynchronous) with the events that mark them written.
+// (pinned: the steps write them themselves, a copy between the steps costs a
+// hand-off to the copy engine) with the events that mark them written.
 struct DoneProbe {
   int* flag = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -695,8 +930,7 @@ int arnoldi_cycle(const KWs& ws, const Operator32& A, int m, int reorth, double 
                   float* x32, double* x64, cudaStream_t s) {
   const long long n = ws.n;
   const ArnState st = arn_state(ws);
-  const size_t smem_dots = (size_t)ws.ch * sizeof(float);
-  const size_t smem_apply = (size_t)(KMAX_RESTART + 1 + ws.ch) * sizeof(float);
+  MPDOK_TRY(set_smem(k_arnoldi_step, arnoldi_smem(m)));
   // Every kernel of an iteration is predicated on the device done flag, so
   // the cycle may be queued whole; but a predicated-off iteration still costs
   // its launches (~75 us at N = 32768, a preconditioned cycle converges in a
@@ -715,7 +949,7 @@ int arnoldi_cycle(const KWs& ws, const Operator32& A, int m, int reorth, double 
   for (int k = 0; k < m; ++k) {
     if (poll && k >= 2) {
       MPDOK_CUDA_TRY(cudaEventSynchronize(pp->ev[k & 1]));  // the flag after iteration k - 2
-      if (pp->flag[k & 1]) break;
+      if (*(volatile int*)&pp->flag[k & 1]) break;
     }
     const float* vk = ws.V + (long long)k * ws.ldv;
     const float* opnd = vk;
@@ -725,25 +959,18 @@ int arnoldi_cycle(const KWs& ws, const Operator32& A, int m, int reorth, double 
       opnd = zk;
     }
     MPDOK_TRY(A.apply(A.ctx, opnd, ws.w, 1, ws.ldv, s, &ws.sc->done));
-    double* Hcol = ws.H + (long long)k * st.ldh;
-    launch(k_dots, ws.nblk, KT, smem_dots, s, ws.V, ws.ldv, k + 1, ws.w, n, ws.ch, ws.parts, ws.tickets + 0, Hcol, ws.sc);
-    if (reorth >= 2) {
-      launch(k_apply<0>, ws.nblk, KT, smem_apply, s, ws.V, ws.ldv, k + 1, ws.w, n, ws.ch, Hcol, ws.parts, ws.tickets + 1,
-                                                  ws.h2, Hcol, ws.sc, st, k, tol_rel);
-      launch(k_apply<1>, ws.nblk, KT, smem_apply, s, ws.V, ws.ldv, k + 1, ws.w, n, ws.ch, ws.h2, ws.parts,
-                                                  ws.tickets + 2, nullptr, nullptr, ws.sc, st, k, tol_rel);
-    } else {
-      launch(k_apply<1>, ws.nblk, KT, smem_apply, s, ws.V, ws.ldv, k + 1, ws.w, n, ws.ch, Hcol, ws.parts,
-                                                  ws.tickets + 2, nullptr, nullptr, ws.sc, st, k, tol_rel);
-    }
-    launch(k_normalize, vec_blocks(n), KT, 0, s, ws.w, ws.V + (long long)(k + 1) * ws.ldv, n, ws.sc);
+    ArnStep step{ws.V, ws.ldv, k + 1, ws.w, ws.V + (long long)(k + 1) * ws.ldv, n, (int)ws.ch, ws.parts, ws.tickets,
+                 tol_rel, reorth, poll ? &pp->flag[k & 1] : nullptr};
+    ArnState state = st;
+    KScal* sc = ws.sc;
+    void* args[] = {&step, &state, &sc};
+    MPDOK_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_arnoldi_step, dim3(ws.nblk), dim3(AT), args,
+                                               arnoldi_smem(k + 1), s));
+    count_launch();
     MPDOK_LAUNCH_CHECK("arnoldi step");
-    if (poll) {
-      MPDOK_CUDA_TRY(cudaMemcpyAsync(&pp->flag[k & 1], &ws.sc->done, sizeof(int), cudaMemcpyDeviceToHost, s));
-      MPDOK_CUDA_TRY(cudaEventRecord(pp->ev[k & 1], s));
-    }
+    if (poll) MPDOK_CUDA_TRY(cudaEventRecord(pp->ev[k & 1], s));
   }
-  launch(k_backsub, 1, 32, 0, s, ws.sc, st);
+  launch(k_backsub, 1, KT, 0, s, ws.sc, st);
   if (pc && pc->apply && pc->Z) {
     // x += M^{-1} V y = Z y
     if (x64) launch(k_update<double>, vec_blocks(n), KT, 0, s, (const float*)pc->Z, pc->ldz, ws.y, ws.sc, n, x64, nullptr);

@@ -16,6 +16,7 @@ struct KScal {
   int m_used;       // Arnoldi steps completed in the current cycle
   int breakdown;    // |w| <= 1e-12 met
   int nonfinite;    // NaN / Inf seen in a device scalar
+  int timeout;      // a grid barrier of an Arnoldi step ran out (kept until the next solve)
 };
 
 // Workspace carve-up for a Krylov solve of size n with restart m.
@@ -24,14 +25,14 @@ struct KWs {
   int m = 0;
   float *V = nullptr, *w = nullptr, *x32 = nullptr, *b32 = nullptr, *p32 = nullptr, *q32 = nullptr;
   double *r64 = nullptr, *x64t = nullptr, *e64 = nullptr;
-  double *H = nullptr, *cs = nullptr, *sn = nullptr, *g = nullptr, *y = nullptr, *h2 = nullptr;
+  double *H = nullptr, *cs = nullptr, *sn = nullptr, *g = nullptr, *y = nullptr;
   double* parts = nullptr;
   unsigned* tickets = nullptr;  // 8 independent tickets
   KScal* sc = nullptr;
   void* gw = nullptr;
   size_t gbytes = 0;
-  int nblk = 1;       // blocks of the row-chunked vector kernels
-  long long ch = 256; // rows per block of those kernels
+  int nblk = 1;       // blocks of an Arnoldi step
+  long long ch = 64;  // rows per block of an Arnoldi step
   size_t total = 0;
 };
 
