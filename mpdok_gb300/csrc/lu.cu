@@ -351,17 +351,6 @@ __device__ __forceinline__ void diag32_column(const float* __restrict__ Tb, floa
   }
 }
 
-// Into shared memory: entry (r, c) of the inverses at XL / XU[r * DP + c].
-__device__ __forceinline__ void diag32_inverses_smem(const float* T, float* XL, float* XU) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp >= 8) return;  // idle during the 32 x 32 substitutions
-  const int o = (warp & 3) * 32;
-  if (warp < 4)
-    diag32_column<true>(T + o * DP + o, XL + o * DP + o + lane, DP, lane);
-  else
-    diag32_column<false>(T + o * DP + o, XU + o * DP + o + lane, DP, lane);
-}
-
 // Into global memory, column-major with pitch ld, through a staging area of
 // 32 x 33 floats per warp: each warp writes its block column by column in
 // 128-byte runs.
@@ -380,22 +369,6 @@ __device__ __forceinline__ void diag32_inverses_global(const float* T, float* Li
 #pragma unroll 4
   for (int c = 0; c < 32; ++c) X[(o + lane) + (long long)(o + c) * ld] = st[lane * 33 + c];
 }
-
-// Inverses by recursive doubling: the 32 x 32 diagonal blocks by substitution,
-// then
-//   [X11 0; L21 X22]^-1 off-diagonal block = -X22 L21 X11,
-//   [X11 U12; 0 X22]^-1 off-diagonal block = -X11 U12 X22,
-// for block sizes 32 and 64, each product spread over all 1024 threads.
-__device__ void tri_inverses(const float* T, float* XL, float* XU, float* Tmp) {
-  const int tid = threadIdx.x;
-  for (int idx = tid; idx < LNB * DP; idx += blockDim.x) { XL[idx] = 0.f; XU[idx] = 0.f; }
-  __syncthreads();
-  diag32_inverses_smem(T, XL, XU);
-  __syncthreads();
-  inverse_doubling<32>(T, XL, XU, Tmp);
-  inverse_doubling<64>(T, XL, XU, Tmp);
-}
-
 
 // Unpivoted LU of the 128 x 128 diagonal block, blocked in four 32-column
 // sub-panels with the block in shared memory (T, pitch DP).  For sub-panel p:
@@ -608,8 +581,11 @@ k_lu_diag(float* __restrict__ W, long long ldw, long long j0, int nbk, F* __rest
 
 // The full 128 x 128 inverses of every diagonal block (for the triangular
 // solves of the preconditioner) from W's factored diagonal blocks and the
-// 32 x 32 diagonal-block inverses that k_lu_diag left in Linv / Uinv: the
-// doubling steps of tri_inverses, one CTA per block.
+// 32 x 32 diagonal-block inverses that k_lu_diag or k_piv_diag left in Linv /
+// Uinv, one CTA per block, by recursive doubling:
+//   [X11 0; L21 X22]^-1 off-diagonal block = -X22 L21 X11,
+//   [X11 U12; 0 X22]^-1 off-diagonal block = -X11 U12 X22,
+// for block sizes 32 and 64, each product spread over all 1024 threads.
 __global__ void __launch_bounds__(DIAG_THREADS, 1)
 k_tri_inv_complete(const float* __restrict__ W, long long ldw, long long n, float* __restrict__ Linv,
                    float* __restrict__ Uinv) {
@@ -1306,11 +1282,12 @@ __global__ void k_scale_out_multi(const float* __restrict__ z, const float* __re
 // power-of-two row and column scales (W = Dr A Dc, exact, |W| <= 1 in every
 // row and column, which keeps 16-bit operands in range), then factored
 // right-looking in 128-column panels:
-//   1. k_getf2: the tall panel W[jp:n, jp:jp+128] with partial pivoting on G
-//      co-resident CTAs, each holding a slice of its rows in shared memory;
-//      one grid barrier per column (pivot search, row exchange, rank-1 update);
+//   1. k_getf2_cluster (up to 6144 rows) or k_getf2: the tall panel
+//      W[jp:n, jp:jp+128] with partial pivoting on one cluster or on G
+//      co-resident CTAs, each holding a slice of its rows in shared memory; one
+//      barrier per column (pivot search, row exchange, rank-1 update);
 //   2. k_laswp: the panel's row exchanges applied to every other column of W;
-//   3. k_piv_diag: the 128 x 128 diagonal block's unit-lower / upper inverses;
+//   3. k_piv_diag: the inverses of the diagonal block's 32 x 32 diagonal blocks;
 //   4. U12 = L11^-1 W12 (the panel solve of the unpivoted path), L21 to the
 //      K-major operand, and W22 -= L21 U12 on the tensor cores;
 // and at the end the strictly lower part of W is rounded into the factor.
@@ -1410,6 +1387,302 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
+}
+
+// The panel's exchanges (s_piv[k]: the row exchanged with jp + k) as row moves:
+// position jp + k receives the content that the exchanges leave there (one warp
+// replays them).
+__device__ void piv_moves(const int* s_piv, long long jp, int nb, int* plan) {
+  const int tid = threadIdx.x;
+  int* cnt = plan;
+  int* dst = plan + 1;
+  int* src = plan + 1 + 2 * LNB;
+  __shared__ int s_in[LNB];        // content of positions jp .. jp + nb - 1
+  __shared__ int s_key[LNB], s_val[LNB];
+  __shared__ int s_nout;
+  for (int k = tid; k < nb; k += 32) s_in[k] = (int)(jp + k);
+  if (tid == 0) s_nout = 0;
+  __syncwarp();
+  for (int k = 0; k < nb; ++k) {
+    const int p = s_piv[k];
+    if (p == (int)(jp + k)) continue;
+    if (p < jp + nb) {
+      if (tid == 0) {
+        const int t = s_in[k];
+        s_in[k] = s_in[p - jp];
+        s_in[p - jp] = t;
+      }
+    } else {
+      // find p among the rows outside the panel moved so far
+      int found = -1;
+      const int nout = s_nout;
+      for (int b = 0; b < nout; b += 32) {
+        const unsigned m = __ballot_sync(0xffffffffu, b + tid < nout && s_key[b + tid] == p);
+        if (m) { found = b + __ffs(m) - 1; break; }
+      }
+      if (tid == 0) {
+        if (found >= 0) {
+          const int t = s_in[k];
+          s_in[k] = s_val[found];
+          s_val[found] = t;
+        } else {
+          s_key[nout] = p;
+          s_val[nout] = s_in[k];
+          s_in[k] = p;
+          s_nout = nout + 1;
+        }
+      }
+    }
+    __syncwarp();
+  }
+  if (tid == 0) {
+    int c = 0;
+    for (int k = 0; k < nb; ++k)
+      if (s_in[k] != (int)(jp + k)) { dst[c] = (int)(jp + k); src[c] = s_in[k]; ++c; }
+    for (int t = 0; t < s_nout; ++t)
+      if (s_val[t] != s_key[t]) { dst[c] = s_key[t]; src[c] = s_val[t]; ++c; }
+    *cnt = c;
+  }
+}
+
+// ---- the same panel factorization inside one thread-block cluster
+// Up to 16 CTAs (384 rows each, one thread to a row) hold the panel in shared
+// memory and meet at one hardware cluster barrier per column; candidates and
+// rows travel through distributed shared memory.  Panels of up to 6144 rows
+// take it: a column costs about 1.5 us against 4.7 us behind a grid barrier in
+// global memory (n = 5000: 9.5 against 24.2 ms for the 40 panels, 238 against
+// 604 us each).  Taller ones do not fit a cluster's shared memory and take
+// k_getf2.
+//
+// Columns are worked off in sub-panels of 32: a thread holds its row's 32
+// entries in registers, shifted left by one per step so that the loop stays
+// rolled (its code is fetched from L2 on every launch), and the columns right of
+// the sub-panel receive its 32 steps at once.  Every entry gets the FMAs of
+// k_getf2 in the same order, so the two give the same bits.
+constexpr int CL_THREADS = 512;
+constexpr int CL_RMAX = 384;
+constexpr int CL_MAX = 16;
+constexpr int CL_SUB = 32;
+
+__host__ __device__ constexpr size_t getf2_cluster_smem(int R) {
+  return ((size_t)LNB * (R + 1) + (LNB - CL_SUB) * CL_SUB + 6 * CL_SUB + 6 * LNB) * sizeof(float);
+}
+
+__device__ __forceinline__ unsigned cl_map(const void* p, unsigned rank) {
+  unsigned a = static_cast<unsigned>(__cvta_generic_to_shared(p)), r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float cl_ld(unsigned a) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cl_st(unsigned a, unsigned long long v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+// every thread of every CTA of the cluster; releases and acquires shared memory
+__device__ __forceinline__ void cl_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(CL_THREADS, 1)
+k_getf2_cluster(float* __restrict__ W, long long ldw, long long n, long long jp, int nb, int R,
+                int* __restrict__ ipiv, int* info, int* plan) {
+  extern __shared__ __align__(16) float csm[];
+  float* Us = csm;                                  // [LNB - 32][32]: a sub-panel's U rows, by column
+  // rows in transit: the entries j .. of the sub-panel as 32 aligned floats (c..),
+  // the columns outside the sub-panel at their own places
+  float* csub = Us + (LNB - CL_SUB) * CL_SUB;       // [2][32]: this CTA's candidate
+  float* tsub = csub + 2 * CL_SUB;                  // [2][32]: the row at position j (CTA 0)
+  float* s_v = tsub + 2 * CL_SUB;                   // [32]: the pivot row
+  float* s_w = s_v + CL_SUB;                        // [32]: the row that it replaces
+  float* crow = s_w + CL_SUB;                       // [2][LNB]: this CTA's candidate
+  float* top = crow + 2 * LNB;                      // [2][LNB]: the row at position j (CTA 0)
+  float* s_u = top + 2 * LNB;                       // [LNB]: the pivot row
+  float* s_t = s_u + LNB;                           // [LNB]: the row that it replaces
+  float* P = s_t + LNB;                             // [nb][RS]: this CTA's rows
+  const int RS = R + 1;                             // (odd: rows and columns both conflict-free)
+  __shared__ unsigned long long cand[2][CL_MAX];
+  __shared__ unsigned s_key[CL_THREADS / 32];
+  __shared__ int s_row[CL_THREADS / 32];
+  __shared__ int corg[2], torg[2], s_org[2];  // where the rows in transit came from: candidate, position j; as read
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int C = gridDim.x, g = blockIdx.x;
+  const int rows = (int)max(0LL, min((long long)R, n - jp - (long long)g * R));
+  const int pos = g * R + t;                        // this thread's position in the panel
+  const bool mine = t < rows;
+  int org = pos;                                    // the position this thread's row came from
+  if (g == 0 && t == 0) plan[0] = 0;
+  for (int e = t; e < nb * R; e += CL_THREADS) {
+    const int c = e / R, r = e % R;
+    P[c * RS + r] = r < rows ? W[(jp + pos - t + r) + (jp + c) * ldw] : 0.f;
+  }
+  __syncthreads();
+  for (int s0 = 0; s0 < nb; s0 += CL_SUB) {
+    const int se = min(s0 + CL_SUB, nb);
+    float x[CL_SUB];  // columns j .. of this row (zero or unused past the sub-panel)
+#pragma unroll
+    for (int c = 0; c < CL_SUB; ++c) x[c] = mine && s0 + c < se ? P[(s0 + c) * RS + t] : 0.f;
+#pragma unroll 1
+    for (int j = s0; j < se; ++j) {
+      const int q = j & 1;
+      // this CTA's candidate: the largest |x|, ties to the smaller row (NaN is
+      // never taken); 0: no eligible row, 1: an exact zero
+      unsigned key = 0;
+      if (mine && pos >= j && x[0] == x[0]) key = (__float_as_uint(x[0]) & 0x7fffffffu) + 1u;
+      unsigned m = __reduce_max_sync(0xffffffffu, key);
+      unsigned bal = __ballot_sync(0xffffffffu, key == m);
+      if (lane == 0) {
+        s_key[warp] = m;
+        s_row[warp] = warp * 32 + __ffs(bal) - 1;
+      }
+      __syncthreads();
+      key = lane < CL_THREADS / 32 ? s_key[lane] : 0;
+      m = __reduce_max_sync(0xffffffffu, key);
+      bal = __ballot_sync(0xffffffffu, lane < CL_THREADS / 32 && key == m);
+      const int lw = s_row[__ffs(bal) - 1];
+      // publish the candidate's row and the row at position j
+      const bool outside = t < nb && (t < j || t >= se);
+      if (t == lw || (g == 0 && t == j)) {
+        float4 v[CL_SUB / 4];
+#pragma unroll
+        for (int c = 0; c < CL_SUB; c += 4) v[c / 4] = make_float4(x[c], x[c + 1], x[c + 2], x[c + 3]);
+        float4* a = reinterpret_cast<float4*>(csub + q * CL_SUB);
+        float4* b = reinterpret_cast<float4*>(tsub + q * CL_SUB);
+        if (t == lw)
+#pragma unroll
+          for (int c = 0; c < CL_SUB / 4; ++c) a[c] = v[c];
+        if (t == lw) corg[q] = org;
+        if (g == 0 && t == j) {
+          torg[q] = org;
+#pragma unroll
+          for (int c = 0; c < CL_SUB / 4; ++c) b[c] = v[c];
+        }
+      }
+      if (outside) {
+        crow[q * LNB + t] = P[t * RS + lw];
+        if (g == 0) top[q * LNB + t] = P[t * RS + j];
+      }
+      if (t < C) cl_st(cl_map(&cand[q][g], t), ((unsigned long long)m << 32) | (unsigned)(g * R + lw));
+      cl_sync();
+      const unsigned long long cv = lane < C ? cand[q][lane] : 0ull;
+      key = (unsigned)(cv >> 32);
+      m = __reduce_max_sync(0xffffffffu, key);
+      bal = __ballot_sync(0xffffffffu, lane < C && key == m);
+      const int wc = __ffs(bal) - 1;
+      const int wr = __shfl_sync(0xffffffffu, (int)(unsigned)cv, wc);
+      if (outside) s_u[t] = cl_ld(cl_map(crow + q * LNB + t, wc));
+      else if (warp == 4) s_v[lane] = cl_ld(cl_map(csub + q * CL_SUB + lane, wc));
+      else if (warp == 5) s_w[lane] = cl_ld(cl_map(tsub + q * CL_SUB + lane, 0));
+      else if (warp == 6 && lane < 2)
+        s_org[lane] = __float_as_int(cl_ld(lane == 0 ? cl_map(corg + q, wc) : cl_map(torg + q, 0)));
+      else if (t >= 2 * LNB && t < 2 * LNB + nb) s_t[t - 2 * LNB] = cl_ld(cl_map(top + q * LNB + t - 2 * LNB, 0));
+      __syncthreads();
+      const bool zero = m <= 1u;
+      if (g == 0 && t == 0) {
+        ipiv[jp + j] = (int)jp + (zero ? j : wr);
+        // LAPACK records the first zero pivot and leaves the column
+        if (zero) atomicCAS(info, 0, (int)(jp + j + 1));
+      }
+      if (zero) {
+        if (mine && pos > j) P[j * RS + t] = x[0];
+        if (g == 0 && t == j) {
+#pragma unroll
+          for (int c = 0; c < CL_SUB; ++c)
+            if (c < se - j) P[(j + c) * RS + j] = x[c];
+        }
+#pragma unroll
+        for (int c = 0; c + 1 < CL_SUB; ++c) x[c] = x[c + 1];
+        continue;
+      }
+      if (g == 0 && t < nb) P[t * RS + j] = outside ? s_u[t] : s_v[t - j];
+      if (g == 0 && t == j) org = s_org[0];
+      if (wr != j && g == wc) {  // the winner's row takes the content of position j
+        const int l = wr - g * R;
+        if (outside) P[t * RS + l] = s_t[t];
+        if (t == l) {
+          org = s_org[1];
+          const float4* b = reinterpret_cast<const float4*>(s_w);
+#pragma unroll
+          for (int c = 0; c < CL_SUB; c += 4) {
+            const float4 v = b[c / 4];
+            x[c] = v.x, x[c + 1] = v.y, x[c + 2] = v.z, x[c + 3] = v.w;
+          }
+        }
+      }
+      if (mine && pos > j) {
+        float v[CL_SUB];
+        const float4* b = reinterpret_cast<const float4*>(s_v);
+#pragma unroll
+        for (int c = 0; c < CL_SUB; c += 4) {
+          const float4 u = b[c / 4];
+          v[c] = u.x, v[c + 1] = u.y, v[c + 2] = u.z, v[c + 3] = u.w;
+        }
+        const float l = x[0] * __frcp_rn(v[0]);
+        P[j * RS + t] = l;
+#pragma unroll
+        for (int c = 0; c + 1 < CL_SUB; ++c) x[c] = fmaf(-l, v[c + 1], x[c + 1]);
+      }
+    }
+    if (se < nb) {
+      // the sub-panel's rows of U in the columns to the right (CTA 0 holds them:
+      // R >= 128 where there is more than one CTA), a thread per column
+      __syncthreads();
+      if (g == 0 && t < nb - se) {
+        float u[CL_SUB];
+        float* col = P + (size_t)(se + t) * RS + s0;
+#pragma unroll
+        for (int i = 0; i < CL_SUB; ++i) u[i] = col[i];
+#pragma unroll 1
+        for (int k = 0; k + 1 < CL_SUB; ++k) {
+          const float uk = u[0];
+          col[k] = uk;
+          const float* Lk = P + (size_t)(s0 + k) * RS + s0 + k + 1;  // (rows past the sub-panel: unused)
+#pragma unroll
+          for (int i = 0; i + 1 < CL_SUB; ++i) u[i] = fmaf(-Lk[i], uk, u[i + 1]);
+        }
+        col[CL_SUB - 1] = u[0];
+      }
+      cl_sync();
+#pragma unroll 6
+      for (int e = t; e < (nb - se) * CL_SUB; e += CL_THREADS)
+        Us[e] = cl_ld(cl_map(P + (size_t)(se + e / CL_SUB) * RS + s0 + e % CL_SUB, 0));
+      __syncthreads();
+      if (mine && pos >= se) {
+        float l[CL_SUB];
+#pragma unroll
+        for (int k = 0; k < CL_SUB; ++k) l[k] = P[(s0 + k) * RS + t];
+#pragma unroll 2
+        for (int c = se; c < nb; ++c) {
+          float v = P[c * RS + t];
+          const float4* uc = reinterpret_cast<const float4*>(Us + (c - se) * CL_SUB);
+#pragma unroll
+          for (int k = 0; k < CL_SUB; k += 4) {
+            const float4 u4 = uc[k / 4];
+            v = fmaf(-l[k], u4.x, v);
+            v = fmaf(-l[k + 1], u4.y, v);
+            v = fmaf(-l[k + 2], u4.z, v);
+            v = fmaf(-l[k + 3], u4.w, v);
+          }
+          P[c * RS + t] = v;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  for (int e = t; e < nb * R; e += CL_THREADS) {
+    const int c = e / R, r = e % R;
+    if (r < rows) W[(jp + pos - t + r) + (jp + c) * ldw] = P[c * RS + r];
+  }
+  // the exchanges as row moves, in any order (at most two per column)
+  if (mine && org != pos) {
+    const int i = atomicAdd(plan, 1);
+    plan[1 + i] = (int)jp + pos;
+    plan[1 + 2 * LNB + i] = (int)jp + org;
+  }
+  cl_sync();  // no CTA leaves while another may still read its shared memory
 }
 
 constexpr int GETF2_THREADS = 512;
@@ -1532,59 +1805,7 @@ k_getf2(float* __restrict__ W, long long ldw, long long n, long long jp, int nb,
     const int c = e / R, r = e % R;
     if (r < rows) W[(rbeg + r) + (jp + c) * ldw] = P[e];
   }
-  // the panel's exchanges as row moves: position jp + k receives the content
-  // that the exchanges leave there (warp 0 of CTA 0 replays them)
-  if (g == 0 && tid < 32) {
-    int* cnt = plan;
-    int* dst = plan + 1;
-    int* src = plan + 1 + 2 * LNB;
-    __shared__ int s_in[LNB];        // content of positions jp .. jp + nb - 1
-    __shared__ int s_key[LNB], s_val[LNB];
-    __shared__ int s_nout;
-    for (int k = tid; k < nb; k += 32) s_in[k] = (int)(jp + k);
-    if (tid == 0) s_nout = 0;
-    __syncwarp();
-    for (int k = 0; k < nb; ++k) {
-      const int p = s_piv[k];
-      if (p == (int)(jp + k)) continue;
-      if (p < jp + nb) {
-        if (tid == 0) {
-          const int t = s_in[k];
-          s_in[k] = s_in[p - jp];
-          s_in[p - jp] = t;
-        }
-      } else {
-        // find p among the rows outside the panel moved so far
-        int found = -1;
-        const int nout = s_nout;
-        for (int b = 0; b < nout; b += 32) {
-          const unsigned m = __ballot_sync(0xffffffffu, b + tid < nout && s_key[b + tid] == p);
-          if (m) { found = b + __ffs(m) - 1; break; }
-        }
-        if (tid == 0) {
-          if (found >= 0) {
-            const int t = s_in[k];
-            s_in[k] = s_val[found];
-            s_val[found] = t;
-          } else {
-            s_key[nout] = p;
-            s_val[nout] = s_in[k];
-            s_in[k] = p;
-            s_nout = nout + 1;
-          }
-        }
-      }
-      __syncwarp();
-    }
-    if (tid == 0) {
-      int c = 0;
-      for (int k = 0; k < nb; ++k)
-        if (s_in[k] != (int)(jp + k)) { dst[c] = (int)(jp + k); src[c] = s_in[k]; ++c; }
-      for (int t = 0; t < s_nout; ++t)
-        if (s_val[t] != s_key[t]) { dst[c] = s_key[t]; src[c] = s_val[t]; ++c; }
-      *cnt = c;
-    }
-  }
+  if (g == 0 && tid < 32) piv_moves(s_piv, jp, nb, plan);
 }
 
 // The panel's row moves (dst <- src, all reads before all writes) applied to
@@ -1623,33 +1844,27 @@ k_laswp(float* __restrict__ W, long long ldw, const int* __restrict__ plan, long
   }
 }
 
-// Inverses of the factored diagonal block (unit-lower and upper triangles)
-// and the block itself rounded into the factor.
+// The factored diagonal block rounded into the factor and the inverses of its
+// 32 x 32 diagonal blocks, which is what the panel solve needs
+// (k_tri_inv_complete fills in the rest after the factorization; the full
+// inverses here took 46 us of every panel).
 template <typename F>
-__global__ void __launch_bounds__(DIAG_THREADS, 1)
+__global__ void __launch_bounds__(DIAG_LU_THREADS, 1)
 k_piv_diag(const float* __restrict__ W, long long ldw, long long j0, int nbk, F* __restrict__ LU, long long ldf,
            float* __restrict__ Linv, float* __restrict__ Uinv) {
   extern __shared__ float sm[];
   float* T = sm;
-  float* XL = sm + LNB * DP;
-  float* XU = sm + 2 * LNB * DP;
-  float* Tmp = sm + 3 * LNB * DP;
-  const int tid = threadIdx.x;
-  for (int idx = tid; idx < LNB * LNB; idx += DIAG_THREADS) {
+  float* stage = sm + LNB * DP;
+#pragma unroll 8
+  for (int idx = threadIdx.x; idx < LNB * LNB; idx += DIAG_LU_THREADS) {
     const int r = idx % LNB, c = idx / LNB;
-    T[r * DP + c] = (r < nbk && c < nbk) ? W[(j0 + r) + (j0 + c) * ldw] : (r == c ? 1.f : 0.f);
+    const bool in = r < nbk && c < nbk;
+    const float v = in ? W[(j0 + r) + (j0 + c) * ldw] : (r == c ? 1.f : 0.f);
+    T[r * DP + c] = v;
+    if (in) LU[(j0 + r) + (j0 + c) * ldf] = from_f32<F>(v);
   }
   __syncthreads();
-  for (int idx = tid; idx < nbk * nbk; idx += blockDim.x) {
-    const int r = idx % nbk, c = idx / nbk;
-    LU[(j0 + r) + (j0 + c) * ldf] = from_f32<F>(T[r * DP + c]);
-  }
-  tri_inverses(T, XL, XU, Tmp);
-  for (int idx = tid; idx < LNB * LNB; idx += blockDim.x) {
-    const int r = idx % LNB, c = idx / LNB;
-    Linv[c * LNB + r] = XL[r * DP + c];
-    Uinv[c * LNB + r] = XU[r * DP + c];
-  }
+  diag32_inverses_global(T, Linv, Uinv, LNB, stage);
 }
 
 // L21 (rows [r0, n) of the panel's columns in W) into the K-major operand
@@ -2166,6 +2381,63 @@ static int lu_factor_t(const double* A, long long lda, long long n, int fdtype, 
   return MPDOK_OK;
 }
 
+// Largest panel that k_getf2_cluster takes on the current device: CL_RMAX rows
+// per CTA of the largest cluster that can run (0: none).  Asked once per device
+// and host thread.
+static long long getf2_cluster_rows() {
+  constexpr int MAX_DEV = 64;
+  thread_local long long known[MAX_DEV] = {};  // rows + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEV) return 0;
+  if (known[dev] == 0) {
+    const size_t smem = getf2_cluster_smem(CL_RMAX);
+    int C = 0;
+    if (set_smem(k_getf2_cluster, smem) == MPDOK_OK &&
+        cudaFuncSetAttribute((const void*)k_getf2_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+            cudaSuccess) {
+      for (C = CL_MAX; C > 0; C /= 2) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        cfg.gridDim = dim3(C);
+        cfg.blockDim = dim3(CL_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = C;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, (const void*)k_getf2_cluster, &cfg) == cudaSuccess && fit >= 1) break;
+      }
+    }
+    cudaGetLastError();  // (what does not fit is not an error of the caller's)
+    known[dev] = (long long)C * CL_RMAX + 1;
+  }
+  return known[dev] - 1;
+}
+
+static int launch_getf2_cluster(float* W, long long ldw, long long n, long long jp, int nb, int* ipiv, int* info,
+                                int* plan, cudaStream_t s) {
+  const long long m = n - jp;
+  int C = 1;  // a power of two; above one CTA every one has at least 193 rows
+  while ((long long)C * CL_RMAX < m) C *= 2;
+  const int R = (int)(((m + C - 1) / C + 31) / 32 * 32);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  cfg.gridDim = dim3(C);
+  cfg.blockDim = dim3(CL_THREADS);
+  cfg.dynamicSmemBytes = getf2_cluster_smem(R);
+  cfg.stream = s;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = C;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  MPDOK_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_getf2_cluster, W, ldw, n, jp, nb, R, ipiv, info, plan));
+  count_launch();
+  return MPDOK_OK;
+}
+
 // Rows per CTA of the pivoted panel factorization for m panel rows, or -1
 // when the slices would not fit in shared memory.
 static int piv_rows_per_cta(long long m, int nb, int* grid) {
@@ -2221,31 +2493,36 @@ static int lu_factor_piv(const double* A, long long lda, long long n, int fdtype
   launch(k_col_scale_copy, (unsigned)n, 256, 0, s, A, lda, n, (const float*)dr, dc, W, w.ldw);
   MPDOK_LAUNCH_CHECK("lu equilibration");
   constexpr size_t smem_tp = trsm_pair_smem(64);
-  MPDOK_TRY(set_smem(k_piv_diag<F>, DIAG_SMEM));
+  MPDOK_TRY(set_smem(k_piv_diag<F>, DIAG_RR_SMEM));
   MPDOK_TRY(set_smem(k_trsm_pair<F, 64>, smem_tp));
+  const long long cl_rows = getf2_cluster_rows();
   for (long long jp = 0; jp < n; jp += LNB) {
     const int nb = (int)std::min<long long>(LNB, n - jp);
     const long long m = n - jp;
-    int G = 0;
-    const int R = piv_rows_per_cta(m, nb, &G);
-    if (R < 0) {
-      set_error("pivoted LU: a %lld-row panel does not fit the co-resident CTAs' shared memory (n too large for "
-                "pivoting = 1 on this device)", m);
-      return MPDOK_ERR_UNSUPPORTED;
-    }
-    const size_t smem = (size_t)nb * R * sizeof(float);
-    MPDOK_TRY(set_smem(k_getf2, smem));
-    MPDOK_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(unsigned), s));
-    {
-      float* aW = W;
-      long long aldw = w.ldw, an = n, ajp = jp;
-      int anb = nb, aR = R;
-      int* aipiv = ipiv;
-      int* ainfo = errw + 2;
-      int* aerr = errw + 3;
-      void* args[] = {&aW, &aldw, &an, &ajp, &anb, &aR, &aipiv, &ainfo, &cand, &crow, &top, &bar, &plan, &aerr};
-      MPDOK_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_getf2, dim3(G), dim3(GETF2_THREADS), args, smem, s));
-      count_launch();
+    if (m <= cl_rows) {
+      MPDOK_TRY(launch_getf2_cluster(W, w.ldw, n, jp, nb, ipiv, errw + 2, plan, s));
+    } else {
+      int G = 0;
+      const int R = piv_rows_per_cta(m, nb, &G);
+      if (R < 0) {
+        set_error("pivoted LU: a %lld-row panel does not fit the co-resident CTAs' shared memory (n too large for "
+                  "pivoting = 1 on this device)", m);
+        return MPDOK_ERR_UNSUPPORTED;
+      }
+      const size_t smem = (size_t)nb * R * sizeof(float);
+      MPDOK_TRY(set_smem(k_getf2, smem));
+      MPDOK_CUDA_TRY(cudaMemsetAsync(bar, 0, sizeof(unsigned), s));
+      {
+        float* aW = W;
+        long long aldw = w.ldw, an = n, ajp = jp;
+        int anb = nb, aR = R;
+        int* aipiv = ipiv;
+        int* ainfo = errw + 2;
+        int* aerr = errw + 3;
+        void* args[] = {&aW, &aldw, &an, &ajp, &anb, &aR, &aipiv, &ainfo, &cand, &crow, &top, &bar, &plan, &aerr};
+        MPDOK_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_getf2, dim3(G), dim3(GETF2_THREADS), args, smem, s));
+        count_launch();
+      }
     }
     const long long rest = n - jp - nb;
     if (jp + rest > 0) {
@@ -2253,7 +2530,7 @@ static int lu_factor_piv(const double* A, long long lda, long long n, int fdtype
       launch(k_laswp, gl, 256, 0, s, W, w.ldw, (const int*)plan, 0LL, jp, jp + nb, rest);
     }
     const int k = (int)(jp / LNB);
-    launch(k_piv_diag<F>, 1, DIAG_THREADS, DIAG_SMEM, s, (const float*)W, w.ldw, jp, nb, LU, L.ldf,
+    launch(k_piv_diag<F>, 1, DIAG_LU_THREADS, DIAG_RR_SMEM, s, (const float*)W, w.ldw, jp, nb, LU, L.ldf,
            Linv + (size_t)k * LNB * LNB, Uinv + (size_t)k * LNB * LNB);
     MPDOK_LAUNCH_CHECK("pivoted panel");
     if (rest <= 0) continue;
@@ -2273,6 +2550,8 @@ static int lu_factor_piv(const double* A, long long lda, long long n, int fdtype
   {
     dim3 g2((unsigned)std::min<long long>((n + 255) / 256, 16), (unsigned)std::min<long long>(n, 65535));
     launch(k_store_lower<F>, g2, 256, 0, s, (const float*)W, w.ldw, n, LU, L.ldf);
+    MPDOK_TRY(set_smem(k_tri_inv_complete, DIAG_SMEM));
+    launch(k_tri_inv_complete, L.nblk, DIAG_THREADS, DIAG_SMEM, s, (const float*)W, w.ldw, n, Linv, Uinv);
     const size_t smem_ct = 2 * (size_t)LNB * LNB * sizeof(float);
     MPDOK_TRY(set_smem(k_trsv_chain_tiles<F>, smem_ct));
     launch(k_trsv_chain_tiles<F>, dim3(L.nblk, 2), 256, smem_ct, s, (const F*)LU, L.ldf, (const float*)Linv,
