@@ -410,8 +410,8 @@ MPDOK_API int mpdok_batch_graph_launch(void* plan, cudaStream_t stream);
 MPDOK_API long long mpdok_batch_graph_nodes(void* plan);
 /* Schedule of mpdok_batch_step and of the captured graph.  0: level
  * synchronous, three launches per 64-column block level (diagonal factor,
- * panel solve, trailing update over every active system) plus the level
- * scheduled solves.  1: the whole step as ONE persistent launch of
+ * panel solve, trailing update over every active system) plus one launch per
+ * triangular solve.  1: the whole step as ONE persistent launch of
  * ctas_per_sm (1..3) CTAs per SM that take tile tasks (assembly, Cholesky,
  * solve, FP64 refinement) from a queue in a topological order and start each
  * one as soon as its inputs are final; results are bit-identical to 0. */
@@ -419,8 +419,8 @@ MPDOK_API int mpdok_batch_schedule(void* plan, int schedule, int ctas_per_sm);
 /* One step on B / X: assembly + factor + solve + `refine` refinement steps
  * under the plan's schedule (no host synchronisation). */
 MPDOK_API int mpdok_batch_step(void* plan, const double* B, double* X, int refine, cudaStream_t stream);
-/* MPDOK_ERR_TIMEOUT when a task of the last task-graph step gave up waiting
- * on its inputs (synchronises the stream), else 0. */
+/* MPDOK_ERR_TIMEOUT when a task of the last task-graph step, or a block of the
+ * last solve, gave up waiting on its inputs (synchronises the stream), else 0. */
 MPDOK_API int mpdok_batch_dag_status(void* plan, cudaStream_t stream);
 
 /* --------------------------------------------------------- instrumentation

@@ -6,7 +6,7 @@ Cholesky on 64 x 64 tiles (double-float trailing update), FP64 triangular
 solves and FP64 refinement.  Two schedules run the same tile arithmetic:
 ``levels`` (three launches per block level over every active system, a
 persistent trailing-update grid over the level's (system, tile) tasks, then
-level-scheduled solves) and ``dag`` (the whole step, assembly to the last
+one launch per triangular solve) and ``dag`` (the whole step, assembly to the last
 refinement, as ONE persistent launch whose CTAs take tile tasks from a queue
 in topological order and start each one when its inputs are final).  The
 step is captured into a CUDA graph and replayed with a single launch.

@@ -22,6 +22,8 @@
 //    and the trailing update (one task per (system, lower tile), run by a
 //    persistent grid that strides over the task list).  Task lists are
 //    prefix sums per level, decoded on the device.
+//  * The triangular solves of all systems are one launch per direction, a CTA
+//    per row block that waits for its predecessors' values.
 //  * Nothing in factor / solve / refine synchronises with the host, so the
 //    whole sequence is captured once into a CUDA graph and replayed with a
 //    single graph launch.
@@ -66,13 +68,15 @@ struct BatchPlan {
   std::vector<long long> preT, preS;  // per level: prefix sums (act[k] + 1 entries each)
   std::vector<long long> preT_off, preS_off;
   std::vector<long long> preRow;      // prefix of nblk over all systems (row-tile tasks)
+  std::vector<long long> preLvl;      // prefix of act over the levels (the solves' tickets)
   long long total_x = 0, total_c = 0;
   BSys* d_sys = nullptr;
   long long* d_pre = nullptr;         // preT | preS | preRow
-  long long d_preS_base = 0, d_preRow_base = 0;
+  long long d_preS_base = 0, d_preRow_base = 0, d_preLvl_base = 0;
   double* arena = nullptr;            // A | Linv | V | R | rowscratch
   double *A = nullptr, *Linv = nullptr, *V = nullptr, *R = nullptr, *rows = nullptr, *coords = nullptr;
   int* d_pert = nullptr;
+  int* d_ticket = nullptr;            // the solves: forward and backward ticket, timed-out wait
   size_t bytes = 0;
   int syrk_grid = 0;
   cudaStream_t cap = nullptr;
@@ -192,60 +196,119 @@ __global__ void __launch_bounds__(BT) k_bassemble(const BSys* __restrict__ sys, 
 }
 
 // ------------------------------------------------------------------ level k: diagonal block
-// Cholesky of the 64x64 diagonal block (FP64, in shared memory), its inverse,
-// L11 written over the lower triangle, Linv kept for the panel and the solves.
+// Cholesky of the 64x64 diagonal block (FP64) and its inverse.  One elimination
+// with 64 steps does both: with multipliers m_i = a_ij / d_j,
+//   a_il -= m_i a_lj  (l > j),     x_ic -= m_i x_jc  (c <= j, X = I at first)
+// give L D L^T and X = (unit L)^-1; the scaling by 1 / sqrt(d_j) comes last:
+// L_ij = a_ij / sqrt(d_j), Linv_ic = x_ic / sqrt(d_i).  Thread (ty, tx) of a 16 x 16
+// grid keeps rows ty + 16 u and columns tx + 16 v of both in registers.  Bound by
+// FP64, an instruction every 16 clocks and dependent ones 170 apart: per step the
+// reciprocal (three dependent operations from the FP32 one), the multipliers and
+// the update, about ten instructions per warp, whole 16-row strips above the
+// pivot skipped.  The inverse by rows after the factorization, its sums
+// sequential, took 170 of the 223 us of the former kernel; now 95 us in all.
+// `scr`: 64 x 3 doubles of shared memory.  Ends with L and Linv in sL / sI
+// (Linv zero above its diagonal and past nb).
+__device__ __forceinline__ void potrf_tile(double* sL, double* sI, double* scr, int nb, double dref, int* pert) {
+  double* sc = scr;            // column j of a
+  double* sx = scr + BNB;      // row j of x
+  double* sd = scr + 2 * BNB;  // pivots
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  double a[4][4], x[4][4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int i = ty + 16 * u, l = tx + 16 * v;
+      a[u][v] = l <= i ? sL[i * BPAD + l] : 0.0;
+      x[u][v] = i == l ? 1.0 : 0.0;
+    }
+#pragma unroll
+  for (int jb = 0; jb < 4; ++jb) {
+#pragma unroll 1
+    for (int j16 = 0; j16 < 16; ++j16) {
+      const int j = 16 * jb + j16;
+      if (j >= nb) break;
+      if (tx == j16)
+#pragma unroll
+        for (int u = jb; u < 4; ++u) sc[ty + 16 * u] = a[u][jb];
+      if (ty == j16)
+#pragma unroll
+        for (int v = 0; v <= jb; ++v) sx[tx + 16 * v] = x[jb][v];
+      __syncthreads();
+      double d = sc[j];
+      if (!(d > 1e-15 * dref)) {  // not positive in FP64: perturb and count
+        d = 1e-15 * dref;
+        if (threadIdx.x == 0) atomicAdd(pert, 1);
+      }
+      // 1 / d: r0 (1 + e + e^2), e = 1 - d r0 below 2^-22 (d outside FP32's range: the division)
+      const float df = (float)d;
+      double rd;
+      if (df > 1e-37f && df < 1e37f) {
+        const double r0 = (double)(1.f / df);
+        const double e = fma(-d, r0, 1.0);
+        rd = fma(r0, fma(e, e, e), r0);
+      } else {
+        rd = 1.0 / d;
+      }
+      double m[4], cl[4];
+#pragma unroll
+      for (int u = jb; u < 4; ++u) m[u] = ty + 16 * u > j ? -(sc[ty + 16 * u] * rd) : 0.0;
+#pragma unroll
+      for (int v = jb; v < 4; ++v) cl[v] = sc[tx + 16 * v];
+#pragma unroll
+      for (int u = jb; u < 4; ++u) {
+        if (16 * u + 15 <= j) continue;
+#pragma unroll
+        for (int v = jb; v <= u; ++v)
+          if (tx + 16 * v > j) a[u][v] = fma(m[u], cl[v], a[u][v]);
+#pragma unroll
+        for (int v = 0; v <= jb; ++v) x[u][v] = fma(m[u], sx[tx + 16 * v], x[u][v]);
+      }
+      if (threadIdx.x == 0) sd[j] = d;
+      __syncthreads();
+    }
+  }
+  // 1 / sqrt(d_j) once per pivot, then both scalings
+  if (threadIdx.x < BNB) {
+    const double d = threadIdx.x < nb ? sd[threadIdx.x] : 1.0;
+    const double p = sqrt(d);
+    sc[threadIdx.x] = p;
+    sx[threadIdx.x] = 1.0 / p;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int i = ty + 16 * u, l = tx + 16 * v;
+      const bool in = l <= i && i < nb;
+      sL[i * BPAD + l] = !in ? 0.0 : i == l ? sc[l] : a[u][v] * sx[l];
+      sI[i * BPAD + l] = in ? x[u][v] * sx[i] : 0.0;
+    }
+  __syncthreads();
+}
+
 __global__ void __launch_bounds__(BT) k_bpotrf(const BSys* __restrict__ sys, int k, double* __restrict__ A,
                                                 double* __restrict__ Linv, int* __restrict__ pert) {
   extern __shared__ double smem[];
   double* sL = smem;                 // BNB x BPAD, sL[i * BPAD + j] = L(i, j)
   double* sI = smem + BNB * BPAD;    // inverse, same layout
-  __shared__ double s_inv;
+  __shared__ double scr[3 * BNB];
   const BSys q = sys[blockIdx.x];
   const int kb = k * BNB;
   const int nb = min(BNB, q.n - kb);
   double* Ab = A + q.offA;
   const long long lda = q.n;
+#pragma unroll 8
   for (int e = threadIdx.x; e < BNB * BNB; e += BT) {
     const int i = e & 63, j = e >> 6;
     double v = 0.0;
     if (i < nb && j < nb && i >= j) v = df_to_f64(ld_df(Ab + (long long)(kb + i) + (long long)(kb + j) * lda));
     sL[i * BPAD + j] = v;
-    sI[i * BPAD + j] = 0.0;
   }
   __syncthreads();
-  const double dref = 1.0 + q.reg;  // phi(0) + reg: the diagonal of A
-  for (int j = 0; j < nb; ++j) {
-    if (threadIdx.x == 0) {
-      double d = sL[j * BPAD + j];
-      if (!(d > 1e-15 * dref)) {  // not positive in FP64: perturb and count
-        d = 1e-15 * dref;
-        atomicAdd(pert, 1);
-      }
-      const double p = sqrt(d);
-      sL[j * BPAD + j] = p;
-      s_inv = 1.0 / p;
-    }
-    __syncthreads();
-    const double ip = s_inv;
-    for (int i = j + 1 + threadIdx.x; i < nb; i += BT) sL[i * BPAD + j] *= ip;
-    __syncthreads();
-    const int m = nb - j - 1;
-    for (int e = threadIdx.x; e < m * m; e += BT) {
-      const int i = j + 1 + e / m, l = j + 1 + e % m;
-      if (l <= i) sL[i * BPAD + l] -= sL[i * BPAD + j] * sL[l * BPAD + j];
-    }
-    __syncthreads();
-  }
-  // inverse of the lower-triangular L11, row by row: Linv(i, c) for c <= i
-  for (int i = 0; i < nb; ++i) {
-    const int c = threadIdx.x;
-    if (c <= i && c < BNB) {
-      double acc = (c == i) ? 1.0 : 0.0;
-      for (int l = c; l < i; ++l) acc -= sL[i * BPAD + l] * sI[l * BPAD + c];
-      sI[i * BPAD + c] = acc / sL[i * BPAD + i];
-    }
-    __syncthreads();
-  }
+  potrf_tile(sL, sI, scr, nb, 1.0 + q.reg, pert);  // phi(0) + reg: the diagonal of A
   for (int e = threadIdx.x; e < BNB * BNB; e += BT) {
     const int i = e & 63, j = e >> 6;
     if (i < nb && j < nb && i >= j) st_df(Ab + (long long)(kb + i) + (long long)(kb + j) * lda, to_df(sL[i * BPAD + j]));
@@ -268,6 +331,35 @@ __device__ __forceinline__ void tile_fma_f64(const double* sA, const double* sB,
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
+  }
+}
+
+// The panel solve's product A21 Linv11^T, FP64: sA[kk][row], sB[kk][col] =
+// Linv(col, kk), zero for kk > col, so column quad c needs kk < 4 c + 4 only.  A
+// warp takes quads w and 15 - w (68 of 128 steps, the same for every warp), a
+// lane two rows (59 levels of 32 systems: 12.3 -> 7.4 ms).  put(row, col, value).
+template <typename Put>
+__device__ __forceinline__ void trsm_tile(const double* sA, const double* sB, Put put) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int c0 = 4 * (h == 0 ? warp : 15 - warp);
+    double acc[2][4] = {};
+#pragma unroll 4
+    for (int kk = 0; kk < c0 + 4; ++kk) {
+      const double a0 = sA[kk * BPAD + 2 * lane], a1 = sA[kk * BPAD + 2 * lane + 1];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const double b = sB[kk * BPAD + c0 + j];
+        acc[0][j] = fma(a0, b, acc[0][j]);
+        acc[1][j] = fma(a1, b, acc[1][j]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      put(2 * lane, c0 + j, acc[0][j]);
+      put(2 * lane + 1, c0 + j, acc[1][j]);
+    }
   }
 }
 
@@ -338,16 +430,9 @@ __global__ void __launch_bounds__(BT) k_btrsm(const BSys* __restrict__ sys, cons
     sB[kk * BPAD + col] = Li[col + kk * BNB];
   }
   __syncthreads();
-  double acc[4][4] = {};
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  tile_fma_f64(sA, sB, acc, ty, tx);
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int row = ty * 4 + i, col = tx * 4 + j;
-      if (row < nr && col < nb) st_df(Ab + (long long)(r0 + row) + (long long)(kb + col) * lda, to_df(acc[i][j]));
-    }
+  trsm_tile(sA, sB, [&](int row, int col, double v) {
+    if (row < nr && col < nb) st_df(Ab + (long long)(r0 + row) + (long long)(kb + col) * lda, to_df(v));
+  });
 }
 
 // ------------------------------------------------------------------ level k: trailing update
@@ -414,101 +499,169 @@ __global__ void __launch_bounds__(BT) k_bsyrk(const BSys* __restrict__ sys, cons
   }
 }
 
-// ------------------------------------------------------------------ triangular solves (FP64, nrhs <= 8)
-// V_k := Linv_k V_k (forward) or Linv_k^T V_k (backward) for each active system.
-template <bool TRANS>
-__global__ void __launch_bounds__(BT) k_bsolve_diag(const BSys* __restrict__ sys, int k, int nrhs,
-                                                    const double* __restrict__ Linv, double* __restrict__ V) {
-  __shared__ double sX[BNB * BMAX_RHS];
-  __shared__ double sLi[BNB * BPAD];
-  const BSys q = sys[blockIdx.x];
-  const int kb = k * BNB, nb = min(BNB, q.n - kb);
-  double* Vb = V + q.offX;
-  const double* Li = Linv + q.offL + (long long)k * BNB * BNB;
-  for (int e = threadIdx.x; e < BNB * nrhs; e += BT) {
-    const int i = e % BNB, r = e / BNB;
-    sX[e] = (i < nb) ? Vb[(long long)(kb + i) + (long long)r * q.n] : 0.0;
+// ------------------------------------------------------------------ triangular solves (nrhs <= 8)
+// One entry of L(r, k) V_k (or its transpose) over a 64-wide block.  The
+// products run in double-float on the FP32 pipe (the factor is stored that way;
+// V_k is split once per tile), the subtraction from V_r in FP64: these are
+// correction solves inside FP64 refinement, where 2^-48 products are ample, and
+// FP64 arithmetic here would run at 1/64 of the FP32 rate.
+// sT[kk * BPAD + row], sX[kk].
+__device__ __forceinline__ double df_dot64(const DF* sT, int row, const DF* sX) {
+  float sh = 0.f, sl = 0.f;
+#pragma unroll 4
+  for (int kk = 0; kk < BNB; ++kk) {
+    const DF a = sT[kk * BPAD + row], b = sX[kk];
+    const float ph = a.h * b.h;
+    float pl = fmaf(a.h, b.h, -ph);
+    pl = fmaf(a.h, b.l, pl);
+    pl = fmaf(a.l, b.h, pl);
+    const float tt = sh + ph;
+    const float bp = tt - sh;
+    const float er = (sh - (tt - bp)) + (ph - bp);
+    sh = tt;
+    sl += er + pl;
   }
-  for (int e = threadIdx.x; e < BNB * BNB; e += BT) {
-    const int i = e & 63, j = e >> 6;
-    sLi[i * BPAD + j] = Li[i + j * BNB];  // sLi[i][j] = Linv(i, j)
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < BNB * nrhs; e += BT) {
-    const int i = e % BNB, r = e / BNB;
-    if (i >= nb) continue;
-    double acc = 0.0;
-    if (!TRANS) {
-      for (int c = 0; c <= i; ++c) acc = fma(sLi[i * BPAD + c], sX[r * BNB + c], acc);
-    } else {
-      for (int c = i; c < nb; ++c) acc = fma(sLi[c * BPAD + i], sX[r * BNB + c], acc);
-    }
-    Vb[(long long)(kb + i) + (long long)r * q.n] = acc;
-  }
+  return (double)sh + (double)sl;
 }
 
-// Forward: V_r -= L(r, k) V_k for r > k.  Backward: V_r -= L(k, r)^T V_k for r < k.
-// The products run in double-float on the FP32 pipe (the factor is stored
-// that way; V_k is split once per tile), the subtraction from V_r in FP64:
-// these are correction solves inside FP64 refinement, where 2^-48 products
-// are ample, and FP64 arithmetic here would run at 1/64 of the FP32 rate.
+// Entry i of Linv_k x (or Linv_k^T x), FP64, in four interleaved sums: dependent
+// FP64 operations are about 170 clocks apart.  Linv holds exact zeros above its
+// diagonal, and x zeros past the block.
 template <bool TRANS>
-__global__ void __launch_bounds__(BT) k_bsolve_upd(const BSys* __restrict__ sys, const long long* __restrict__ pre,
-                                                   int cnt, int k, int nrhs, const double* __restrict__ A,
-                                                   double* __restrict__ V) {
-  __shared__ DF sT[BNB * BPAD];   // sT[kk][row] = multiplier (row of the target, kk of V_k)
-  __shared__ DF sX[BNB * BMAX_RHS];
-  const long long t = blockIdx.x;
-  int s, r;
+__device__ __forceinline__ double diag_dot(const double* sLi, const double* sx, int i) {
+  double a[4] = {0.0, 0.0, 0.0, 0.0};
   if (!TRANS) {
-    s = task_system(pre, cnt + 1, t);
-    r = k + 1 + (int)(t - pre[s]);
+    for (int c = 0; c <= i; c += 4)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) a[u] = fma(sLi[i * BPAD + c + u], sx[c + u], a[u]);
   } else {
-    s = (int)(t / k);
-    r = (int)(t % k);
+    for (int c = i & ~3; c < BNB; c += 4)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) a[u] = fma(sLi[(c + u) * BPAD + i], sx[c + u], a[u]);
   }
-  const BSys q = sys[s];
-  const int kb = k * BNB, r0 = r * BNB;
-  const int nb = min(BNB, q.n - kb), nr = min(BNB, q.n - r0);
-  const double* Ab = A + q.offA;
-  const long long lda = q.n;
-  double* Vb = V + q.offX;
-  if (!TRANS) {
-    stage_block(sT, Ab + r0 + (long long)kb * lda, lda, nr, nb);  // sT[kk][row] = L(r0+row, kb+kk)
-  } else {
-    // sT[kk][row] = L(kb+kk, r0+row): read the tile (kb rows, r0 cols) coalesced along kk
-    for (int e = threadIdx.x; e < BNB * BNB; e += BT) {
-      const int kk = e & 63, row = e >> 6;
-      DF v;
-      v.h = 0.f;
-      v.l = 0.f;
-      if (kk < nb && row < nr) v = ld_df(Ab + (long long)(kb + kk) + (long long)(r0 + row) * lda);
-      sT[kk * BPAD + row] = v;
-    }
-  }
-  for (int e = threadIdx.x; e < BNB * nrhs; e += BT) {
-    const int i = e % BNB, rr = e / BNB;
-    sX[e] = to_df((i < nb) ? Vb[(long long)(kb + i) + (long long)rr * q.n] : 0.0);
+  return (a[0] + a[1]) + (a[2] + a[3]);
+}
+
+// Results start as this bit pattern; consumers poll the values themselves.
+constexpr unsigned long long BSOLVE_EMPTY = 0xffffffffffffffffull;
+constexpr long long BSOLVE_WAIT = 1LL << 24;
+constexpr int BSOLVE_RHS = 4;    // right-hand sides of one CTA
+constexpr size_t BSOLVE_SMEM = (size_t)BNB * BPAD * (sizeof(double) + sizeof(DF)) +
+                               (size_t)BNB * BSOLVE_RHS * (sizeof(double) + sizeof(DF));
+
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const double* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed_u64(double* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// OUT := L^-1 IN (or L^-T IN) for every system in one launch.  A CTA owns one
+// 64-row block of one system and up to four right-hand sides.  CTAs take their
+// blocks from a ticket in level order (block 0 of every system, block 1, ..;
+// backward from the last ones), so a block's predecessors are always held by
+// CTAs that run or have finished; it subtracts each predecessor's product as
+// soon as that block's values appear (bounded wait; the next factor tile is
+// loaded meanwhile) and finally multiplies by the diagonal block's inverse.
+// Bound by the chain of blocks, about 11 us each: walk, FP64 product with the
+// inverse (3 us; four columns to a CTA, since FP64 is what an SM has least of),
+// publish.  32 systems of 300 .. 4000, 8 columns: 0.73 ms forward, 0.69 ms
+// backward; two launches per level took 2.2 and 2.1 ms.
+template <bool TRANS>
+__global__ void __launch_bounds__(BT) k_bsolve_chain(const BSys* __restrict__ sys, const long long* __restrict__ lvl,
+                                                     int maxblk, int nrhs, const double* __restrict__ A,
+                                                     const double* __restrict__ Linv, const double* __restrict__ IN,
+                                                     double* OUT, int* ticket, int* err) {
+  extern __shared__ double smem[];
+  double* sLi = smem;                                            // [i][c]
+  double* sx = sLi + BNB * BPAD;                                 // [rhs][64]
+  DF* sT = reinterpret_cast<DF*>(sx + BNB * BSOLVE_RHS);         // [kk][row]
+  DF* sX = sT + BNB * BPAD;                                      // [rhs][64]
+  __shared__ int s_t, s_abort;
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    s_t = atomicAdd(ticket, 1);
+    s_abort = 0;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < BNB * nrhs; e += BT) {
-    const int row = e % BNB, rr = e / BNB;
-    if (row >= nr) continue;
-    float sh = 0.f, sl = 0.f;
-#pragma unroll 4
-    for (int kk = 0; kk < BNB; ++kk) {
-      const DF a = sT[kk * BPAD + row], b = sX[rr * BNB + kk];
-      const float ph = a.h * b.h;
-      float pl = fmaf(a.h, b.h, -ph);
-      pl = fmaf(a.h, b.l, pl);
-      pl = fmaf(a.l, b.h, pl);
-      const float tt = sh + ph;
-      const float bp = tt - sh;
-      const float er = (sh - (tt - bp)) + (ph - bp);
-      sh = tt;
-      sl += er + pl;
+  const int groups = (nrhs + BSOLVE_RHS - 1) / BSOLVE_RHS;
+  const long long t = s_t / groups;
+  const int r8 = (s_t % groups) * BSOLVE_RHS;
+  if (t >= lvl[maxblk]) return;
+  int lo = 0, hi = maxblk - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (lvl[mid] <= t) lo = mid; else hi = mid - 1;
+  }
+  const BSys q = sys[t - lvl[lo]];
+  const int r = TRANS ? q.nblk - 1 - lo : lo;
+  const int cnt = TRANS ? q.nblk - 1 - r : r;  // blocks this one waits for
+  const int r0 = r * BNB, nr = min(BNB, q.n - r0);
+  const double* Ab = A + q.offA;
+  const long long lda = q.n;
+  const int row = tid & 63, rr = tid >> 6;
+  const bool live = row < nr && r8 + rr < nrhs;
+  const long long col = q.offX + (long long)(r8 + rr) * q.n;     // this thread's column
+  const double* Li = Linv + q.offL + (long long)r * BNB * BNB;
+  auto block_of = [&](int j) { return TRANS ? q.nblk - 1 - j : j; };
+  // the factor tile of predecessor j: 16 entries per thread, as they lie in memory
+  float2 T[16];
+  auto load_tile = [&](int j) {
+    const int k = block_of(j), kb = k * BNB, nb = min(BNB, q.n - kb);
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int i = tid & 63, c = (tid >> 6) + 4 * u;
+      // forward: rows of r, columns of k; backward: rows of k, columns of r
+      const bool ok = TRANS ? (i < nb && c < nr) : (i < nr && c < nb);
+      const double* p = TRANS ? Ab + kb + i + (long long)(r0 + c) * lda : Ab + r0 + i + (long long)(kb + c) * lda;
+      T[u] = ok ? __ldg(reinterpret_cast<const float2*>(p)) : make_float2(0.f, 0.f);
     }
-    Vb[(long long)(r0 + row) + (long long)rr * q.n] -= (double)sh + (double)sl;
+  };
+  if (cnt > 0) load_tile(0);
+  double acc = live ? IN[col + r0 + row] : 0.0;
+  for (int e = tid; e < BNB * BNB; e += BT) sLi[(e & 63) * BPAD + (e >> 6)] = __ldg(Li + e);
+  for (int j = 0; j < cnt; ++j) {
+    const int kb = block_of(j) * BNB, nb = min(BNB, q.n - kb);
+    // its values, one per thread
+    double v = 0.0;
+    if (row < nb && r8 + rr < nrhs) {
+      unsigned long long b = BSOLVE_EMPTY;
+      for (long long it = 0; it < BSOLVE_WAIT; ++it) {
+        b = ld_relaxed_u64(OUT + col + kb + row);
+        if (b != BSOLVE_EMPTY) break;
+        if (it > 64) {
+          if ((it & 255) == 0 && *(volatile const int*)err) break;
+          __nanosleep(32);
+        }
+      }
+      if (b == BSOLVE_EMPTY) {
+        s_abort = 1;
+        atomicExch(err, 1);
+      }
+      v = __longlong_as_double((long long)b);
+    }
+    __syncthreads();  // the previous tile has been used
+    if (s_abort) return;
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const int i = tid & 63, c = (tid >> 6) + 4 * u;
+      const DF d = {T[u].x, T[u].y};
+      if (TRANS) sT[i * BPAD + c] = d;
+      else sT[c * BPAD + i] = d;
+    }
+    sX[tid] = to_df(v);
+    __syncthreads();
+    if (j + 1 < cnt) load_tile(j + 1);
+    if (live) acc -= df_dot64(sT, row, sX + rr * BNB);
+  }
+  sx[tid] = acc;
+  __syncthreads();
+  if (live) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(diag_dot<TRANS>(sLi, sx + rr * BNB, row));
+    // (a NaN of the caller's with the empty pattern becomes another NaN)
+    st_relaxed_u64(OUT + col + r0 + row, b == BSOLVE_EMPTY ? 0x7ff8000000000000ull : b);
   }
 }
 
@@ -844,8 +997,9 @@ __device__ __forceinline__ void syrk_tiles(int kind, int k, long long u, int& ti
   tj = k + sh + b;
 }
 
+// (three CTAs per SM: 80 registers, which the diagonal factor alone would exceed)
 template <int KIND, int D, int ARITH>
-__global__ void __launch_bounds__(BT) k_bstep_dag(const BSys* __restrict__ sys, const long long* __restrict__ pre,
+__global__ void __launch_bounds__(BT, 3) k_bstep_dag(const BSys* __restrict__ sys, const long long* __restrict__ pre,
                                                   const DagSec* __restrict__ secs, int nsec, long long total,
                                                   const long long* __restrict__ st_off, const long long* __restrict__ v_off,
                                                   long long v_total, int nsys, int nrhs,
@@ -987,7 +1141,6 @@ __global__ void __launch_bounds__(BT) k_bstep_dag(const BSys* __restrict__ sys, 
       case BT_POTRF: {
         double* sL = smem;
         double* sI = smem + BNB * BPAD;
-        double* s_inv = smem + 2 * BNB * BPAD;
         const int kb = k * BNB;
         const int nb = min(BNB, q.n - kb);
         for (int e = tid; e < BNB * BNB; e += BT) {
@@ -995,41 +1148,9 @@ __global__ void __launch_bounds__(BT) k_bstep_dag(const BSys* __restrict__ sys, 
           double v = 0.0;
           if (i < nb && j < nb && i >= j) v = df_to_f64(ld_df_cg(Ab + (long long)(kb + i) + (long long)(kb + j) * lda));
           sL[i * BPAD + j] = v;
-          sI[i * BPAD + j] = 0.0;
         }
         __syncthreads();
-        const double dref = 1.0 + q.reg;
-        for (int j = 0; j < nb; ++j) {
-          if (tid == 0) {
-            double d = sL[j * BPAD + j];
-            if (!(d > 1e-15 * dref)) {
-              d = 1e-15 * dref;
-              atomicAdd(pert, 1);
-            }
-            const double p = sqrt(d);
-            sL[j * BPAD + j] = p;
-            *s_inv = 1.0 / p;
-          }
-          __syncthreads();
-          const double ip = *s_inv;
-          for (int i = j + 1 + tid; i < nb; i += BT) sL[i * BPAD + j] *= ip;
-          __syncthreads();
-          const int m = nb - j - 1;
-          for (int e = tid; e < m * m; e += BT) {
-            const int i = j + 1 + e / m, l = j + 1 + e % m;
-            if (l <= i) sL[i * BPAD + l] -= sL[i * BPAD + j] * sL[l * BPAD + j];
-          }
-          __syncthreads();
-        }
-        for (int i = 0; i < nb; ++i) {
-          const int c = tid;
-          if (c <= i && c < BNB) {
-            double acc = (c == i) ? 1.0 : 0.0;
-            for (int l = c; l < i; ++l) acc -= sL[i * BPAD + l] * sI[l * BPAD + c];
-            sI[i * BPAD + c] = acc / sL[i * BPAD + i];
-          }
-          __syncthreads();
-        }
+        potrf_tile(sL, sI, smem + 2 * BNB * BPAD, nb, 1.0 + q.reg, pert);
         for (int e = tid; e < BNB * BNB; e += BT) {
           const int i = e & 63, j = e >> 6;
           if (i < nb && j < nb && i >= j)
@@ -1052,16 +1173,9 @@ __global__ void __launch_bounds__(BT) k_bstep_dag(const BSys* __restrict__ sys, 
           sB[kk * BPAD + col] = __ldcg(Li + col + kk * BNB);
         }
         __syncthreads();
-        double acc[4][4] = {};
-        tile_fma_f64(sA, sB, acc, ty, tx);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int row = ty * 4 + i, col = tx * 4 + j;
-            if (row < nr && col < nb)
-              st_df(Ab + (long long)(r0 + row) + (long long)(kb + col) * lda, to_df(acc[i][j]));
-          }
+        trsm_tile(sA, sB, [&](int row, int col, double v) {
+          if (row < nr && col < nb) st_df(Ab + (long long)(r0 + row) + (long long)(kb + col) * lda, to_df(v));
+        });
         pub = st + tri_idx(ti, k);
         pub_val = k + 1;
         break;
@@ -1187,12 +1301,7 @@ __global__ void __launch_bounds__(BT) k_bstep_dag(const BSys* __restrict__ sys, 
         for (int e = tid; e < BNB * nrhs; e += BT) {
           const int i = e % BNB, r = e / BNB;
           if (i >= nb) continue;
-          double acc = 0.0;
-          if (!trans) {
-            for (int c = 0; c <= i; ++c) acc = fma(sLi[i * BPAD + c], sX[r * BNB + c], acc);
-          } else {
-            for (int c = i; c < nb; ++c) acc = fma(sLi[c * BPAD + i], sX[r * BNB + c], acc);
-          }
+          const double acc = trans ? diag_dot<true>(sLi, sX + r * BNB, i) : diag_dot<false>(sLi, sX + r * BNB, i);
           Vb[(long long)(kb + i) + (long long)r * q.n] = acc;
         }
         if (!trans) {
@@ -1235,22 +1344,8 @@ __global__ void __launch_bounds__(BT) k_bstep_dag(const BSys* __restrict__ sys, 
         for (int e = tid; e < BNB * nrhs; e += BT) {
           const int row = e % BNB, rr = e / BNB;
           if (row >= nr) continue;
-          float sh = 0.f, sl = 0.f;
-#pragma unroll 4
-          for (int kk = 0; kk < BNB; ++kk) {
-            const DF a = sT[kk * BPAD + row], b = sX[rr * BNB + kk];
-            const float ph = a.h * b.h;
-            float pl = fmaf(a.h, b.h, -ph);
-            pl = fmaf(a.h, b.l, pl);
-            pl = fmaf(a.l, b.h, pl);
-            const float tt = sh + ph;
-            const float bp = tt - sh;
-            const float er = (sh - (tt - bp)) + (ph - bp);
-            sh = tt;
-            sl += er + pl;
-          }
           double* pv = Vb + (long long)(r0 + row) + (long long)rr * q.n;
-          *pv = __ldcg(pv) - ((double)sh + (double)sl);
+          *pv = __ldcg(pv) - df_dot64(sT, row, sX + rr * BNB);
         }
         if (!trans) {
           pub = fw + r;
@@ -1289,6 +1384,7 @@ __global__ void __launch_bounds__(BT) k_bstep_dag(const BSys* __restrict__ sys, 
 static const long long* preT_dev(const BatchPlan* p, int k) { return p->d_pre + p->preT_off[k]; }
 static const long long* preS_dev(const BatchPlan* p, int k) { return p->d_pre + p->d_preS_base + p->preS_off[k]; }
 static const long long* preRow_dev(const BatchPlan* p) { return p->d_pre + p->d_preRow_base; }
+static const long long* preLvl_dev(const BatchPlan* p) { return p->d_pre + p->d_preLvl_base; }
 
 #define BKIND_DIM_SWITCH(KIND, DIM, ...)                                           \
   do {                                                                             \
@@ -1338,23 +1434,22 @@ static int batch_factor(BatchPlan* p, cudaStream_t s) {
   return MPDOK_OK;
 }
 
-// V := A^{-1} V in place (V in the caller's packing).
+// V := A^{-1} V in place (V in the caller's packing), through the plan's R.
 static int batch_solve_inplace(BatchPlan* p, double* V, cudaStream_t s) {
-  for (int k = 0; k < p->maxblk; ++k) {
-    const int cnt = p->act[k];
-    launch(k_bsolve_diag<false>, dim3(cnt), BT, 0, s, (const BSys*)p->d_sys, k, p->nrhs, (const double*)p->Linv, V);
-    const long long nt = p->preT[p->preT_off[k] + cnt];
-    if (nt > 0)
-      launch(k_bsolve_upd<false>, dim3((unsigned)nt), BT, 0, s, (const BSys*)p->d_sys, preT_dev(p, k), cnt, k,
-             p->nrhs, (const double*)p->A, V);
-  }
-  for (int k = p->maxblk - 1; k >= 0; --k) {
-    const int cnt = p->act[k];
-    launch(k_bsolve_diag<true>, dim3(cnt), BT, 0, s, (const BSys*)p->d_sys, k, p->nrhs, (const double*)p->Linv, V);
-    if (k > 0)
-      launch(k_bsolve_upd<true>, dim3((unsigned)((long long)cnt * k)), BT, 0, s, (const BSys*)p->d_sys,
-             (const long long*)nullptr, cnt, k, p->nrhs, (const double*)p->A, V);
-  }
+  const size_t bytes = (size_t)p->total_x * sizeof(double);
+  const int groups = (p->nrhs + BSOLVE_RHS - 1) / BSOLVE_RHS;
+  const unsigned grid = (unsigned)(p->preLvl.back() * groups);
+  if (grid == 0) return MPDOK_OK;
+  MPDOK_TRY(set_smem(k_bsolve_chain<false>, BSOLVE_SMEM));
+  MPDOK_TRY(set_smem(k_bsolve_chain<true>, BSOLVE_SMEM));
+  MPDOK_CUDA_TRY(cudaMemsetAsync(p->d_ticket, 0, 2 * sizeof(int), s));
+  MPDOK_CUDA_TRY(cudaMemsetAsync(p->R, 0xff, bytes, s));
+  launch(k_bsolve_chain<false>, dim3(grid), BT, BSOLVE_SMEM, s, (const BSys*)p->d_sys, preLvl_dev(p), p->maxblk,
+         p->nrhs, (const double*)p->A, (const double*)p->Linv, (const double*)V, p->R, p->d_ticket, p->d_ticket + 2);
+  MPDOK_CUDA_TRY(cudaMemsetAsync(V, 0xff, bytes, s));
+  launch(k_bsolve_chain<true>, dim3(grid), BT, BSOLVE_SMEM, s, (const BSys*)p->d_sys, preLvl_dev(p), p->maxblk,
+         p->nrhs, (const double*)p->A, (const double*)p->Linv, (const double*)p->R, V, p->d_ticket + 1,
+         p->d_ticket + 2);
   MPDOK_LAUNCH_CHECK("batch solve");
   return MPDOK_OK;
 }
@@ -1371,6 +1466,7 @@ static int batch_residual(BatchPlan* p, const double* B, const double* X, double
 static int batch_solve(BatchPlan* p, const double* B, double* X, int refine, cudaStream_t s) {
   const long long nx = p->total_x;
   if (nx == 0) return MPDOK_OK;
+  MPDOK_CUDA_TRY(cudaMemsetAsync(p->d_ticket + 2, 0, sizeof(int), s));
   MPDOK_CUDA_TRY(cudaMemcpyAsync(X, B, (size_t)nx * sizeof(double), cudaMemcpyDeviceToDevice, s));
   MPDOK_TRY(batch_solve_inplace(p, X, s));
   const unsigned g = (unsigned)std::min<long long>((nx + 255) / 256, (long long)num_sms() * 8);
@@ -1552,7 +1648,7 @@ static int batch_step_dag(BatchPlan* p, const double* B, double* X, int refine, 
   S.asm_done = S.done + (refine + 1) * p->nsys;
   S.head = reinterpret_cast<unsigned long long*>(base + p->dag_head_idx);
   S.err = base + p->dag_head_idx + 2;
-  const size_t smem = (2 * (size_t)BNB * BPAD + 32) * sizeof(double);
+  const size_t smem = (2 * (size_t)BNB * BPAD + 3 * BNB) * sizeof(double);
   const int grid = std::max(1, p->dag_ctas_per_sm) * num_sms();
   const long long* sto = p->d_dagpre + p->dag_st_off;
   const long long* vo = p->d_dagpre + p->dag_v_off;
@@ -1582,6 +1678,7 @@ static void plan_free(BatchPlan* p) {
   if (p->d_sys) cudaFree(p->d_sys);
   if (p->d_pre) cudaFree(p->d_pre);
   if (p->d_pert) cudaFree(p->d_pert);
+  if (p->d_ticket) cudaFree(p->d_ticket);
   delete p;
 }
 
@@ -1668,6 +1765,10 @@ extern "C" int mpdok_batch_create(int nsys, const long long* n, int dim, int nrh
   p->d_preRow_base = (long long)all.size();
   all.insert(all.end(), p->preRow.begin(), p->preRow.end());
   all.insert(all.end(), preA.begin(), preA.end());
+  p->preLvl.push_back(0);
+  for (int k = 0; k < p->maxblk; ++k) p->preLvl.push_back(p->preLvl.back() + p->act[k]);
+  p->d_preLvl_base = (long long)all.size();
+  all.insert(all.end(), p->preLvl.begin(), p->preLvl.end());
   auto fail = [&](cudaError_t e, const char* what) {
     cuda_status(e, what);
     plan_free(p);
@@ -1681,6 +1782,10 @@ extern "C" int mpdok_batch_create(int nsys, const long long* n, int dim, int nrh
   if (e != cudaSuccess) return fail(e, "cudaMalloc (batch systems)");
   e = cudaMalloc(&p->d_pert, sizeof(int));
   if (e != cudaSuccess) return fail(e, "cudaMalloc (batch counter)");
+  e = cudaMalloc(&p->d_ticket, 4 * sizeof(int));
+  if (e != cudaSuccess) return fail(e, "cudaMalloc (batch tickets)");
+  e = cudaMemset(p->d_ticket, 0, 4 * sizeof(int));
+  if (e != cudaSuccess) return fail(e, "cudaMemset (batch tickets)");
   const size_t nA = align_up((size_t)aA, 32), nL = align_up((size_t)aL, 32), nV = align_up((size_t)ax, 32),
                nR = align_up((size_t)aR, 32), nCo = align_up((size_t)ac, 32);
   p->bytes = (nA + nL + 2 * nV + nR + nCo) * sizeof(double);
@@ -1894,8 +1999,14 @@ extern "C" int mpdok_batch_step(void* plan, const double* B, double* X, int refi
 extern "C" int mpdok_batch_dag_status(void* plan, cudaStream_t s) {
   MPDOK_ARG_CHECK(plan, "null plan");
   BatchPlan* p = (BatchPlan*)plan;
-  if (!p->d_dagstate) return MPDOK_OK;
   int h = 0;
+  MPDOK_CUDA_TRY(cudaMemcpyAsync(&h, p->d_ticket + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
+  MPDOK_CUDA_TRY(cudaStreamSynchronize(s));
+  if (h) {
+    set_error("batch triangular solve: a block's wait on its predecessor ran out");
+    return MPDOK_ERR_TIMEOUT;
+  }
+  if (!p->d_dagstate) return MPDOK_OK;
   const int* err = p->d_dagstate + p->dag_head_idx + 2;
   MPDOK_CUDA_TRY(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, s));
   MPDOK_CUDA_TRY(cudaStreamSynchronize(s));
