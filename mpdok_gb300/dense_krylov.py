@@ -47,15 +47,19 @@ class DenseLinearOperator:
         """A @ x with the FP32 matrix; x (N,) or (N, k) -> FP32 CUDA tensor of the same shape."""
         xt = x if isinstance(x, torch.Tensor) else torch.as_tensor(x)
         squeeze = xt.dim() == 1
-        X = as_fortran(xt.reshape(-1, 1) if squeeze else xt, torch.float32)
-        k = X.shape[1]
-        Y = fortran_empty(self.N, k, torch.float32)
+        n = self.N
+        if squeeze and xt.is_cuda and xt.dtype == torch.float32 and xt.stride(0) == 1:
+            X, k = xt, 1  # one column as it is
+            Y = torch.empty(n, dtype=torch.float32, device=require_cuda())
+        else:
+            X = as_fortran(xt.reshape(-1, 1) if squeeze else xt, torch.float32)
+            k = X.shape[1]
+            Y = fortran_empty(n, k, torch.float32)
         lib = N.load()
-        wbytes = lib.mpdok_gemv_workspace_size(N.F32, self.N, self.N, k, 0)
-        w = self._ws.get(wbytes)
-        N.check(lib.mpdok_gemv(N.F32, 0, ptr(self.A_fp32), self.N, self.N, self.N, ptr(X), max(1, self.N), k,
-                               ptr(Y), max(1, self.N), 1.0, 0.0, ptr(w), w.numel(), stream_handle()), "matvec")
-        return Y.reshape(-1) if squeeze else Y
+        w = self._ws.get(lib.mpdok_gemv_workspace_size(N.F32, n, n, k, 0))
+        N.check(lib.mpdok_gemv(N.F32, 0, self.A_fp32.data_ptr(), n, n, n, X.data_ptr(), max(1, n), k,
+                               Y.data_ptr(), max(1, n), 1.0, 0.0, w.data_ptr(), w.numel(), stream_handle()), "matvec")
+        return Y.reshape(-1) if squeeze and Y.dim() == 2 else Y
 
     def rmatvec(self, x) -> torch.Tensor:
         """A^T @ x with the FP32 matrix (used by the adjoint)."""
