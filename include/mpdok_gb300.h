@@ -316,6 +316,15 @@ MPDOK_API int mpdok_lu_ir_solve_multi(const double* A, long long lda, long long 
                                       int nrhs, const double* B, long long ldb, double* X, long long ldx, double tol,
                                       int maxiter_outer, void* work, size_t work_bytes, mpdok_solve_info* info,
                                       cudaStream_t stream);
+/* The same for any number of right-hand sides, eight columns to a group: the
+ * groups iterate as mpdok_lu_ir_solve_multi would on each, and up to 16 of them
+ * share every triangular sweep.  infos (may be NULL) holds one report per group,
+ * (nrhs + 7) / 8 of them. */
+MPDOK_API size_t mpdok_lu_ir_many_work_size(long long n, int nrhs);
+MPDOK_API int mpdok_lu_ir_solve_many(const double* A, long long lda, long long n, const void* factors, int fdtype,
+                                     int nrhs, const double* B, long long ldb, double* X, long long ldx, double tol,
+                                     int maxiter_outer, void* work, size_t work_bytes, mpdok_solve_info* infos,
+                                     cudaStream_t stream);
 MPDOK_API size_t mpdok_lu_gmres_ir_work_size(long long n, int restart);
 MPDOK_API int mpdok_lu_gmres_ir(const double* A64, long long lda, const float* A32, long long lda32, long long n,
                                 const void* factors, int fdtype, const double* b, double* x, double tol,

@@ -161,6 +161,9 @@ _SIGS = {
     "mpdok_lu_ir_multi_work_size": (c_size_t, [c_ll, c_int]),
     "mpdok_lu_ir_solve_multi": (c_int, [c_void_p, c_ll, c_ll, c_void_p, c_int, c_int, c_void_p, c_ll, c_void_p, c_ll,
                                         c_double, c_int, c_void_p, c_size_t, ctypes.POINTER(SolveInfo), c_void_p]),
+    "mpdok_lu_ir_many_work_size": (c_size_t, [c_ll, c_int]),
+    "mpdok_lu_ir_solve_many": (c_int, [c_void_p, c_ll, c_ll, c_void_p, c_int, c_int, c_void_p, c_ll, c_void_p, c_ll,
+                                       c_double, c_int, c_void_p, c_size_t, ctypes.POINTER(SolveInfo), c_void_p]),
     "mpdok_profile_bytes": (c_double, [c_int]),
     "mpdok_profile_timeline": (c_ll, [ctypes.POINTER(c_double), c_ll]),
     "mpdok_lu_schedule": (c_ll, [c_ll, c_int, ctypes.POINTER(c_ll), c_ll]),

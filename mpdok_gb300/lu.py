@@ -97,7 +97,7 @@ class LUFactorization:
         return x, _info(info)
 
     def solve_ir_many(self, A, B, tol: float = 1e-11, maxiter_outer: int = 3):
-        """LU-IR for many right-hand sides at once (columns of B), 8 per sweep.
+        """LU-IR for many right-hand sides at once (columns of B), in groups of 8 that share the sweeps.
 
         Returns (X (n, k) FP64, info) with info["relres"] the worst column and
         info["converged"] true when every column met tol.
@@ -107,21 +107,18 @@ class LUFactorization:
         k = Bc.shape[1]
         X = fortran_empty(self.n, k, torch.float64)
         lib = N.load()
-        worst, conv, outer = 0.0, True, 0
-        hist = []
-        for j0 in range(0, k, 8):
-            kk = min(8, k - j0)
-            Bj = Bc[:, j0:j0 + kk]
-            w = self._ws.get(lib.mpdok_lu_ir_multi_work_size(self.n, kk))
-            info = N.SolveInfo()
-            N.check(lib.mpdok_lu_ir_solve_multi(ptr(A64), self.n, self.n, ptr(self.factors), self.fdtype, kk,
-                                                ptr(Bj), Bc.stride(1) if k > 1 else self.n, ptr(X[:, j0:j0 + kk]),
-                                                self.n, float(tol), int(maxiter_outer), ptr(w), w.numel(),
-                                                ctypes.byref(info), stream_handle()), "lu_ir_solve_multi")
-            worst = max(worst, float(info.relres))
-            conv = conv and bool(info.converged)
-            outer = max(outer, int(info.outer_iters))
-            hist.append(info.history_list())
+        if k == 0:
+            return X, {"converged": True, "relres": 0.0, "outer_iters": 0, "history": []}
+        w = self._ws.get(lib.mpdok_lu_ir_many_work_size(self.n, k))
+        infos = (N.SolveInfo * ((k + 7) // 8))()
+        N.check(lib.mpdok_lu_ir_solve_many(ptr(A64), self.n, self.n, ptr(self.factors), self.fdtype, k, ptr(Bc),
+                                           Bc.stride(1) if k > 1 else self.n, ptr(X), self.n, float(tol),
+                                           int(maxiter_outer), ptr(w), w.numel(), infos, stream_handle()),
+                "lu_ir_solve_many")
+        worst = max(float(i.relres) for i in infos)
+        conv = all(bool(i.converged) for i in infos)
+        outer = max(int(i.outer_iters) for i in infos)
+        hist = [i.history_list() for i in infos]
         squeeze = (B.dim() == 1) if isinstance(B, torch.Tensor) else (np.asarray(B).ndim == 1)
         return (X.reshape(-1) if squeeze else X), {"converged": conv, "relres": worst, "outer_iters": outer,
                                                    "history": hist}
