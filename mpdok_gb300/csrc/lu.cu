@@ -23,6 +23,7 @@
 #include "krylov.cuh"
 #include "matfree.cuh"
 #include "split.cuh"
+#include "residual64.cuh"
 #include "tc_gemm.cuh"
 
 #include <cmath>
@@ -1943,7 +1944,8 @@ static int err_finish(const int* err, int status, cudaStream_t s) {
   MPDOK_CUDA_TRY(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, s));
   MPDOK_CUDA_TRY(cudaStreamSynchronize(s));
   if (h != 0) {
-    set_error("triangular solve: a block's wait on its predecessor ran out (device wait limit)");
+    set_error(h == 5 ? "FP64 residual: a wait on its own loads or products ran out (device wait limit)"
+                     : "triangular solve: a block's wait on its predecessor ran out (device wait limit)");
     return MPDOK_ERR_TIMEOUT;
   }
   return status;
@@ -2877,7 +2879,7 @@ static int lu_ir_body(const double* A, long long lda, long long n, const void* f
 // ---------------------------------------------------- multi-RHS LU-IR
 struct MultiWork {
   size_t off_y = 0, off_z = 0, off_v = 0, off_tk = 0, off_err = 0, off_r = 0, off_nrm = 0,
-         off_g = 0, total = 0;
+         off_g = 0, off_q = 0, total = 0;
 };
 
 static MultiWork multi_layout(long long n, int K) {
@@ -2893,6 +2895,7 @@ static MultiWork multi_layout(long long n, int K) {
   m.off_r = take(nv * sizeof(double));
   m.off_nrm = take((size_t)K * sizeof(double));
   m.off_g = take(gemv_workspace_bytes(MPDOK_F64, n, n, std::min(K, 8), false));
+  m.off_q = take(residual64_work_bytes(n, K));
   m.total = off;
   return m;
 }
@@ -3022,8 +3025,14 @@ static int lu_ir_groups(const double* A, long long lda, long long n, const void*
       return MPDOK_OK;
     };
     MPDOK_TRY(correct(B, ldb, 1));
+    // many columns of a large matrix: one residual of all of them on the tensor
+    // cores (the FP64 pipe takes 0.9 ms per eight columns at n = 8192)
+    const bool tc = residual64_pays(n, nc);
+    void* rw = wb + mw.off_q;
+    if (tc) MPDOK_TRY(residual64_prepare(A, lda, n, nc, rw, s));
     for (int it = 0; it <= maxiter_outer; ++it) {
-      for (int a = 0; a < act.n; ++a) {
+      if (tc) MPDOK_TRY(residual64(A, lda, n, X, ldx, nc, B, ldb, R, n, rw, merr, s));
+      for (int a = 0; !tc && a < act.n; ++a) {
         const long long c = (long long)act.id[a] * K;
         MPDOK_TRY(gemv_launch(MPDOK_F64, false, A, lda, n, n, X + c * ldx, ldx, K, R + c * n, n, -1.0, 1.0, B + c * ldb,
                               ldb, nullptr, gw, gbytes, s, true, nullptr));

@@ -1,0 +1,19 @@
+// FP64 residuals of several columns on the tensor cores (residual64.cu).
+#pragma once
+#include "common.cuh"
+
+namespace mpdok {
+
+// Whether R = B - A X of nc columns should take residual64 (else the FP64 GEMV):
+// a tile of up to 32 columns costs 2.0e-12 n^2 s, the FP64 pipe 1.6e-12 n^2 s per
+// column, and below n = 2048 the extra launches and the ramp-up of one CTA per
+// SM weigh as much as the product.
+bool residual64_pays(long long n, int nc);
+size_t residual64_work_bytes(long long n, int nc);  // 0 where it does not pay
+// The row exponents of A (kept in the workspace until A changes).
+int residual64_prepare(const double* A, long long lda, long long n, int nc, void* work, cudaStream_t s);
+// R = B - A X; *err = 5 when a bounded wait ran out.
+int residual64(const double* A, long long lda, long long n, const double* X, long long ldx, int nc, const double* B,
+               long long ldb, double* R, long long ldr, void* work, int* err, cudaStream_t s);
+
+}  // namespace mpdok
