@@ -292,9 +292,15 @@ tc_gemm_update(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
 // ------------------------------------------------------------------------
 // Warp-specialised form for the LU's updates (K >= 128): one CTA per SM walks a
-// strip of T tiles (128 x 256) that share their A rows, with
-//   * a 4-stage TMA ring (48 KB per stage: the A and B blocks of one 64-deep
-//     K step), so four loads are in flight while the tensor cores work;
+// strip of T tiles (128 x 256) that share their A rows, or a pair of CTAs (two
+// neighbouring SMs, cta_group::2) a strip of 256 x 256 tiles, with
+//   * a TMA ring of 192 KB: four stages of the A and B blocks of one 64-deep K
+//     step, or in a pair six of its own A rows and half of B's, so that as many
+//     loads are in flight while the tensor cores work.  The bytes in flight
+//     bound the deep updates: 96 bytes per cycle and SM at the full rate for
+//     one CTA, 64 in a pair (the update of n = 16384 at K = 2048: 864 us,
+//     1273 TFLOP/s, against 794 us, 1384 TFLOP/s; with the grid's order below
+//     n = 30720 3400 -> 2740 us, 1137 -> 1411 TFLOP/s);
 //   * two TMEM accumulators (2 x 256 columns, all 512), so the MMAs of tile
 //     t + 1 run while the epilogue drains tile t;
 //   * warp 0 the TMA producer, warp 1 the MMA issuer, warps 2..9 the epilogue
@@ -306,29 +312,99 @@ tc_gemm_update(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // wait is bounded and also gives up as soon as another role has failed; a
 // failed CTA waits (bounded) for its own loads in flight before it releases
 // its tensor memory and returns.
+// Row block and strip of CTA `i` of an update's grid (`ntm` row blocks, `ns`
+// strips): bands of `band` row blocks, strip by strip within a band.
+__device__ __forceinline__ void band_order(int i, int ntm, int ns, int band, int* row, int* strip) {
+  const int b = i / (band * ns), rem = i - b * band * ns;
+  const int rows = min(band, ntm - b * band);
+  *strip = rem / rows;
+  *row = b * band + rem % rows;
+}
+
 namespace ws {
 
-constexpr int STAGES = 4;
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 32 * (2 + EPI_WARPS);
 constexpr int TMEM_COLS = 512;
-constexpr int A_SUB = BM * BK * 2;   // 16 KB
-constexpr int B_SUB = BN * BK * 2;   // 32 KB
-constexpr int STAGE = A_SUB + B_SUB;
 // epilogue staging: per epilogue warp two 16-column x 32-row FP32 buffers
 // ([column][row], 2 KB each), drained into C by TMA reduce-add
 constexpr int EPI_COLS = 16;
 constexpr int EPI_BUF = 32 * EPI_COLS * 4;
-constexpr int STAGING_OFF = STAGES * STAGE;
-constexpr int BAR_OFF = STAGING_OFF + EPI_WARPS * 2 * EPI_BUF;
-constexpr int NBAR = 2 * STAGES + 5;
-constexpr int TOTAL = BAR_OFF + 8 * NBAR + 16;
-constexpr int ALLOC = TOTAL + 1024;
-static_assert(ALLOC <= 232448, "shared memory of one CTA");
+// CG CTAs work on one tile of 128 CG x 256: each stages its own 128 rows of A
+// and its share of B's 256 rows, and holds its own rows of the accumulators.
+template <int CG>
+struct Ring {
+  static constexpr int B_ROWS = BN / CG;
+  static constexpr int A_SUB = BM * BK * 2;      // 16 KB
+  static constexpr int B_SUB = B_ROWS * BK * 2;  // 32 or 16 KB
+  static constexpr int STAGE = A_SUB + B_SUB;
+  static constexpr int STAGES = CG == 1 ? 4 : 6;
+  static constexpr int STAGING_OFF = STAGES * STAGE;
+  static constexpr int BAR_OFF = STAGING_OFF + EPI_WARPS * 2 * EPI_BUF;
+  static constexpr int NBAR = 2 * STAGES + 5;
+  static constexpr int TOTAL = BAR_OFF + 8 * NBAR + 16;
+  static constexpr int ALLOC = TOTAL + 1024;
+  static_assert(ALLOC <= 232448, "shared memory of one CTA");
+};
 
+// CTA pairs: address of the same shared-memory offset in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      " .reg .pred p;\n"
+      " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+      " selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// arrival on a barrier of the pair's first CTA (a shared::cluster address)
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// load into this CTA's shared memory, counted on a barrier of either CTA of the pair
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.cta_group::2"
+      " [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void mma_f16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      " .reg .pred p;\n"
+      " setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrives on the barrier at this offset in both CTAs once the MMAs issued so far are done
+__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+      "h"((uint16_t)3)
+      : "memory");
+}
+
+template <int CG>
 __device__ __forceinline__ bool wait_or_fail(uint32_t bar, uint32_t parity, volatile int* fail) {
   for (long long i = 0; i < WAIT_LIMIT; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (CG == 1 ? mbar_try_wait(bar, parity) : mbar_try_wait_cluster(bar, parity)) return true;
     if ((i & 63) == 63) {
       if (*fail) return false;
       __nanosleep(32);
@@ -357,27 +433,40 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+template <int CG>
 __global__ void __launch_bounds__(THREADS, 1)
 tc_gemm_update_ws(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                  const __grid_constant__ CUtensorMap tmC, int M, int N, int K, int T, int bf16, int* err) {
+                  const __grid_constant__ CUtensorMap tmC, int M, int N, int K, int T, int band, int bf16, int* err) {
+  using S = Ring<CG>;
+  constexpr int STAGES = S::STAGES;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (base - raw);
-  const uint32_t bar_full = base + BAR_OFF;
+  const uint32_t bar_full = base + S::BAR_OFF;
   const uint32_t bar_empty = bar_full + 8 * STAGES;
   const uint32_t bar_accf = bar_empty + 8 * STAGES;
   const uint32_t bar_acce = bar_accf + 16;
   const uint32_t bar_drain = bar_acce + 16;  // the MMA issuer's last commit: all its MMAs are done
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + BAR_OFF + 8 * NBAR);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + S::BAR_OFF + 8 * S::NBAR);
   __shared__ int s_fail;
   volatile int* fail = &s_fail;
+  // the pair's first CTA issues the MMAs of both; rank 0 of itself without a pair
+  const uint32_t rank = CG == 1 ? 0 : blockIdx.x & 1;
+  auto give_up = [&](int code) {  // ends the other CTA's waits too
+    atomicExch(&s_fail, code);
+    if constexpr (CG == 2)
+      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_rank(smem_u32(&s_fail), rank ^ 1)), "r"(code) : "memory");
+  };
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * BM;
-  const int tile0 = blockIdx.y * T;
   const int ntiles_n = (N + BN - 1) / BN;
+  const int ns = (ntiles_n + T - 1) / T;
+  int row_block, strip;
+  band_order(blockIdx.x, gridDim.x / ns, ns, band, &row_block, &strip);
+  const int m0 = row_block * BM;
+  const int tile0 = strip * T;
   const int nt = max(0, min(T, ntiles_n - tile0));
   const int KB = K / BK;
 
@@ -389,45 +478,63 @@ tc_gemm_update_ws(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     mbar_init(bar_accf, 1);
     mbar_init(bar_accf + 8, 1);
-    mbar_init(bar_acce, EPI_WARPS);
-    mbar_init(bar_acce + 8, EPI_WARPS);
+    mbar_init(bar_acce, CG * EPI_WARPS);
+    mbar_init(bar_acce + 8, CG * EPI_WARPS);
     mbar_init(bar_drain, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    if constexpr (CG == 1) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                   "r"(TMEM_COLS));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    } else {
+      asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                   "r"(TMEM_COLS));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if constexpr (CG == 2) cluster_sync();  // barriers and tensor memory of both are ready
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
     if (lane == 0) {
       // TMA producer over every (tile, K block) of the strip
+      // (a pair's loads all count on the first CTA's barriers)
       int g = 0;
       bool ok = true;
+      const uint32_t full = CG == 1 ? bar_full : map_rank(bar_full, 0);
       for (int t = 0; t < nt && ok; ++t) {
-        const int n0 = (tile0 + t) * BN;
+        const int n0 = (tile0 + t) * BN + (int)rank * S::B_ROWS;
         for (int kb = 0; kb < KB; ++kb, ++g) {
           const int st = g % STAGES, round = g / STAGES;
-          if (round > 0 && !wait_or_fail(bar_empty + 8 * st, (round - 1) & 1, fail)) {
-            atomicExch(&s_fail, 1);
+          if (round > 0 && !wait_or_fail<CG>(bar_empty + 8 * st, (round - 1) & 1, fail)) {
+            give_up(1);
             ok = false;
             break;
           }
-          const uint32_t sa = base + st * STAGE;
-          mbar_expect_tx(bar_full + 8 * st, (uint32_t)STAGE);
-          tma_load_2d(sa, &tmA, bar_full + 8 * st, kb * BK, m0);
-          tma_load_2d(sa + A_SUB, &tmB, bar_full + 8 * st, kb * BK, n0);
+          const uint32_t sa = base + st * S::STAGE;
+          if (rank == 0) mbar_expect_tx(bar_full + 8 * st, (uint32_t)(CG * S::STAGE));
+          if constexpr (CG == 1) {
+            tma_load_2d(sa, &tmA, full + 8 * st, kb * BK, m0);
+            tma_load_2d(sa + S::A_SUB, &tmB, full + 8 * st, kb * BK, n0);
+          } else {
+            tma_load_2d_pair(sa, &tmA, full + 8 * st, kb * BK, m0);
+            tma_load_2d_pair(sa + S::A_SUB, &tmB, full + 8 * st, kb * BK, n0);
+          }
         }
       }
       if (!ok || *fail) {
         // loads still in flight land in this CTA's shared memory: wait for
-        // each stage's last issued load (bounded) before the CTA may exit
-        for (int st = 0; st < STAGES && st < g; ++st) {
+        // each stage's last issued load (bounded) before the CTA may exit.  The
+        // second CTA of a pair has no barrier of its own for them: it gives
+        // them 2 ms, and then waits for the first CTA before it exits
+        if (rank != 0)
+          for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+        for (int st = 0; rank == 0 && st < STAGES && st < g; ++st) {
           const int last = g - 1 - ((g - 1 - st) % STAGES);
           const int round = last / STAGES;
           for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(bar_full + 8 * st, round & 1); ++i) {
@@ -436,14 +543,18 @@ tc_gemm_update_ws(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = idesc_f16(bf16 != 0, BM, BN);
+    if (lane == 0 && rank == 0) {
+      const uint32_t idesc = idesc_f16(bf16 != 0, CG * BM, BN);
+      auto commit = [](uint32_t bar) {
+        if constexpr (CG == 1) mma_commit(bar);
+        else mma_commit_pair(bar);
+      };
       int g = 0;
       bool ok = true;
       for (int t = 0; t < nt && ok; ++t) {
         const int a = t & 1, use = t >> 1;
-        if (use > 0 && !wait_or_fail(bar_acce + 8 * a, (use - 1) & 1, fail)) {
-          atomicExch(&s_fail, 2);
+        if (use > 0 && !wait_or_fail<CG>(bar_acce + 8 * a, (use - 1) & 1, fail)) {
+          give_up(2);
           ok = false;
           break;
         }
@@ -451,26 +562,27 @@ tc_gemm_update_ws(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         const uint32_t dacc = tmem + (uint32_t)(a * BN);
         for (int kb = 0; kb < KB; ++kb, ++g) {
           const int st = g % STAGES, round = g / STAGES;
-          if (!wait_or_fail(bar_full + 8 * st, round & 1, fail)) {
-            atomicExch(&s_fail, 3);
+          if (!wait_or_fail<CG>(bar_full + 8 * st, round & 1, fail)) {
+            give_up(3);
             ok = false;
             break;
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t sa = base + st * STAGE;
+          const uint32_t sa = base + st * S::STAGE;
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
             const uint64_t ad = smem_desc_sw128(sa + k * 32);
-            const uint64_t bd = smem_desc_sw128(sa + A_SUB + k * 32);
-            mma_f16(dacc, ad, bd, idesc, (kb | k) ? 1u : 0u);
+            const uint64_t bd = smem_desc_sw128(sa + S::A_SUB + k * 32);
+            if constexpr (CG == 1) mma_f16(dacc, ad, bd, idesc, (kb | k) ? 1u : 0u);
+            else mma_f16_pair(dacc, ad, bd, idesc, (kb | k) ? 1u : 0u);
           }
-          mma_commit(bar_empty + 8 * st);
+          commit(bar_empty + 8 * st);
         }
-        if (ok) mma_commit(bar_accf + 8 * a);
+        if (ok) commit(bar_accf + 8 * a);
       }
       // before the tensor memory may be released, every MMA issued here must
       // have completed (also after a failure, when no epilogue waited for them)
-      mma_commit(bar_drain);
+      commit(bar_drain);
       for (long long i = 0; i < WAIT_LIMIT && !mbar_try_wait(bar_drain, 0); ++i) {
         if (i > 64) __nanosleep(32);
       }
@@ -483,16 +595,17 @@ tc_gemm_update_ws(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     // while the last one drains.
     const int q = warp & 3, h = (warp - 2) >> 2;
     const int ew = warp - 2;
-    float* stg = reinterpret_cast<float*>(gbase + STAGING_OFF + ew * 2 * EPI_BUF);
-    const uint32_t stg_s = base + STAGING_OFF + ew * 2 * EPI_BUF;
+    float* stg = reinterpret_cast<float*>(gbase + S::STAGING_OFF + ew * 2 * EPI_BUF);
+    const uint32_t stg_s = base + S::STAGING_OFF + ew * 2 * EPI_BUF;
     constexpr int HALF = BN / 2;
     constexpr int NCH = HALF / EPI_COLS;
+    const uint32_t acce = CG == 1 ? bar_acce : map_rank(bar_acce, 0);
     int nbuf = 0;
     for (int t = 0; t < nt; ++t) {
       const int a = t & 1, use = t >> 1;
       const int nbase = (tile0 + t) * BN + h * HALF;
-      if (!wait_or_fail(bar_accf + 8 * a, use & 1, fail)) {
-        atomicExch(&s_fail, 4);
+      if (!wait_or_fail<CG>(bar_accf + 8 * a, use & 1, fail)) {
+        give_up(4);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -522,17 +635,31 @@ tc_gemm_update_ws(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       // this warp has read its part of accumulator a: hand it back to the MMA
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_acce + 8 * a);
+      if (lane == 0) {
+        if constexpr (CG == 1) mbar_arrive(acce + 8 * a);
+        else mbar_arrive_cluster(acce + 8 * a);
+      }
     }
     if (lane == 0) bulk_wait<0>();  // every reduce of this warp has completed
     __syncwarp();
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  // a pair: neither CTA frees its tensor memory or exits while the other may
+  // still read its operands or arrive on its barriers (the first CTA gets here
+  // only after bar_drain)
+  if constexpr (CG == 2) cluster_sync();
   if (threadIdx.x == 0 && s_fail != 0 && err) atomicExch(err, 1);
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+    if constexpr (CG == 1)
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+    else
+      asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+  }
+  if constexpr (CG == 2) {
+    __syncwarp();
+    cluster_sync();
   }
 }
 
@@ -600,7 +727,7 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
 
 __global__ void __launch_bounds__(THREADS3, 1)
 tc_gemm_update_split3(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                      const __grid_constant__ CUtensorMap tmC, int M, int N, int K, int T, int* err) {
+                      const __grid_constant__ CUtensorMap tmC, int M, int N, int K, int T, int band, int* err) {
   using namespace ws;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -617,9 +744,12 @@ tc_gemm_update_split3(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * BM;
-  const int tile0 = blockIdx.y * T;
   const int ntiles_n = (N + BN - 1) / BN;
+  const int ns = (ntiles_n + T - 1) / T;
+  int row_block, strip;
+  band_order(blockIdx.x, gridDim.x / ns, ns, band, &row_block, &strip);
+  const int m0 = row_block * BM;
+  const int tile0 = strip * T;
   const int nt = max(0, min(T, ntiles_n - tile0));
   const int KB = K / BK3;
 
@@ -657,7 +787,7 @@ tc_gemm_update_split3(const __grid_constant__ CUtensorMap tmA, const __grid_cons
           for (int i = 0; i < 3; ++i, ++g) {
             const int plane = i == 0 ? 0 : 3 - i;
             const int st = g % SLOTS, round = g / SLOTS;
-            if (round > 0 && !wait_or_fail(bar_empty + 8 * st, (round - 1) & 1, fail)) {
+            if (round > 0 && !wait_or_fail<1>(bar_empty + 8 * st, (round - 1) & 1, fail)) {
               atomicExch(&s_fail, 1);
               ok = false;
               break;
@@ -686,7 +816,7 @@ tc_gemm_update_split3(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       int g = 0, gc = 0;
       bool ok = true;
       auto full = [&](int slot_g) {
-        if (!wait_or_fail(bar_full + 8 * (slot_g % SLOTS), (slot_g / SLOTS) & 1, fail)) {
+        if (!wait_or_fail<1>(bar_full + 8 * (slot_g % SLOTS), (slot_g / SLOTS) & 1, fail)) {
           atomicExch(&s_fail, 3);
           return false;
         }
@@ -704,7 +834,7 @@ tc_gemm_update_split3(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 #pragma unroll
           for (int k = 0; k < BK3 / 16; ++k, ++gc) {
             const int a = gc & 1, use = gc >> 1;
-            if (use > 0 && !wait_or_fail(bar_acce + 8 * a, (use - 1) & 1, fail)) {
+            if (use > 0 && !wait_or_fail<1>(bar_acce + 8 * a, (use - 1) & 1, fail)) {
               atomicExch(&s_fail, 2);
               ok = false;
               break;
@@ -749,7 +879,7 @@ tc_gemm_update_split3(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       for (int c = 0; c < COLS / 2; ++c) sum[c] = make_float2(0.f, 0.f);
       for (int kb = 0; kb < K / 16; ++kb, ++gc) {
         const int a = gc & 1, use = gc >> 1;
-        if (!wait_or_fail(bar_accf + 8 * a, use & 1, fail)) {
+        if (!wait_or_fail<1>(bar_accf + 8 * a, use & 1, fail)) {
           atomicExch(&s_fail, 4);
           ok = false;
           break;
@@ -926,6 +1056,29 @@ constexpr int WS_TILES = 2;
 // other kernel remains for K = 64.
 constexpr int WS_MIN_K = 128;
 
+// CTA pairs take the far updates: from K = PAIR_MIN_K on, where the matrix
+// instructions and not C bound the update (one update at n = 8192 / 16384 /
+// 30720, against single CTAs: K = 2048 215 / 794 / 2740 against 222 / 864 / 3400
+// us, K = 1024 no difference, K = 128 112 / 409 / 1418 against 104 / 379 / 1325),
+// and with at least two tiles per SM (n = 2048, K = 2048: 19.6 against 18.8 us).
+// A pair stages two thirds of the bytes per product, so its CTAs can be fewer
+// and longer: four tiles each (the 16-bit solve at n = 32768: 58.6 ms with two,
+// 58.3 with four, 58.3 with eight; single CTAs 61.0, 60.4 with four), while
+// there are eight waves of them: below, the last wave costs more (one update of
+// n = 8192: 218 us with two, 232 with four).
+constexpr int PAIR_MIN_K = 2048;
+constexpr int PAIR_TILES = 4;
+// Row blocks of one band of a deep update's grid.  The CTAs in flight then work on
+// about as many rows as columns; in the order of whole columns they cover 20000
+// rows, and every strip reads all of A again from DRAM once A (126 MB at
+// n = 30720, K = 2048) does not stay in L2 beside C: 2990 us there, 2740 with
+// bands of 16 to 64 row blocks, and 59.1 -> 58.3 ms for the solve.  A shallow
+// 16-bit update keeps whole columns: its C traffic runs better in long ones
+// (n = 8192, K = 128: 104 us, 116 in bands).  The FP32 form takes bands at every
+// K (factorization of n = 32768: 123.5 -> 122.4 ms, 16384: 22.0 -> 21.9).
+constexpr int BAND = 32;
+
+
 // Streaming multiprocessors of the current device (cached per host thread and
 // device).
 static int sm_count() {
@@ -943,23 +1096,43 @@ static int sm_count() {
 // Tiles per CTA along N for a grid of ntm row blocks: WS_TILES, fewer while the
 // strips would not fill the GPU once (the 128-row block updates of the
 // left-looking panels).
-static int strip_tiles(int ntm, int ntn) {
-  int T = WS_TILES;
+static int strip_tiles(int ntm, int ntn, int T = WS_TILES) {
   while (T > 1 && (long long)ntm * ((ntn + T - 1) / T) < sm_count()) T >>= 1;
   return T;
 }
 
 static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, float* C, long long ldc, int M, int N, int K,
-                     int bf16, int* err, cudaStream_t s) {
+                     int bf16, bool pair, int* err, cudaStream_t s) {
   if (K >= WS_MIN_K && aligned16(C) && ldc % 4 == 0) {
     CUtensorMap mc;
     MPDOK_TRY(make_map_c(&mc, C, M, N, ldc, tc::ws::EPI_COLS));
-    MPDOK_TRY(set_smem(tc::ws::tc_gemm_update_ws, tc::ws::ALLOC));
     const int ntm = (M + tc::BM - 1) / tc::BM;
     const int ntn = (N + tc::BN - 1) / tc::BN;
-    const int T = strip_tiles(ntm, ntn);
-    dim3 grid(ntm, (ntn + T - 1) / T);
-    tc::ws::tc_gemm_update_ws<<<grid, tc::ws::THREADS, tc::ws::ALLOC, s>>>(ma, mb, mc, M, N, K, T, bf16, err);
+    if (pair) {
+      const int rows = 2 * ((ntm + 1) / 2);
+      const bool many = (long long)rows * (ntn / PAIR_TILES) >= 8LL * sm_count();
+      const int T = strip_tiles(rows, ntn, many ? PAIR_TILES : WS_TILES);
+      using R = tc::ws::Ring<2>;
+      MPDOK_TRY(set_smem(tc::ws::tc_gemm_update_ws<2>, R::ALLOC));
+      cudaLaunchAttribute at;
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim = {2, 1, 1};
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(rows * ((ntn + T - 1) / T));
+      cfg.blockDim = dim3(tc::ws::THREADS);
+      cfg.dynamicSmemBytes = R::ALLOC;
+      cfg.stream = s;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      MPDOK_CUDA_TRY(cudaLaunchKernelEx(&cfg, tc::ws::tc_gemm_update_ws<2>, ma, mb, mc, M, N, K, T,
+                                        BAND, bf16, err));
+    } else {
+      using R = tc::ws::Ring<1>;
+      const int T = strip_tiles(ntm, ntn);
+      MPDOK_TRY(set_smem(tc::ws::tc_gemm_update_ws<1>, R::ALLOC));
+      dim3 grid(ntm * ((ntn + T - 1) / T));
+      tc::ws::tc_gemm_update_ws<1><<<grid, tc::ws::THREADS, R::ALLOC, s>>>(ma, mb, mc, M, N, K, T, ntm, bf16, err);
+    }
     count_launch();
     MPDOK_LAUNCH_CHECK("tc_gemm_update_ws");
     return MPDOK_OK;
@@ -991,8 +1164,10 @@ int gemm_update(float* C, long long ldc, const void* A, const void* B, long long
     MPDOK_ARG_CHECK(aligned16(A) && aligned16(B) && (ldk * 2) % 16 == 0, "operands must be 16-byte aligned");
     CUtensorMap ma, mb;
     MPDOK_TRY(make_map(&ma, A, M, K, ldk, tc::BM, bf16));
-    MPDOK_TRY(make_map(&mb, B, N, K, ldk, tc::BN, bf16));
-    MPDOK_TRY(launch_tc(ma, mb, C, ldc, M, N, K, bf16, err, s));
+    const long long tiles = (long long)((M + tc::BM - 1) / tc::BM) * ((N + tc::BN - 1) / tc::BN);
+    const bool pair = deep && M > tc::BM && K >= PAIR_MIN_K && tiles >= 2LL * sm_count();
+    MPDOK_TRY(make_map(&mb, B, N, K, ldk, pair ? tc::ws::Ring<2>::B_ROWS : tc::BN, bf16));
+    MPDOK_TRY(launch_tc(ma, mb, C, ldc, M, N, K, bf16, pair, err, s));
   }
   prof_stop(slot, s, 2.0 * (double)M * (double)N * (double)K);
   // C read and written in FP32, both 16-bit operands read once
@@ -1017,8 +1192,8 @@ int gemm_update_split3(float* C, long long ldc, const __nv_bfloat16* A, const __
   MPDOK_TRY(set_smem(tc::split3::tc_gemm_update_split3, tc::split3::ALLOC));
   const int ntm = (M + tc::BM - 1) / tc::BM, ntn = (N + tc::BN - 1) / tc::BN;
   const int T = strip_tiles(ntm, ntn);
-  dim3 grid(ntm, (ntn + T - 1) / T);
-  tc::split3::tc_gemm_update_split3<<<grid, tc::split3::THREADS3, tc::split3::ALLOC, s>>>(ma, mb, mc, M, N, K, T, err);
+  dim3 grid(ntm * ((ntn + T - 1) / T));
+  tc::split3::tc_gemm_update_split3<<<grid, tc::split3::THREADS3, tc::split3::ALLOC, s>>>(ma, mb, mc, M, N, K, T, BAND, err);
   count_launch();
   MPDOK_LAUNCH_CHECK("tc_gemm_update_split3");
   prof_stop(slot, s, 2.0 * (double)M * (double)N * (double)K);
