@@ -274,6 +274,11 @@ MPDOK_API size_t mpdok_lu_factor_size(long long n, int fdtype);
 MPDOK_API size_t mpdok_lu_work_size(long long n, int fdtype);
 MPDOK_API int mpdok_lu_factor(const double* A, long long lda, long long n, int fdtype, int pivoting, void* factors,
                               size_t factor_bytes, void* work, size_t work_bytes, cudaStream_t stream);
+/* The same, and A32 (n x n, lda32) receives A rounded to FP32, the operator of
+ * mpdok_lu_gmres_ir, from the pass that scales A (A32 NULL: no copy). */
+MPDOK_API int mpdok_lu_factor_copy(const double* A, long long lda, long long n, int fdtype, int pivoting,
+                                   void* factors, size_t factor_bytes, void* work, size_t work_bytes, float* A32,
+                                   long long lda32, cudaStream_t stream);
 /* The launch schedule of mpdok_lu_factor for n and fdtype, host only (no
  * device call): every launch, event record and event wait across its three
  * streams (0 caller's, 1 chain, 2 strip), in issue order.  12 integers per

@@ -35,7 +35,7 @@ def _info(info: N.SolveInfo) -> dict:
 class LUFactorization:
     """Factors of one dense matrix, owned in a device buffer."""
 
-    def __init__(self, A, dtype: str = "fp16", pivoting: bool = False, work: Workspace | None = None):
+    def __init__(self, A, dtype: str = "fp16", pivoting: bool = False, work: Workspace | None = None, *, _a32=None):
         """pivoting=False: W = D A D with D = diag(1/sqrt|a_ii|), no row exchanges
         (SPD / diagonally dominant systems; tiny pivots perturbed, counted in
         ``n_perturbed``).  pivoting=True: power-of-two row / column
@@ -51,8 +51,9 @@ class LUFactorization:
                                    device=A64.device)
         ws = work or Workspace()
         w = ws.get(lib.mpdok_lu_work_size(n, self.fdtype))
-        st = lib.mpdok_lu_factor(ptr(A64), n, n, self.fdtype, 1 if self.pivoting else 0, ptr(self.factors),
-                                 self.factors.numel(), ptr(w), w.numel(), stream_handle())
+        # _a32: an (n, n) FP32 tensor that receives A rounded, from the pass that scales A
+        st = lib.mpdok_lu_factor_copy(ptr(A64), n, n, self.fdtype, 1 if self.pivoting else 0, ptr(self.factors),
+                                      self.factors.numel(), ptr(w), w.numel(), ptr(_a32), n, stream_handle())
         N.check(st, "lu_factor")
         self.n_perturbed = 0 if self.pivoting else int(st)
         self.info = int(st) if self.pivoting else 0

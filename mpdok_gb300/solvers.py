@@ -87,9 +87,7 @@ class MixedSolver:
         from .lu import LUFactorization
         ev = [torch.cuda.Event(enable_timing=True) for _ in range(3)]
         ev[0].record()
-        if not a32_ready:
-            N.check(lib.mpdok_convert(ptr(A64), N.F64, ptr(self._a32), N.F32, n * n, stream_handle()), "convert")
-        lu = LUFactorization(A64, dtype=self.factor_dtype, work=self._fws)
+        lu = LUFactorization(A64, dtype=self.factor_dtype, work=self._fws, _a32=None if a32_ready else self._a32)
         ev[1].record()
         x, d = lu.gmres_ir(A64, b64, A32=self._a32, tol=tol, maxiter_outer=self.maxiter_outer,
                            restart=self.restart, inner_tol=self.inner_tol)
