@@ -432,6 +432,20 @@ int gemv_launch(int a_dtype, bool trans, const void* A, long long lda, long long
   return MPDOK_OK;
 }
 
+int gemv_partials_f32(const float* A, long long lda, long long m, long long n, const float* x, void* work,
+                      size_t work_bytes, cudaStream_t s, const int* skip, const float** P, int* S) {
+  MPDOK_ARG_CHECK(m >= 1 && n >= 1 && lda >= m, "bad GEMV shape / lda");
+  const GemvPlan p = plan_gemv(MPDOK_F32, m, n, 1, false);
+  MPDOK_ARG_CHECK(work != nullptr && work_bytes >= p.total_bytes, "GEMV workspace too small");
+  const int pslot = prof_start(MPDOK_PROF_GEMV_F32, s);
+  launch_stage1<float, 1>(false, p, A, lda, m, n, x, n, work, aligned16(A) && lda % 4 == 0, skip, s);
+  prof_stop(pslot, s, (double)m * (double)n * 4 + (double)(m + n) * 4, skip);
+  MPDOK_LAUNCH_CHECK("gemv stage1");
+  *P = (const float*)work;
+  *S = p.S;
+  return MPDOK_OK;
+}
+
 size_t gemv_workspace_bytes(int a_dtype, long long m, long long n, int nrhs, bool trans) {
   size_t best = 0;
   for (int K : {1, 2, 4, 8}) {

@@ -66,6 +66,11 @@ int gemv_launch(int a_dtype, bool trans, const void* A, long long lda, long long
                 const void* Bsrc, long long ldb, double* nrm2, void* work, size_t work_bytes,
                 cudaStream_t s, bool zero_ticket, const int* skip = nullptr);
 
+// The FP32 product y = A x of one column left as *S partial sums, *P = [S][m] in
+// `work`, for a consumer that adds them (in gemv_finalize's order).
+int gemv_partials_f32(const float* A, long long lda, long long m, long long n, const float* x, void* work,
+                      size_t work_bytes, cudaStream_t s, const int* skip, const float** P, int* S);
+
 size_t gemv_workspace_bytes(int a_dtype, long long m, long long n, int nrhs, bool trans);
 
 }  // namespace mpdok

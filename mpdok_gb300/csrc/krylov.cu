@@ -62,7 +62,10 @@ struct ArnState {
 // from the second pass instead (||w||^2 - ||h2||^2, right to 1e-8) would spare
 // that barrier, but a stagnating restarted solve then leaves the reference's
 // trajectory.  n = 8192, 1 to 50 columns: 26.4 us per step on average, the four
-// kernels that it replaces 50 us and three more launches.
+// kernels that it replaces 50 us and three more launches.  A stored operator
+// leaves w as the split sums of its product, and the step adds them where it
+// stages w: 29.2 us, against 27.2 and a launch of 6.0 us that only did that
+// (GMRES-IR of n = 8192, 350 steps: 30.5 -> 28.4 ms).
 constexpr int AT = 512;              // threads
 constexpr int A_SUB = 1024;          // rows staged at a time
 constexpr int A_SL = 4;              // row slices of the dot products
@@ -98,6 +101,8 @@ struct ArnStep {
   double tol_rel;
   int passes;
   int* hdone;        // pinned host copy of the done flag after this step, or null
+  const float* P;    // w as the S partial sums ([S][n]) of its product, or null: w is there
+  int S;
 };
 
 // The previous rotations on the new column h (in place), by one warp: the
@@ -330,7 +335,29 @@ __global__ void __launch_bounds__(AT, 1) k_arnoldi_step(ArnStep p, ArnState st, 
   for (int s0 = 0; s0 < rows; s0 += A_SUB) {
     const int len = min(A_SUB, rows - s0);
     __syncthreads();
-    for (int i = tid; i < len; i += AT) sw[i] = (double)p.w[r0 + s0 + i];
+    if (p.P == nullptr) {
+      for (int i = tid; i < len; i += AT) sw[i] = (double)p.w[r0 + s0 + i];
+    } else {
+      // four threads to a row, every fourth split each, as gemv_finalize adds them
+      const int r = tid % (AT / 4), q = tid / (AT / 4);
+      for (int i0 = 0; i0 < len; i0 += AT / 4) {
+        const int i = i0 + r;
+        float sum = 0.f;
+        if (i < len) {
+          const float* pp = p.P + r0 + s0 + i;
+#pragma unroll 8
+          for (int u = q; u < p.S; u += 4) sum += pp[u * p.n];
+        }
+        spart[tid] = sum;
+        __syncthreads();
+        if (q == 0 && i < len) {
+          sum = ((sum + spart[AT / 4 + r]) + spart[AT / 2 + r]) + spart[3 * (AT / 4) + r];
+          p.w[r0 + s0 + i] = sum;
+          sw[i] = (double)sum;
+        }
+        __syncthreads();
+      }
+    }
     __syncthreads();
     dots(s0, len);
   }
@@ -856,6 +883,12 @@ static int stored_apply32(const void* ctx, const float* x, float* y, int nrhs, l
                      nullptr, c->gw, c->gbytes, s, false, skip);
 }
 
+static int stored_partials32(const void* ctx, const float* x, cudaStream_t s, const int* skip, const float** P,
+                             int* S) {
+  const StoredCtx* c = (const StoredCtx*)ctx;
+  return gemv_partials_f32(c->A32, c->lda32, c->n, c->n, x, c->gw, c->gbytes, s, skip, P, S);
+}
+
 static int stored_residual64(const void* ctx, const double* b, const double* x, double* r, double* nrm2, int nrhs,
                              long long ld, cudaStream_t s) {
   const StoredCtx* c = (const StoredCtx*)ctx;
@@ -870,6 +903,7 @@ static int stored_residual64(const void* ctx, const double* b, const double* x, 
 Operator32 stored_op32(const StoredCtx* c) {
   Operator32 o;
   o.apply = stored_apply32;
+  o.partials = stored_partials32;
   o.ctx = c;
   return o;
 }
@@ -958,9 +992,12 @@ int arnoldi_cycle(const KWs& ws, const Operator32& A, int m, int reorth, double 
       MPDOK_TRY(pc->apply(pc->ctx, vk, zk, s, &ws.sc->done));
       opnd = zk;
     }
-    MPDOK_TRY(A.apply(A.ctx, opnd, ws.w, 1, ws.ldv, s, &ws.sc->done));
+    const float* parts = nullptr;
+    int S = 0;
+    if (A.partials) MPDOK_TRY(A.partials(A.ctx, opnd, s, &ws.sc->done, &parts, &S));
+    else MPDOK_TRY(A.apply(A.ctx, opnd, ws.w, 1, ws.ldv, s, &ws.sc->done));
     ArnStep step{ws.V, ws.ldv, k + 1, ws.w, ws.V + (long long)(k + 1) * ws.ldv, n, (int)ws.ch, ws.parts, ws.tickets,
-                 tol_rel, reorth, poll ? &pp->flag[k & 1] : nullptr};
+                 tol_rel, reorth, poll ? &pp->flag[k & 1] : nullptr, parts, S};
     ArnState state = st;
     KScal* sc = ws.sc;
     void* args[] = {&step, &state, &sc};

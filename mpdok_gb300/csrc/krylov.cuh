@@ -58,6 +58,9 @@ struct Operator32 {
   int (*apply)(const void* ctx, const float* x, float* y, int nrhs, long long ld, cudaStream_t s,
                const int* skip) = nullptr;
   const void* ctx = nullptr;
+  // optional, one column: y left as S partial sums ([S][n], in the operator's
+  // workspace until its next product), which an Arnoldi step adds itself
+  int (*partials)(const void* ctx, const float* x, cudaStream_t s, const int* skip, const float** P, int* S) = nullptr;
 };
 
 // FP64 residual r = b - A x (nrhs columns, leading dimension ld) with
