@@ -775,23 +775,30 @@ __global__ void k_badd(double* __restrict__ X, const double* __restrict__ D, lon
 // p; the Gaussian p runs on the integer pipe (phi64.cuh).  NR, the number of
 // right-hand sides rounded up to a power of two, is compiled in: eight columns
 // for a single one were 28 of 46 operations (n = 6000, D = 2, one column:
-// 4.60 ms for all eight with CUDA's exp, 1.13 ms now).  Four threads per row split the columns; their
-// partial sums combine by shuffles in a fixed order.
-template <int KIND, int D, int NR>
+// 4.60 ms for all eight with CUDA's exp, 1.13 ms with this rule and the tables).
+// A block of 64 rows goes to one CTA, or to SP of them where the blocks would
+// not fill the SMs twice (one system of n = 6000 has 94 blocks for 152 SMs:
+// 1.13 -> 0.79 ms); five and more right-hand sides stay at one CTA, whose staged
+// columns fill the shared memory that four would need.
+// 4 SP threads per row split the columns; their partial sums combine by shuffles
+// in a fixed order.
+template <int KIND, int D, int NR, int SP>
 __global__ void __launch_bounds__(BT) k_badjoint(const BSys* __restrict__ sys, const long long* __restrict__ pre,
                                                  int nsys, int nrhs, const double* __restrict__ coords,
                                                  const double* __restrict__ X, const double* __restrict__ Lam,
                                                  double* __restrict__ gC, double* __restrict__ rowscr) {
   __shared__ uint64_t sPhi[KIND == MPDOK_KERNEL_GAUSSIAN ? PHI_TAB : 1];
-  __shared__ double sC[BNB * D];
-  __shared__ double sXj[NR * BNB], sLj[NR * BNB];
+  constexpr int Q = 4 * SP;       // threads per row
+  constexpr int CB = BNB * SP;    // columns staged at a time: sixteen per thread
+  __shared__ double sC[CB * D];
+  __shared__ double sXj[NR * CB], sLj[NR * CB];
   if constexpr (KIND == MPDOK_KERNEL_GAUSSIAN) phi_table(sPhi);
-  const long long t = blockIdx.x;
+  const long long t = blockIdx.x / SP;
   const int s = task_system(pre, nsys + 1, t);
   const BSys q = sys[s];
   const int r = (int)(t - pre[s]);
   const int r0 = r * BNB;
-  const int lr = threadIdx.x >> 2, part = threadIdx.x & 3;
+  const int lr = (int)(blockIdx.x % SP) * (BNB / SP) + threadIdx.x / Q, part = threadIdx.x % Q;
   const int k = r0 + lr;
   const bool live = k < q.n;
   const double* Cb = coords + q.offC;
@@ -806,12 +813,12 @@ __global__ void __launch_bounds__(BT) k_badjoint(const BSys* __restrict__ sys, c
   double G[D], E = 0.0;
 #pragma unroll
   for (int d = 0; d < D; ++d) G[d] = 0.0;
-  for (int c = 0; c < q.nblk; ++c) {
-    const int c0 = c * BNB, nc = min(BNB, q.n - c0);
+  for (int c0 = 0; c0 < q.n; c0 += CB) {
+    const int nc = min(CB, q.n - c0);
     __syncthreads();
-    for (int e = threadIdx.x; e < BNB * D; e += BT) sC[e] = (e / D < nc) ? Cb[(long long)c0 * D + e] : 0.0;
-    for (int e = threadIdx.x; e < BNB * NR; e += BT) {
-      const int j = e % BNB, rr = e / BNB;
+    for (int e = threadIdx.x; e < CB * D; e += BT) sC[e] = (e / D < nc) ? Cb[(long long)c0 * D + e] : 0.0;
+    for (int e = threadIdx.x; e < CB * NR; e += BT) {
+      const int j = e % CB, rr = e / CB;
       const bool ok = j < nc && rr < nrhs;
       sXj[e] = ok ? X[q.offX + c0 + j + (long long)rr * q.n] : 0.0;
       sLj[e] = ok ? Lam[q.offX + c0 + j + (long long)rr * q.n] : 0.0;
@@ -819,7 +826,7 @@ __global__ void __launch_bounds__(BT) k_badjoint(const BSys* __restrict__ sys, c
     __syncthreads();
     if (!live) continue;
 #pragma unroll 2
-    for (int j = part; j < nc; j += 4) {
+    for (int j = part; j < nc; j += Q) {
       double df[D], r2 = 0.0;
 #pragma unroll
       for (int d = 0; d < D; ++d) {
@@ -831,8 +838,8 @@ __global__ void __launch_bounds__(BT) k_badjoint(const BSys* __restrict__ sys, c
       double w = 0.0;
 #pragma unroll
       for (int rr = 0; rr < NR; ++rr) {
-        w = fma(lk[rr], sXj[rr * BNB + j], w);
-        w = fma(xk[rr], sLj[rr * BNB + j], w);
+        w = fma(lk[rr], sXj[rr * CB + j], w);
+        w = fma(xk[rr], sLj[rr * CB + j], w);
       }
       w *= p;
 #pragma unroll
@@ -840,9 +847,9 @@ __global__ void __launch_bounds__(BT) k_badjoint(const BSys* __restrict__ sys, c
       E = fma(w, r2, E);
     }
   }
-  // combine the four column parts (lanes 4m .. 4m+3) in a fixed order
+  // combine the column parts (Q neighbouring lanes) in a fixed order
 #pragma unroll
-  for (int o = 1; o < 4; o <<= 1) {
+  for (int o = 1; o < Q; o <<= 1) {
 #pragma unroll
     for (int d = 0; d < D; ++d) G[d] += __shfl_xor_sync(0xffffffffu, G[d], o);
     E += __shfl_xor_sync(0xffffffffu, E, o);
@@ -864,9 +871,13 @@ template <int KIND, int D>
 static void launch_badjoint(unsigned grid, const BSys* sys, const long long* pre, int nsys, int nrhs,
                             const double* coords, const double* X, const double* Lam, double* gC, double* rowscr,
                             cudaStream_t s) {
-  auto* kern = nrhs == 1 ? k_badjoint<KIND, D, 1> : nrhs == 2 ? k_badjoint<KIND, D, 2>
-               : nrhs <= 4 ? k_badjoint<KIND, D, 4> : k_badjoint<KIND, D, BMAX_RHS>;
-  launch(kern, dim3(grid), BT, 0, s, sys, pre, nsys, nrhs, coords, X, Lam, gC, rowscr);
+  constexpr int SP = 4;
+  const bool split = (long long)grid < 2LL * num_sms();
+  auto* kern = nrhs == 1 ? (split ? k_badjoint<KIND, D, 1, SP> : k_badjoint<KIND, D, 1, 1>)
+               : nrhs == 2 ? (split ? k_badjoint<KIND, D, 2, SP> : k_badjoint<KIND, D, 2, 1>)
+               : nrhs <= 4 ? (split ? k_badjoint<KIND, D, 4, SP> : k_badjoint<KIND, D, 4, 1>)
+                           : k_badjoint<KIND, D, BMAX_RHS, 1>;
+  launch(kern, dim3(grid * (split && nrhs <= 4 ? SP : 1)), BT, 0, s, sys, pre, nsys, nrhs, coords, X, Lam, gC, rowscr);
 }
 
 // Per system: grad_eps = sum_k partial, grad_reg = sum_k partial (fixed order).
