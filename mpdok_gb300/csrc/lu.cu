@@ -1505,9 +1505,11 @@ __device__ void piv_moves(const int* s_piv, long long jp, int nb, int* plan) {
 // Up to 16 CTAs (384 rows each, one thread to a row) hold the panel in shared
 // memory and meet at one hardware cluster barrier per column; candidates and
 // rows travel through distributed shared memory.  Panels of up to 6144 rows
-// take it: a column costs about 1.5 us against 4.7 us behind a grid barrier in
-// global memory (n = 5000: 9.5 against 24.2 ms for the 40 panels, 238 against
-// 604 us each).  Taller ones do not fit a cluster's shared memory and take
+// take it: a column costs about 1.6 us against 4.7 us behind a grid barrier in
+// global memory (n = 5000: 8.8 against 24.2 ms for the 40 panels, 220 against
+// 604 us each).  Of its 3700 cycles the barrier takes 1500 (800 with four CTAs),
+// the rows' copies 430, the argmax 370, the elimination 560, the columns right
+// of the sub-panel 690.  Taller ones do not fit a cluster's shared memory and take
 // k_getf2.
 //
 // Columns are worked off in sub-panels of 32: a thread holds its row's 32
@@ -1521,7 +1523,7 @@ constexpr int CL_MAX = 16;
 constexpr int CL_SUB = 32;
 
 __host__ __device__ constexpr size_t getf2_cluster_smem(int R) {
-  return ((size_t)LNB * (R + 1) + (LNB - CL_SUB) * CL_SUB + 6 * CL_SUB + 6 * LNB) * sizeof(float);
+  return ((size_t)LNB * (R + 1) + (LNB - CL_SUB) * CL_SUB + (2 * CL_MAX + 4) * CL_SUB + 4 * LNB) * sizeof(float);
 }
 
 __device__ __forceinline__ unsigned cl_map(const void* p, unsigned rank) {
@@ -1537,6 +1539,13 @@ __device__ __forceinline__ float cl_ld(unsigned a) {
 __device__ __forceinline__ void cl_st(unsigned a, unsigned long long v) {
   asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
 }
+__device__ __forceinline__ void cl_st4(unsigned a, float4 v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+               : "memory");
+}
+__device__ __forceinline__ void cl_st(unsigned a, int v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
 // every thread of every CTA of the cluster; releases and acquires shared memory
 __device__ __forceinline__ void cl_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -1548,34 +1557,75 @@ k_getf2_cluster(float* __restrict__ W, long long ldw, long long n, long long jp,
                 int* __restrict__ ipiv, int* info, int* plan) {
   extern __shared__ __align__(16) float csm[];
   float* Us = csm;                                  // [LNB - 32][32]: a sub-panel's U rows, by column
-  // rows in transit: the entries j .. of the sub-panel as 32 aligned floats (c..),
-  // the columns outside the sub-panel at their own places
-  float* csub = Us + (LNB - CL_SUB) * CL_SUB;       // [2][32]: this CTA's candidate
-  float* tsub = csub + 2 * CL_SUB;                  // [2][32]: the row at position j (CTA 0)
-  float* s_v = tsub + 2 * CL_SUB;                   // [32]: the pivot row
-  float* s_w = s_v + CL_SUB;                        // [32]: the row that it replaces
-  float* crow = s_w + CL_SUB;                       // [2][LNB]: this CTA's candidate
+  // rows in transit: the entries j .. of the sub-panel as 32 aligned floats, sent
+  // to every CTA before the barrier; the columns outside the sub-panel at their
+  // own places, fetched after it by the two CTAs that need them
+  float* sv = Us + (LNB - CL_SUB) * CL_SUB;         // [2][CL_MAX][32]: each CTA's candidate
+  float* sw = sv + 2 * CL_MAX * CL_SUB;             // [2][32]: the row at position j (from CTA 0)
+  float* cstage = sw + 2 * CL_SUB;                  // [32], [32]: the two on their way out
+  float* tstage = cstage + CL_SUB;
+  float* crow = tstage + CL_SUB;                    // [2][LNB]: this CTA's candidate
   float* top = crow + 2 * LNB;                      // [2][LNB]: the row at position j (CTA 0)
-  float* s_u = top + 2 * LNB;                       // [LNB]: the pivot row
-  float* s_t = s_u + LNB;                           // [LNB]: the row that it replaces
-  float* P = s_t + LNB;                             // [nb][RS]: this CTA's rows
+  float* P = top + 2 * LNB;                         // [nb][RS]: this CTA's rows
   const int RS = R + 1;                             // (odd: rows and columns both conflict-free)
   __shared__ unsigned long long cand[2][CL_MAX];
   __shared__ unsigned s_key[CL_THREADS / 32];
   __shared__ int s_row[CL_THREADS / 32];
-  __shared__ int corg[2], torg[2], s_org[2];  // where the rows in transit came from: candidate, position j; as read
+  __shared__ int corg[2][CL_MAX], torg[2];  // where the rows in transit came from
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int C = gridDim.x, g = blockIdx.x;
   const int rows = (int)max(0LL, min((long long)R, n - jp - (long long)g * R));
   const int pos = g * R + t;                        // this thread's position in the panel
   const bool mine = t < rows;
   int org = pos;                                    // the position this thread's row came from
+  // the row of lane `src` of this warp, from its registers to dst / odst of every CTA
+  auto send = [&](const float (&x)[CL_SUB], int src, float* stage, float* dst, int* odst) {
+    float4* st = reinterpret_cast<float4*>(stage);
+    if (lane == src)
+#pragma unroll
+      for (int c = 0; c < CL_SUB; c += 4) st[c / 4] = make_float4(x[c], x[c + 1], x[c + 2], x[c + 3]);
+    const int o = __shfl_sync(0xffffffffu, org, src);
+    __syncwarp();
+    const int to = lane >> 1, half = lane & 1;
+    if (to < C) {
+      const unsigned a = cl_map(dst + half * (CL_SUB / 2), to);
+#pragma unroll
+      for (int i = 0; i < CL_SUB / 8; ++i) cl_st4(a + 16 * i, st[half * (CL_SUB / 8) + i]);
+      if (half == 0) cl_st(cl_map(odst, to), o);
+    }
+  };
+  // entries of the rows exchanged at the last column, of this thread's column:
+  // fetched then, stored one column later, when they have arrived
+  float pend_u = 0.f, pend_t = 0.f;
+  int at_u = -1, at_t = -1;
+  auto settle = [&]() {
+    if (at_u >= 0) P[t * RS + at_u] = pend_u;
+    if (at_t >= 0) P[t * RS + at_t] = pend_t;
+    at_u = at_t = -1;
+  };
   if (g == 0 && t == 0) plan[0] = 0;
-  for (int e = t; e < nb * R; e += CL_THREADS) {
-    const int c = e / R, r = e % R;
-    P[c * RS + r] = r < rows ? W[(jp + pos - t + r) + (jp + c) * ldw] : 0.f;
+  // a warp per two columns, all their loads in flight (one element at a time the
+  // load took 48000 of a panel's 570000 cycles)
+  constexpr int LR = CL_RMAX / 32;
+  for (int c = 2 * warp; c < nb; c += 2 * (CL_THREADS / 32)) {
+    const float* src = W + jp + (long long)g * R + (jp + c) * ldw;
+    float v[2][LR];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < LR; ++i) {
+        const int r = lane + 32 * i;
+        v[h][i] = r < rows && c + h < nb ? src[h * ldw + r] : 0.f;
+      }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < LR; ++i) {
+        const int r = lane + 32 * i;
+        if (r < R && c + h < nb) P[(c + h) * RS + r] = v[h][i];
+      }
   }
-  __syncthreads();
+  cl_sync();  // (every CTA has started before any writes into another)
   for (int s0 = 0; s0 < nb; s0 += CL_SUB) {
     const int se = min(s0 + CL_SUB, nb);
     float x[CL_SUB];  // columns j .. of this row (zero or unused past the sub-panel)
@@ -1601,22 +1651,9 @@ k_getf2_cluster(float* __restrict__ W, long long ldw, long long n, long long jp,
       const int lw = s_row[__ffs(bal) - 1];
       // publish the candidate's row and the row at position j
       const bool outside = t < nb && (t < j || t >= se);
-      if (t == lw || (g == 0 && t == j)) {
-        float4 v[CL_SUB / 4];
-#pragma unroll
-        for (int c = 0; c < CL_SUB; c += 4) v[c / 4] = make_float4(x[c], x[c + 1], x[c + 2], x[c + 3]);
-        float4* a = reinterpret_cast<float4*>(csub + q * CL_SUB);
-        float4* b = reinterpret_cast<float4*>(tsub + q * CL_SUB);
-        if (t == lw)
-#pragma unroll
-          for (int c = 0; c < CL_SUB / 4; ++c) a[c] = v[c];
-        if (t == lw) corg[q] = org;
-        if (g == 0 && t == j) {
-          torg[q] = org;
-#pragma unroll
-          for (int c = 0; c < CL_SUB / 4; ++c) b[c] = v[c];
-        }
-      }
+      if (warp == lw >> 5) send(x, lw & 31, cstage, sv + (q * CL_MAX + g) * CL_SUB, &corg[q][g]);
+      if (g == 0 && warp == j >> 5) send(x, j & 31, tstage, sw + q * CL_SUB, &torg[q]);
+      settle();
       if (outside) {
         crow[q * LNB + t] = P[t * RS + lw];
         if (g == 0) top[q * LNB + t] = P[t * RS + j];
@@ -1629,13 +1666,6 @@ k_getf2_cluster(float* __restrict__ W, long long ldw, long long n, long long jp,
       bal = __ballot_sync(0xffffffffu, lane < C && key == m);
       const int wc = __ffs(bal) - 1;
       const int wr = __shfl_sync(0xffffffffu, (int)(unsigned)cv, wc);
-      if (outside) s_u[t] = cl_ld(cl_map(crow + q * LNB + t, wc));
-      else if (warp == 4) s_v[lane] = cl_ld(cl_map(csub + q * CL_SUB + lane, wc));
-      else if (warp == 5) s_w[lane] = cl_ld(cl_map(tsub + q * CL_SUB + lane, 0));
-      else if (warp == 6 && lane < 2)
-        s_org[lane] = __float_as_int(cl_ld(lane == 0 ? cl_map(corg + q, wc) : cl_map(torg + q, 0)));
-      else if (t >= 2 * LNB && t < 2 * LNB + nb) s_t[t - 2 * LNB] = cl_ld(cl_map(top + q * LNB + t - 2 * LNB, 0));
-      __syncthreads();
       const bool zero = m <= 1u;
       if (g == 0 && t == 0) {
         ipiv[jp + j] = (int)jp + (zero ? j : wr);
@@ -1653,14 +1683,25 @@ k_getf2_cluster(float* __restrict__ W, long long ldw, long long n, long long jp,
         for (int c = 0; c + 1 < CL_SUB; ++c) x[c] = x[c + 1];
         continue;
       }
-      if (g == 0 && t < nb) P[t * RS + j] = outside ? s_u[t] : s_v[t - j];
-      if (g == 0 && t == j) org = s_org[0];
+      const float* s_v = sv + (q * CL_MAX + wc) * CL_SUB;  // the pivot row
+      if (g == 0 && t < nb) {
+        if (outside) {
+          pend_u = cl_ld(cl_map(crow + q * LNB + t, wc));
+          at_u = j;
+        } else {
+          P[t * RS + j] = s_v[t - j];
+        }
+      }
+      if (g == 0 && t == j) org = corg[q][wc];
       if (wr != j && g == wc) {  // the winner's row takes the content of position j
         const int l = wr - g * R;
-        if (outside) P[t * RS + l] = s_t[t];
+        if (outside) {
+          pend_t = cl_ld(cl_map(top + q * LNB + t, 0));
+          at_t = l;
+        }
         if (t == l) {
-          org = s_org[1];
-          const float4* b = reinterpret_cast<const float4*>(s_w);
+          org = torg[q];
+          const float4* b = reinterpret_cast<const float4*>(sw + q * CL_SUB);
 #pragma unroll
           for (int c = 0; c < CL_SUB; c += 4) {
             const float4 v = b[c / 4];
@@ -1682,6 +1723,7 @@ k_getf2_cluster(float* __restrict__ W, long long ldw, long long n, long long jp,
         for (int c = 0; c + 1 < CL_SUB; ++c) x[c] = fmaf(-l, v[c + 1], x[c + 1]);
       }
     }
+    settle();
     if (se < nb) {
       // the sub-panel's rows of U in the columns to the right (CTA 0 holds them:
       // R >= 128 where there is more than one CTA), a thread per column
