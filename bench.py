@@ -49,7 +49,7 @@ def _peaks():
 # the kernels behind the profiled classes
 KERNEL_NAMES = {
     "lu_gemm_deep": "tc::ws::tc_gemm_update_ws (the 16-bit factorization's tcgen05 trailing updates, K >= 128)",
-    "lu_gemm": "k_gemm_update_f32 (FP32 factors) and tc::tc_gemm_update (K = 64)",
+    "lu_gemm": "tc::split3::tc_gemm_update_split3 (FP32 factors) and tc::tc_gemm_update (K = 64)",
     "lu_panel": "k_lu_diag + k_trsm_pair (the chain and below-panel windows)",
     "trsv": "k_trsv + k_scale_out",
     "gemv_f32": "gemv_n_stage1 (FP32 and 16-bit stored operator)",
