@@ -3114,9 +3114,10 @@ __global__ void k_add_f32_cols(const float* __restrict__ e32, double* __restrict
 // steps it would take alone.
 static int lu_ir_groups(const double* A, long long lda, long long n, const void* factors, int fdtype, int K, int ng,
                         const double* B, long long ldb, double* X, long long ldx, double tol, int maxiter_outer,
-                        void* work, mpdok_solve_info* infos, cudaStream_t s) {
+                        void* work, size_t work_bytes, mpdok_solve_info* infos, cudaStream_t s) {
   const int nc = K * ng;
   const MultiWork mw = multi_layout(n, nc);
+  MPDOK_ARG_CHECK(work_bytes >= mw.total, "multi-RHS LU-IR work buffer too small");
   char* wb = (char*)work;
   float* y = (float*)(wb + mw.off_y);
   float* zz = (float*)(wb + mw.off_z);
@@ -3238,13 +3239,26 @@ extern "C" int mpdok_lu_ir_solve_multi(const double* A, long long lda, long long
   MPDOK_ARG_CHECK(lda >= n && ldb >= n && ldx >= n, "leading dimensions must be >= n");
   MPDOK_ARG_CHECK(work_bytes >= mpdok_lu_ir_multi_work_size(n, nrhs), "multi-RHS LU-IR work buffer too small");
   MPDOK_TRY(check_factored(factors, n, fdtype, s));
-  return lu_ir_groups(A, lda, n, factors, fdtype, nrhs, 1, B, ldb, X, ldx, tol, maxiter_outer, work, info, s);
+  return lu_ir_groups(A, lda, n, factors, fdtype, nrhs, 1, B, ldb, X, ldx, tol, maxiter_outer, work, work_bytes, info,
+                      s);
 }
 
+// The next pass over `left` right-hand sides: ng groups of K columns.
+static void next_pass(int left, int* K, int* ng) {
+  *K = std::min(8, left);
+  *ng = *K == 8 ? std::min(MAX_GROUPS, left / 8) : 1;
+}
+
+// (every pass counts: one of fewer columns may need more, since its residual
+// splits K further)
 extern "C" size_t mpdok_lu_ir_many_work_size(long long n, int nrhs) {
   if (n < 0 || nrhs < 1) return 0;
-  const int ng = std::min(MAX_GROUPS, std::max(1, nrhs / 8));
-  return std::max(multi_layout(n, 8 * ng).total, multi_layout(n, std::min(nrhs, 8)).total) + 256;
+  size_t most = 0;
+  for (int c = 0, K = 0, ng = 0; c < nrhs; c += K * ng) {
+    next_pass(nrhs - c, &K, &ng);
+    most = std::max(most, multi_layout(n, K * ng).total);
+  }
+  return most + 256;
 }
 
 extern "C" int mpdok_lu_ir_solve_many(const double* A, long long lda, long long n, const void* factors, int fdtype,
@@ -3262,12 +3276,10 @@ extern "C" int mpdok_lu_ir_solve_many(const double* A, long long lda, long long 
   MPDOK_ARG_CHECK(lda >= n && ldb >= n && ldx >= n, "leading dimensions must be >= n");
   MPDOK_ARG_CHECK(work_bytes >= mpdok_lu_ir_many_work_size(n, nrhs), "multi-RHS LU-IR work buffer too small");
   MPDOK_TRY(check_factored(factors, n, fdtype, s));
-  for (int c = 0; c < nrhs;) {
-    const int K = std::min(8, nrhs - c);
-    const int ng = K == 8 ? std::min(MAX_GROUPS, (nrhs - c) / 8) : 1;
+  for (int c = 0, K = 0, ng = 0; c < nrhs; c += K * ng) {
+    next_pass(nrhs - c, &K, &ng);
     MPDOK_TRY(lu_ir_groups(A, lda, n, factors, fdtype, K, ng, B + (long long)c * ldb, ldb, X + (long long)c * ldx, ldx,
-                           tol, maxiter_outer, work, infos ? infos + c / 8 : nullptr, s));
-    c += K * ng;
+                           tol, maxiter_outer, work, work_bytes, infos ? infos + c / 8 : nullptr, s));
   }
   return MPDOK_OK;
 }
