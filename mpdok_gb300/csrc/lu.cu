@@ -3024,7 +3024,7 @@ static MultiWork multi_layout(long long n, int K) {
   m.off_tk = take(4 * sizeof(int));
   m.off_err = take(16);
   m.off_r = take(nv * sizeof(double));
-  m.off_nrm = take((size_t)K * sizeof(double));
+  m.off_nrm = take((size_t)K * (sizeof(double) + sizeof(int)));  // norms, then the residual's lossy flags
   m.off_g = take(gemv_workspace_bytes(MPDOK_F64, n, n, std::min(K, 8), false));
   m.off_q = take(residual64_work_bytes(n, K));
   m.total = off;
@@ -3158,20 +3158,42 @@ static int lu_ir_groups(const double* A, long long lda, long long n, const void*
     };
     MPDOK_TRY(correct(B, ldb, 1));
     // many columns of a large matrix: one residual of all of them on the tensor
-    // cores (the FP64 pipe takes 0.9 ms per eight columns at n = 8192)
-    const bool tc = residual64_pays(n, nc);
+    // cores (the FP64 pipe takes 0.9 ms per eight columns at n = 8192).  A group
+    // with a column that the digits would lose more of than an FP64 product does
+    // (residual64.cu) takes that product, from its first such step on.
     void* rw = wb + mw.off_q;
-    if (tc) MPDOK_TRY(residual64_prepare(A, lda, n, nc, rw, s));
-    for (int it = 0; it <= maxiter_outer; ++it) {
-      if (tc) MPDOK_TRY(residual64(A, lda, n, X, ldx, nc, B, ldb, R, n, rw, merr, s));
-      for (int a = 0; !tc && a < act.n; ++a) {
-        const long long c = (long long)act.id[a] * K;
-        MPDOK_TRY(gemv_launch(MPDOK_F64, false, A, lda, n, n, X + c * ldx, ldx, K, R + c * n, n, -1.0, 1.0, B + c * ldb,
-                              ldb, nullptr, gw, gbytes, s, true, nullptr));
-      }
+    std::vector<char> digits(ng, residual64_pays(n, nc));
+    if (digits[0]) MPDOK_TRY(residual64_prepare(A, lda, n, nc, rw, s));
+    auto fp64_residual = [&](int q) -> int {
+      const long long c = (long long)q * K;
+      return gemv_launch(MPDOK_F64, false, A, lda, n, n, X + c * ldx, ldx, K, R + c * n, n, -1.0, 1.0, B + c * ldb, ldb,
+                         nullptr, gw, gbytes, s, true, nullptr);
+    };
+    std::vector<char> report((size_t)nc * (sizeof(double) + sizeof(int)));
+    const int* lossy = (const int*)(report.data() + sizeof(double) * nc);
+    auto read_norms = [&]() -> int {
       MPDOK_TRY(colnorms_f64(R, n, nc, n, nrm, s));
-      MPDOK_CUDA_TRY(cudaMemcpyAsync(rn.data(), nrm, sizeof(double) * nc, cudaMemcpyDeviceToHost, s));
+      MPDOK_CUDA_TRY(cudaMemcpyAsync(report.data(), nrm, report.size(), cudaMemcpyDeviceToHost, s));
       MPDOK_CUDA_TRY(cudaStreamSynchronize(s));
+      std::memcpy(rn.data(), report.data(), sizeof(double) * nc);
+      return MPDOK_OK;
+    };
+    for (int it = 0; it <= maxiter_outer; ++it) {
+      bool tc = false;
+      for (int a = 0; a < act.n; ++a) tc |= digits[act.id[a]] != 0;
+      if (tc) MPDOK_TRY(residual64(A, lda, n, X, ldx, nc, B, ldb, R, n, rw, (int*)(nrm + nc), merr, s));
+      for (int a = 0; a < act.n; ++a)
+        if (!digits[act.id[a]]) MPDOK_TRY(fp64_residual(act.id[a]));
+      MPDOK_TRY(read_norms());
+      bool again = false;
+      for (int a = 0; a < act.n; ++a) {
+        const int q = act.id[a];
+        if (!digits[q] || std::none_of(lossy + q * K, lossy + (q + 1) * K, [](int f) { return f != 0; })) continue;
+        digits[q] = 0;
+        again = true;
+        MPDOK_TRY(fp64_residual(q));
+      }
+      if (again) MPDOK_TRY(read_norms());
       ColGroups next;
       next.n = 0;
       for (int a = 0; a < act.n; ++a) {

@@ -1,4 +1,5 @@
-// FP64 residuals R = B - A X of several columns on the tensor cores, exactly.
+// FP64 residuals R = B - A X of several columns on the tensor cores, from exact
+// products of the leading digits.
 //
 // GB300 multiplies FP64 at two lanes per clock and SM, so a product with eight
 // columns is bound by that pipe (n = 8192: 0.89 ms; reading A takes 0.08 ms).
@@ -9,11 +10,29 @@
 // digits have at most 14 bits, and the sums of up to eight digit pairs over a K
 // of 128 stay below 2^24: the FP32 accumulators of the tensor cores hold them
 // exactly.  Digit pairs (s, t) of equal weight s + t share an accumulator;
-// weights 7 .. 14 are formed (36 of the 64 pairs), which drops what is below
-// 2^-56 of (largest of the row) x (largest of the column) per sum of random
-// signs.  The accumulators are drained as integers, so the order of the sums
-// does not matter: a column's result depends neither on the other columns nor
-// on the split of K.  The final subtraction from B carries its rounding error.
+// weights 7 .. 14 are formed (36 of the 64 pairs).  The accumulators are drained
+// as integers, so the order of the sums does not matter: a column's result
+// depends neither on the other columns nor on the split of K.  The final
+// subtraction from B carries its rounding error.
+//
+// What is dropped is relative to the largest entry of the row of A and of the
+// column of X (2^E_i and 2^F: the powers of two at or below them), not to the terms
+// of the sum: up to seven pairs of weight 6 for each a_ij, as many as it has digits
+// (p_ij; none below 2^-61 of the largest), digits of random signs, rms 74 each,
+//   dropped_i = 2^-60.2 sqrt(sum_j p_ij / 7) 2^(E_i + F).
+// An FP64 product errs by some
+//   rounded_i = 0.27 u g^(1/4) sqrt(sum_j a_ij^2 x_j^2),  u = 2^-53,
+// with g the mean of sum_j p_ij / 7, the terms of a row that count (measured: 0.5 u
+// with 13 of them, 0.9 u with 100, 1.9 u with 1400, 3.2 u with 8192).  The first
+// exceeds the second where the columns of A differ in scale, or where one x_j towers
+// over the others.  So every call compares their norms over the rows (once as they
+// are and once relative to 2^E_i, so that small rows count too) and reports the
+// columns that the FP64 product does better: those with
+//   sum_j x_j^2 S_j < 2^-10.62 sqrt(g) m 2^(2 F),  m = sum_i w_i^2 2^(2 E_i),
+//   S_j = sum_i w_i^2 a_ij^2,  g m = sum_j P_j,  P_j = sum_i w_i^2 2^(2 E_i) p_ij / 7,
+// for w_i = 1 or w_i = 2^-E_i.  Measured (n = 2304 and 8192; kernels, random,
+// positive, integer and Toeplitz matrices, graded ones): where the digits stay
+// their error is 0.005 to 0.7 of the FP64 product's.
 #include "common.cuh"
 #include "residual64.cuh"
 
@@ -113,8 +132,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, float (&v)[16]) {
 }
 
 // The value as an integer below 2^62 in magnitude in units of 2^(E - 1084), E the
-// biased exponent of the row's or column's largest entry, plus the bias that
-// turns the signed base-256 digits into bytes: digit k = byte k - 128.
+// biased exponent of the row's or column's largest entry, plus a bias that turns
+// the signed base-256 digits into bytes: digit k = byte k - 128 (UP 0, digits -128
+// .. 127) or byte k - 127 (UP 1, -127 .. 128).  The two alternate along K: an
+// entry's lowest digit is often a multiple of 128 or 64, and digits of one form
+// would have a mean of -64 or -32 there, which the dropped pairs then sum over
+// all of K (a matrix of positive entries, n = 8192: up to 1.7 times an FP64
+// product's error; with both forms 0.3).
+// An entry above 2^-41 of the largest that does not fit becomes odd (von
+// Neumann's rounding, off by zero on average); smaller ones are cut off.
+template <int UP>
 __device__ __forceinline__ unsigned long long biased_digits(double a, int E) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(a);
   const int e = (int)(b >> 52) & 0x7ff;
@@ -122,17 +149,32 @@ __device__ __forceinline__ unsigned long long biased_digits(double a, int E) {
   if (e) m |= 0x10000000000000ull;
   const int sh = E - max(e, 1);
   m = (m << 9) >> min(sh, 63);
-  constexpr unsigned long long BIAS = 0x8080808080808080ull;
+  if (__funnelshift_lc(0u, (uint32_t)b, (uint32_t)(41 - sh)) != 0u) m |= 1ull;  // the sh - 9 low bits, lost
+  constexpr unsigned long long BIAS = UP ? 0x7f7f7f7f7f7f7f7full : 0x8080808080808080ull;
   return (long long)b < 0 ? BIAS - m : BIAS + m;
 }
+// The form of column j of A and row j of X: the parity of the low three bits of j
+// (no step of two or four through K meets one form only).
+constexpr int digit_form(int j) { return (j ^ j >> 1 ^ j >> 2) & 1; }
 
-// Byte k of two biased values as two FP16 digits: 0x6400 | byte is 1024 + byte.
+// Byte k of two biased values of forms UP and 1 - UP as two FP16 digits: 0x6400 |
+// byte is 1024 + byte.
+template <int UP>
 __device__ __forceinline__ uint32_t digit_pair(unsigned long long a, unsigned long long b, int k) {
   const uint32_t x = k < 4 ? (uint32_t)a : (uint32_t)(a >> 32), y = k < 4 ? (uint32_t)b : (uint32_t)(b >> 32);
   const int q = k & 3;
   const uint32_t h = (__byte_perm(x, y, (uint32_t)(q | ((4 + q) << 8))) & 0x00ff00ffu) | 0x64006400u;
-  const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&h), __half2half2(__ushort_as_half(0x6480)));
+  constexpr uint32_t off = UP ? 0x6480647fu : 0x647f6480u;
+  const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&h), *reinterpret_cast<const __half2*>(&off));
   return *reinterpret_cast<const uint32_t*>(&d);
+}
+
+// |a| relative to 2^(E - 1023), E at least its exponent, below 2; to 24 bits, and
+// 0 below 2^-60.
+__device__ __forceinline__ float relative_to(double a, int E) {
+  const uint32_t hi = (uint32_t)__double2hiint(a), lo = (uint32_t)__double2loint(a);
+  const int e = (int)(hi >> 20) & 0x7ff, d = e - E;
+  return e == 0 || d < -60 ? 0.f : __uint_as_float((uint32_t)(d + 127) << 23 | (hi & 0xfffffu) << 3 | lo >> 29);
 }
 
 // E[i] = the largest biased exponent of row i (at least 1), over a column chunk.
@@ -147,12 +189,63 @@ k_row_exponent(const double* __restrict__ A, long long lda, long long n, long lo
   atomicMax(E + i, m);
 }
 
+// rel[i] = 2^(E_i - max E) (0 below 2^-60), *sum = the sum of its squares; one block.
+__global__ void __launch_bounds__(1024) k_row_weights(const int* __restrict__ E, long long n, float* __restrict__ rel,
+                                                      float* __restrict__ sum) {
+  __shared__ int mx[32];
+  __shared__ float red[32];
+  int m = 1;
+  for (long long i = threadIdx.x; i < n; i += blockDim.x) m = max(m, E[i]);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) mx[threadIdx.x >> 5] = m;
+  __syncthreads();
+  m = __reduce_max_sync(0xffffffffu, mx[threadIdx.x & 31]);
+  float s = 0.f;
+  for (long long i = threadIdx.x; i < n; i += blockDim.x) {
+    const int d = E[i] - m;
+    const float r = d < -60 ? 0.f : __uint_as_float((uint32_t)(d + 127) << 23);
+    rel[i] = r;
+    s = fmaf(r, r, s);
+  }
+  s = block_sum(s, red);
+  if (threadIdx.x == 0) *sum = s;
+}
+
+// W[j] = (S_j, P_j) of the rule above with w_i = 2^-E_i, then with w_i = 1 (in units
+// of the matrix's largest exponent).  A warp to a column: one more read of A
+// (n = 8192: 0.1 ms a solve).
+__global__ void __launch_bounds__(256)
+k_column_weights(const double* __restrict__ A, long long lda, long long n, const int* __restrict__ E,
+                 const float* __restrict__ rel, float4* __restrict__ W) {
+  const long long j = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (j >= n) return;
+  const double* a = A + j * lda;
+  float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+  for (long long i = threadIdx.x & 31; i < n; i += 32) {
+    const double x = __ldg(a + i);
+    const int Ei = __ldg(E + i), d = Ei - (int)((uint32_t)__double2hiint(x) >> 20 & 0x7ff);
+    const float v = relative_to(x, Ei), r = __ldg(rel + i), w = v * r;
+    const float p = d > 61 ? 0.f : (float)min(7, ((61 - d) >> 3) + 1) * (1.f / 7.f);
+    t.x = fmaf(v, v, t.x);
+    t.y += p;
+    t.z = fmaf(w, w, t.z);
+    t.w = fmaf(p * r, r, t.w);
+  }
+  t = make_float4(warp_sum(t.x), warp_sum(t.y), warp_sum(t.z), warp_sum(t.w));
+  if ((threadIdx.x & 31) == 0) W[j] = t;
+}
+
 // Digits of the columns of X, one block per (padded) column: D[digit][column][k],
-// k < kpad, zero past row n and for the padding columns; F[column] = exponent.
+// k < kpad, zero past row n and for the padding columns; F[column] = exponent;
+// lossy[column] = 1 where what the digits drop exceeds the rounding of an FP64
+// product (a column of zeros drops nothing).
 __global__ void __launch_bounds__(256)
 k_column_digits(const double* __restrict__ X, long long ldx, long long n, int nc, long long kpad, int ncpad,
-                int* __restrict__ F, uint32_t* __restrict__ D) {
+                int* __restrict__ F, uint32_t* __restrict__ D, const float4* __restrict__ W,
+                const float* __restrict__ sum_rel, int* __restrict__ lossy) {
   __shared__ int red[8];
+  __shared__ float fred[32];
   const int c = blockIdx.x;
   const double* x = X + (long long)c * ldx;
   int m = 1;
@@ -167,10 +260,39 @@ k_column_digits(const double* __restrict__ X, long long ldx, long long n, int nc
   if (threadIdx.x == 0 && c < nc) F[c] = m;
   for (long long i = threadIdx.x; i < kpad / 2; i += blockDim.x) {
     const double a = c < nc && 2 * i < n ? x[2 * i] : 0.0, b = c < nc && 2 * i + 1 < n ? x[2 * i + 1] : 0.0;
-    const unsigned long long u = biased_digits(a, m), v = biased_digits(b, m);
+    uint32_t* out = D + (long long)c * (kpad / 2) + i;
+    const long long step = (long long)ncpad * (kpad / 2);
+    static_assert(digit_form(0) == 0 && digit_form(2) == 1 && digit_form(4) == 1 && digit_form(6) == 0, "pairs");
+    if ((i ^ i >> 1) & 1) {
+      const unsigned long long u = biased_digits<1>(a, m), v = biased_digits<0>(b, m);
 #pragma unroll
-    for (int k = 0; k < DIG; ++k) D[((long long)k * ncpad + c) * (kpad / 2) + i] = digit_pair(u, v, k);
+      for (int k = 0; k < DIG; ++k) out[k * step] = digit_pair<1>(u, v, k);
+    } else {
+      const unsigned long long u = biased_digits<0>(a, m), v = biased_digits<1>(b, m);
+#pragma unroll
+      for (int k = 0; k < DIG; ++k) out[k * step] = digit_pair<0>(u, v, k);
+    }
   }
+  if (c >= nc) return;
+  // the rule above
+  float q1 = 0.f, q2 = 0.f, p1 = 0.f, p2 = 0.f;
+  int any = 0;
+  for (long long i = threadIdx.x; i < n; i += blockDim.x) {
+    const float v = relative_to(x[i], m);
+    const float4 t = W[i];
+    q1 = fmaf(v * v, t.x, q1);
+    q2 = fmaf(v * v, t.z, q2);
+    p1 += t.y;
+    p2 += t.w;
+    any |= x[i] != 0.0;
+  }
+  any = __syncthreads_or(any);
+  q1 = block_sum(q1, fred);
+  q2 = block_sum(q2, fred);
+  p1 = block_sum(p1, fred);
+  p2 = block_sum(p2, fred);
+  constexpr float LIM = 6.354e-4f;  // 2^-10.62
+  if (threadIdx.x == 0) lossy[c] = any && !(q1 >= LIM * sqrtf(p1 * (float)n) && q2 >= LIM * sqrtf(p2 * *sum_rel));
 }
 
 // One CTA: rows [128 bx, ..), columns [32 by, ..), K chunks [bz per, ..).  Warp 0
@@ -352,14 +474,14 @@ k_residual64(const double* __restrict__ A, long long lda, int n, const int* __re
         for (int u = 0; u < 2; ++u) {
           unsigned long long d[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) d[e] = biased_digits(v[u][e], Ei);
+          for (int e = 0; e < 8; ++e) d[e] = digit_form(e) ? biased_digits<1>(v[u][e], Ei) : biased_digits<0>(v[u][e], Ei);
           uint32_t off = (uint32_t)(r * 64 + (kc + 2 * u) * 16);
           off ^= ((off >> 7) & 3u) << 4;
 #pragma unroll
           for (int k = 0; k < DIG; ++k)
             *reinterpret_cast<uint4*>(sa + k * A_PLANE + off) =
-                make_uint4(digit_pair(d[0], d[1], k), digit_pair(d[2], d[3], k), digit_pair(d[4], d[5], k),
-                           digit_pair(d[6], d[7], k));
+                make_uint4(digit_pair<0>(d[0], d[1], k), digit_pair<1>(d[2], d[3], k), digit_pair<1>(d[4], d[5], k),
+                           digit_pair<0>(d[6], d[7], k));
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
@@ -441,7 +563,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode() {
 struct Layout {
   long long kpad = 0;
   int ncpad = 0, nchunk = 0, per = 0, S = 1;
-  size_t off_E = 0, off_F = 0, off_D = 0, off_P = 0, total = 0;
+  size_t off_E = 0, off_rel = 0, off_sum = 0, off_W = 0, off_F = 0, off_D = 0, off_P = 0, total = 0;
 };
 
 static Layout layout(long long n, int nc) {
@@ -467,6 +589,9 @@ static Layout layout(long long n, int nc) {
   size_t off = 0;
   auto take = [&](size_t b) { size_t o = off; off = align_up(off + b, 256); return o; };
   l.off_E = take(sizeof(int) * (size_t)n);
+  l.off_rel = take(sizeof(float) * (size_t)n);
+  l.off_sum = take(sizeof(float));
+  l.off_W = take(sizeof(float4) * (size_t)n);
   l.off_F = take(sizeof(int) * (size_t)nc);
   l.off_D = take(sizeof(uint16_t) * (size_t)DIG * l.ncpad * l.kpad);
   l.off_P = take(sizeof(long long) * 2 * (size_t)l.S * nc * n);
@@ -482,17 +607,22 @@ size_t residual64_work_bytes(long long n, int nc) { return residual64_pays(n, nc
 
 int residual64_prepare(const double* A, long long lda, long long n, int nc, void* work, cudaStream_t s) {
   const r64::Layout l = r64::layout(n, nc);
-  int* E = (int*)((char*)work + l.off_E);
+  char* w = (char*)work;
+  int* E = (int*)(w + l.off_E);
+  float* rel = (float*)(w + l.off_rel);
   MPDOK_CUDA_TRY(cudaMemsetAsync(E, 0, sizeof(int) * n, s));
   const long long cchunk = std::max(256LL, (n + 65534) / 65535);
   dim3 grid((unsigned)((n + 255) / 256), (unsigned)((n + cchunk - 1) / cchunk));
   launch(r64::k_row_exponent, grid, 256, 0, s, A, lda, n, cchunk, E);
-  MPDOK_LAUNCH_CHECK("residual row exponents");
+  launch(r64::k_row_weights, 1, 1024, 0, s, (const int*)E, n, rel, (float*)(w + l.off_sum));
+  launch(r64::k_column_weights, (unsigned)((n + 7) / 8), 256, 0, s, A, lda, n, (const int*)E, (const float*)rel,
+         (float4*)(w + l.off_W));
+  MPDOK_LAUNCH_CHECK("residual weights");
   return MPDOK_OK;
 }
 
 int residual64(const double* A, long long lda, long long n, const double* X, long long ldx, int nc, const double* B,
-               long long ldb, double* R, long long ldr, void* work, int* err, cudaStream_t s) {
+               long long ldb, double* R, long long ldr, void* work, int* lossy, int* err, cudaStream_t s) {
   using namespace r64;
   const Layout l = layout(n, nc);
   char* w = (char*)work;
@@ -501,7 +631,8 @@ int residual64(const double* A, long long lda, long long n, const double* X, lon
   uint32_t* D = (uint32_t*)(w + l.off_D);
   long long* P = (long long*)(w + l.off_P);
   const int slot = prof_start(MPDOK_PROF_GEMV_F64, s);
-  launch(k_column_digits, (unsigned)l.ncpad, 256, 0, s, X, ldx, n, nc, l.kpad, l.ncpad, F, D);
+  launch(k_column_digits, (unsigned)l.ncpad, 256, 0, s, X, ldx, n, nc, l.kpad, l.ncpad, F, D,
+         (const float4*)(w + l.off_W), (const float*)(w + l.off_sum), lossy);
   auto enc = encode();
   if (!enc) {
     set_error("cuTensorMapEncodeTiled unavailable from the driver");

@@ -10,10 +10,12 @@ namespace mpdok {
 // SM weigh as much as the product.
 bool residual64_pays(long long n, int nc);
 size_t residual64_work_bytes(long long n, int nc);  // 0 where it does not pay
-// The row exponents of A (kept in the workspace until A changes).
+// The row exponents and column weights of A (kept in the workspace until A changes).
 int residual64_prepare(const double* A, long long lda, long long n, int nc, void* work, cudaStream_t s);
-// R = B - A X; *err = 5 when a bounded wait ran out.
+// R = B - A X; *err = 5 when a bounded wait ran out.  lossy[c] (device) is set to
+// 1 where the FP64 product of column c is the more accurate one, else to 0; the
+// rule reads A and the column only.
 int residual64(const double* A, long long lda, long long n, const double* X, long long ldx, int nc, const double* B,
-               long long ldb, double* R, long long ldr, void* work, int* err, cudaStream_t s);
+               long long ldb, double* R, long long ldr, void* work, int* lossy, int* err, cudaStream_t s);
 
 }  // namespace mpdok
