@@ -1172,12 +1172,6 @@ __global__ void k_scale_out(const float* __restrict__ z, const float* __restrict
 // wait for their predecessors.  Tickets go block by block over the groups, which
 // keeps a block's predecessors ahead of it.  Nine groups of 8 columns, n = 8192,
 // FP32 factors: 415 us per triangle, one group alone 333 us.
-constexpr int MAX_GROUPS = 16;
-struct ColGroups {
-  int n;
-  int id[MAX_GROUPS];
-};
-
 template <typename F, bool LOWER, int K>
 __global__ void __launch_bounds__(256)
 k_trsv_multi(const F* __restrict__ LU, long long ldf, const float* __restrict__ Dinv, const float* __restrict__ Mt,
@@ -3013,20 +3007,20 @@ struct MultiWork {
          off_g = 0, off_q = 0, total = 0;
 };
 
-static MultiWork multi_layout(long long n, int K) {
+static MultiWork multi_layout(long long n, int K, int ng) {
   MultiWork m;
   size_t off = 0;
   auto take = [&](size_t b) { size_t o = off; off = align_up(off + b, 256); return o; };
-  const size_t nv = (size_t)std::max(1LL, n) * K;
+  const size_t nc = (size_t)K * ng, nv = (size_t)std::max(1LL, n) * nc;
   m.off_y = take(nv * sizeof(float));
   m.off_z = take(nv * sizeof(float));
   m.off_v = take(nv * sizeof(float));
   m.off_tk = take(4 * sizeof(int));
   m.off_err = take(16);
   m.off_r = take(nv * sizeof(double));
-  m.off_nrm = take((size_t)K * (sizeof(double) + sizeof(int)));  // norms, then the residual's lossy flags
-  m.off_g = take(gemv_workspace_bytes(MPDOK_F64, n, n, std::min(K, 8), false));
-  m.off_q = take(residual64_work_bytes(n, K));
+  m.off_nrm = take(nc * (sizeof(double) + sizeof(int)));  // norms, then the residual's lossy flags
+  m.off_g = take(gemv_workspace_bytes(MPDOK_F64, n, n, K, false));
+  m.off_q = take(residual64_work_bytes(n, K, ng));
   m.total = off;
   return m;
 }
@@ -3116,7 +3110,7 @@ static int lu_ir_groups(const double* A, long long lda, long long n, const void*
                         const double* B, long long ldb, double* X, long long ldx, double tol, int maxiter_outer,
                         void* work, size_t work_bytes, mpdok_solve_info* infos, cudaStream_t s) {
   const int nc = K * ng;
-  const MultiWork mw = multi_layout(n, nc);
+  const MultiWork mw = multi_layout(n, K, ng);
   MPDOK_ARG_CHECK(work_bytes >= mw.total, "multi-RHS LU-IR work buffer too small");
   char* wb = (char*)work;
   float* y = (float*)(wb + mw.off_y);
@@ -3157,13 +3151,13 @@ static int lu_ir_groups(const double* A, long long lda, long long n, const void*
       return MPDOK_OK;
     };
     MPDOK_TRY(correct(B, ldb, 1));
-    // many columns of a large matrix: one residual of all of them on the tensor
-    // cores (the FP64 pipe takes 0.9 ms per eight columns at n = 8192).  A group
+    // many columns of a large matrix: one residual of all that still iterate on the
+    // tensor cores (the FP64 pipe takes 0.9 ms per eight columns at n = 8192).  A group
     // with a column that the digits would lose more of than an FP64 product does
     // (residual64.cu) takes that product, from its first such step on.
     void* rw = wb + mw.off_q;
-    std::vector<char> digits(ng, residual64_pays(n, nc));
-    if (digits[0]) MPDOK_TRY(residual64_prepare(A, lda, n, nc, rw, s));
+    std::vector<char> digits(ng, residual64_pays(n, K));
+    if (digits[0]) MPDOK_TRY(residual64_prepare(A, lda, n, rw, s));
     auto fp64_residual = [&](int q) -> int {
       const long long c = (long long)q * K;
       return gemv_launch(MPDOK_F64, false, A, lda, n, n, X + c * ldx, ldx, K, R + c * n, n, -1.0, 1.0, B + c * ldb, ldb,
@@ -3179,11 +3173,13 @@ static int lu_ir_groups(const double* A, long long lda, long long n, const void*
       return MPDOK_OK;
     };
     for (int it = 0; it <= maxiter_outer; ++it) {
-      bool tc = false;
-      for (int a = 0; a < act.n; ++a) tc |= digits[act.id[a]] != 0;
-      if (tc) MPDOK_TRY(residual64(A, lda, n, X, ldx, nc, B, ldb, R, n, rw, (int*)(nrm + nc), merr, s));
-      for (int a = 0; a < act.n; ++a)
-        if (!digits[act.id[a]]) MPDOK_TRY(fp64_residual(act.id[a]));
+      ColGroups dig;
+      dig.n = 0;
+      for (int a = 0; a < act.n; ++a) {
+        if (digits[act.id[a]]) dig.id[dig.n++] = act.id[a];
+        else MPDOK_TRY(fp64_residual(act.id[a]));
+      }
+      if (dig.n > 0) MPDOK_TRY(residual64(A, lda, n, X, ldx, K, dig, B, ldb, R, n, rw, (int*)(nrm + nc), merr, s));
       MPDOK_TRY(read_norms());
       bool again = false;
       for (int a = 0; a < act.n; ++a) {
@@ -3243,7 +3239,7 @@ static int check_factored(const void* factors, long long n, int fdtype, cudaStre
 
 extern "C" size_t mpdok_lu_ir_multi_work_size(long long n, int nrhs) {
   if (n < 0 || nrhs < 1 || nrhs > 8) return 0;
-  return multi_layout(n, nrhs).total + 256;
+  return multi_layout(n, nrhs, 1).total + 256;
 }
 
 // LU-IR on nrhs <= 8 right-hand sides together.  The per-solve form of the
@@ -3278,7 +3274,7 @@ extern "C" size_t mpdok_lu_ir_many_work_size(long long n, int nrhs) {
   size_t most = 0;
   for (int c = 0, K = 0, ng = 0; c < nrhs; c += K * ng) {
     next_pass(nrhs - c, &K, &ng);
-    most = std::max(most, multi_layout(n, K * ng).total);
+    most = std::max(most, multi_layout(n, K, ng).total);
   }
   return most + 256;
 }

@@ -236,18 +236,22 @@ k_column_weights(const double* __restrict__ A, long long lda, long long n, const
   if ((threadIdx.x & 31) == 0) W[j] = t;
 }
 
-// Digits of the columns of X, one block per (padded) column: D[digit][column][k],
+// Column of the caller's matrices that column c of the listed groups is.
+__device__ __forceinline__ long long group_column(const ColGroups& g, int K, int c) { return (long long)g.id[c / K] * K + c % K; }
+
+// Digits of the listed columns of X, one block per (padded) column: D[digit][column][k],
 // k < kpad, zero past row n and for the padding columns; F[column] = exponent;
 // lossy[column] = 1 where what the digits drop exceeds the rounding of an FP64
 // product (a column of zeros drops nothing).
 __global__ void __launch_bounds__(256)
 k_column_digits(const double* __restrict__ X, long long ldx, long long n, int nc, long long kpad, int ncpad,
                 int* __restrict__ F, uint32_t* __restrict__ D, const float4* __restrict__ W,
-                const float* __restrict__ sum_rel, int* __restrict__ lossy) {
+                const float* __restrict__ sum_rel, int* __restrict__ lossy, int K, const ColGroups groups) {
   __shared__ int red[8];
   __shared__ float fred[32];
   const int c = blockIdx.x;
-  const double* x = X + (long long)c * ldx;
+  const long long src = c < nc ? group_column(groups, K, c) : 0;
+  const double* x = X + src * ldx;
   int m = 1;
   if (c < nc)
     for (long long i = threadIdx.x; i < n; i += blockDim.x) m = max(m, (__double2hiint(x[i]) >> 20) & 0x7ff);
@@ -292,7 +296,7 @@ k_column_digits(const double* __restrict__ X, long long ldx, long long n, int nc
   p1 = block_sum(p1, fred);
   p2 = block_sum(p2, fred);
   constexpr float LIM = 6.354e-4f;  // 2^-10.62
-  if (threadIdx.x == 0) lossy[c] = any && !(q1 >= LIM * sqrtf(p1 * (float)n) && q2 >= LIM * sqrtf(p2 * *sum_rel));
+  if (threadIdx.x == 0) lossy[src] = any && !(q1 >= LIM * sqrtf(p1 * (float)n) && q2 >= LIM * sqrtf(p2 * *sum_rel));
 }
 
 // One CTA: rows [128 bx, ..), columns [32 by, ..), K chunks [bz per, ..).  Warp 0
@@ -518,10 +522,10 @@ k_residual64(const double* __restrict__ A, long long lda, int n, const int* __re
 __global__ void __launch_bounds__(256)
 k_residual64_finish(const long long* __restrict__ P, int S, long long n, int nc, const int* __restrict__ E,
                     const int* __restrict__ F, const double* __restrict__ B, long long ldb, double* __restrict__ R,
-                    long long ldr) {
+                    long long ldr, int K, const ColGroups groups) {
   const long long total = n * nc;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    const long long c = e / n, i = e % n;
+    const long long c = e / n, i = e % n, src = group_column(groups, K, (int)c);
     long long lo = 0, hi = 0;
     for (int s = 0; s < S; ++s) {
       lo += P[(long long)s * 2 * total + e];
@@ -536,14 +540,14 @@ k_residual64_finish(const long long* __restrict__ P, int S, long long n, int nc,
       constexpr long long MASK = (1ll << 27) - 1;
       const double t3 = -scalbn((double)(hi >> 27), w + 59), t2 = -scalbn((double)(hi & MASK), w + 32);
       const double t1 = -scalbn((double)(lo >> 27), w + 27), t0 = -scalbn((double)(lo & MASK), w);
-      const double b = B[i + c * ldb];
+      const double b = B[i + src * ldb];
       const double s = b + t3, bb = s - b;
       const double err = (b - (s - bb)) + (t3 - bb);
       const double s2 = s + t2, b2 = s2 - s;
       const double err2 = (s - (s2 - b2)) + (t2 - b2);
       r = s2 + ((t1 + t0) + (err + err2));
     }
-    R[i + c * ldr] = r;
+    R[i + src * ldr] = r;
   }
 }
 
@@ -603,10 +607,15 @@ static Layout layout(long long n, int nc) {
 
 bool residual64_pays(long long n, int nc) { return nc >= 4 && n >= 2048 && n <= (1LL << 30); }
 
-size_t residual64_work_bytes(long long n, int nc) { return residual64_pays(n, nc) ? r64::layout(n, nc).total : 0; }
+// (fewer groups may need more: their K is split further)
+size_t residual64_work_bytes(long long n, int K, int ng) {
+  size_t most = 0;
+  for (int g = 1; g <= ng && residual64_pays(n, K); ++g) most = std::max(most, r64::layout(n, K * g).total);
+  return most;
+}
 
-int residual64_prepare(const double* A, long long lda, long long n, int nc, void* work, cudaStream_t s) {
-  const r64::Layout l = r64::layout(n, nc);
+int residual64_prepare(const double* A, long long lda, long long n, void* work, cudaStream_t s) {
+  const r64::Layout l = r64::layout(n, 1);  // (what it fills lies before anything that depends on the columns)
   char* w = (char*)work;
   int* E = (int*)(w + l.off_E);
   float* rel = (float*)(w + l.off_rel);
@@ -621,9 +630,11 @@ int residual64_prepare(const double* A, long long lda, long long n, int nc, void
   return MPDOK_OK;
 }
 
-int residual64(const double* A, long long lda, long long n, const double* X, long long ldx, int nc, const double* B,
-               long long ldb, double* R, long long ldr, void* work, int* lossy, int* err, cudaStream_t s) {
+int residual64(const double* A, long long lda, long long n, const double* X, long long ldx, int K,
+               const ColGroups& groups, const double* B, long long ldb, double* R, long long ldr, void* work,
+               int* lossy, int* err, cudaStream_t s) {
   using namespace r64;
+  const int nc = K * groups.n;
   const Layout l = layout(n, nc);
   char* w = (char*)work;
   int* E = (int*)(w + l.off_E);
@@ -632,7 +643,7 @@ int residual64(const double* A, long long lda, long long n, const double* X, lon
   long long* P = (long long*)(w + l.off_P);
   const int slot = prof_start(MPDOK_PROF_GEMV_F64, s);
   launch(k_column_digits, (unsigned)l.ncpad, 256, 0, s, X, ldx, n, nc, l.kpad, l.ncpad, F, D,
-         (const float4*)(w + l.off_W), (const float*)(w + l.off_sum), lossy);
+         (const float4*)(w + l.off_W), (const float*)(w + l.off_sum), lossy, K, groups);
   auto enc = encode();
   if (!enc) {
     set_error("cuTensorMapEncodeTiled unavailable from the driver");
@@ -655,7 +666,8 @@ int residual64(const double* A, long long lda, long long n, const double* X, lon
   k_residual64<<<grid, THREADS, ALLOC, s>>>(A, lda, (int)n, E, tm, nc, l.nchunk, l.per, P, err);
   count_launch();
   const unsigned g = (unsigned)std::max(1LL, std::min<long long>((n * nc + 255) / 256, (long long)num_sms() * 8));
-  launch(k_residual64_finish, g, 256, 0, s, (const long long*)P, l.S, n, nc, (const int*)E, (const int*)F, B, ldb, R, ldr);
+  launch(k_residual64_finish, g, 256, 0, s, (const long long*)P, l.S, n, nc, (const int*)E, (const int*)F, B, ldb, R, ldr,
+         K, groups);
   prof_stop(slot, s, (double)n * (double)n * 8.0 + 16.0 * (double)nc * (double)n);
   MPDOK_LAUNCH_CHECK("residual64");
   return MPDOK_OK;

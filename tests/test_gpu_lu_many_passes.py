@@ -41,3 +41,30 @@ def test_groups_take_the_steps_they_would_take_alone(n, k):
         assert one.converged and infos[q].converged
         assert torch.equal(Y, X[:, c:c + kk])
         assert one.history_list() == infos[q].history_list()
+
+
+def test_finished_groups_leave_the_residual():
+    """Five groups, four of them zero and so done at once: the products after the
+    first cover the fifth only (8 bytes n^2 + 16 bytes n per column that they
+    multiply), and its steps are the ones it takes alone."""
+    from mpdok_gb300 import _native as N
+    from mpdok_gb300.lu import LUFactorization
+    from mpdok_gb300.rbf_kernel import build_rbf_kernel
+    n = 2304
+    rng = np.random.default_rng(3)
+    Ad, _ = build_rbf_kernel(torch.from_numpy(rng.uniform(0, 1, (n, 2))).cuda(), gamma=0.2 * n, reg=0.1)
+    B = torch.zeros((40, n), dtype=torch.float64, device="cuda").t()
+    B[:, 24:32] = torch.from_numpy(rng.standard_normal((n, 8))).cuda()
+    lu = LUFactorization(Ad, dtype="fp16")
+    Y, alone = lu.solve_ir_many(Ad, B[:, 24:32], tol=1e-12, maxiter_outer=10)
+    N.profile_enable(True)
+    try:
+        X, info = lu.solve_ir_many(Ad, B, tol=1e-12, maxiter_outer=10)
+        torch.cuda.synchronize()
+        _, launches, work = N.profile_query(N.PROF_GEMV_F64)
+    finally:
+        N.profile_enable(False)
+    assert info["converged"] and torch.equal(X[:, 24:32], Y) and info["history"][3] == alone["history"][0]
+    assert torch.all(X[:, :24] == 0) and torch.all(X[:, 32:] == 0)
+    assert launches == len(info["history"][3]) > 2
+    assert work == launches * 8.0 * n * n + 16.0 * n * (40 + 8 * (launches - 1))
