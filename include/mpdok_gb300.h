@@ -77,8 +77,8 @@ MPDOK_API void mpdok_clear_error(void);
 
 /* Test hooks for the failure paths; no counterpart in the reference.
  * MPDOK_DEBUG_WAIT_LIMIT: iteration limit of the triangular solves' bounded
- *   waits on a predecessor block, on the current device (value <= 0 restores
- *   the default).
+ *   waits on a predecessor block, of LU factors and of batches, on the current
+ *   device (value <= 0 restores the default).
  * MPDOK_DEBUG_TRSV_FIRST_TICKET: first ticket that the next triangular solves
  *   of this process hand out (0 = normal).  With a value above 0 no block ever
  *   solves block 0, so the blocks that depend on it wait until their limit
@@ -433,8 +433,12 @@ MPDOK_API int mpdok_batch_schedule(void* plan, int schedule, int ctas_per_sm);
 /* One step on B / X: assembly + factor + solve + `refine` refinement steps
  * under the plan's schedule (no host synchronisation). */
 MPDOK_API int mpdok_batch_step(void* plan, const double* B, double* X, int refine, cudaStream_t stream);
-/* MPDOK_ERR_TIMEOUT when a task of the last task-graph step, or a block of the
- * last solve, gave up waiting on its inputs (synchronises the stream), else 0. */
+/* MPDOK_ERR_TIMEOUT when a task of the last task-graph step, or a block of a
+ * solve, gave up waiting on its inputs (synchronises the stream), else 0.  The
+ * solves do not synchronise: one whose wait ran out leaves NaN in X, and the
+ * first later call on the plan that finds it (any but the graph build) returns
+ * MPDOK_ERR_TIMEOUT, once, without doing its work; mpdok_chol_cg_ir returns it
+ * for its own solves. */
 MPDOK_API int mpdok_batch_dag_status(void* plan, cudaStream_t stream);
 
 /* --------------------------------------------------------- instrumentation

@@ -262,7 +262,11 @@ class BatchedRBFSolver:
         return X
 
     def dag_status(self):
-        """Raise when a task of the last task-graph step gave up waiting on its inputs."""
+        """Raise when a task of the last task-graph step, or a block of a solve, gave up waiting on its inputs.
+
+        A solve returns before its blocks have run.  One whose wait ran out leaves
+        NaN in X, and the next call on this solver (the next load of a training
+        loop, say) raises; this method waits for the stream first."""
         N.check(N.load().mpdok_batch_dag_status(self._plan, stream_handle()), "batch_dag_status")
 
     def relres(self, B, X) -> torch.Tensor:
@@ -330,8 +334,7 @@ class BatchedRBFSolver:
             self.step(Bt, refine=2)
             e1.record()
             torch.cuda.synchronize()
-            if self.schedule == "dag":
-                self.dag_status()
+            self.dag_status()
             return e0.elapsed_time(e1) / 1e3
 
         best, times = choose(cands, measure, reps)

@@ -77,6 +77,7 @@ struct BatchPlan {
   double *A = nullptr, *Linv = nullptr, *V = nullptr, *R = nullptr, *rows = nullptr, *coords = nullptr;
   int* d_pert = nullptr;
   int* d_ticket = nullptr;            // the solves: forward and backward ticket, timed-out wait
+  int* timed_out = nullptr;           // pinned: a wait of some solve ran out (kept until it is reported)
   size_t bytes = 0;
   int syrk_grid = 0;
   cudaStream_t cap = nullptr;
@@ -545,6 +546,7 @@ __device__ __forceinline__ double diag_dot(const double* sLi, const double* sx, 
 // Results start as this bit pattern; consumers poll the values themselves.
 constexpr unsigned long long BSOLVE_EMPTY = 0xffffffffffffffffull;
 constexpr long long BSOLVE_WAIT = 1LL << 24;
+__device__ long long g_bsolve_wait = BSOLVE_WAIT;  // (a device variable so that a test can shorten it)
 constexpr int BSOLVE_RHS = 4;    // right-hand sides of one CTA
 constexpr size_t BSOLVE_SMEM = (size_t)BNB * BPAD * (sizeof(double) + sizeof(DF)) +
                                (size_t)BNB * BSOLVE_RHS * (sizeof(double) + sizeof(DF));
@@ -573,7 +575,7 @@ template <bool TRANS>
 __global__ void __launch_bounds__(BT) k_bsolve_chain(const BSys* __restrict__ sys, const long long* __restrict__ lvl,
                                                      int maxblk, int nrhs, const double* __restrict__ A,
                                                      const double* __restrict__ Linv, const double* __restrict__ IN,
-                                                     double* OUT, int* ticket, int* err) {
+                                                     double* OUT, int* ticket, int* err, int* timed_out) {
   extern __shared__ double smem[];
   double* sLi = smem;                                            // [i][c]
   double* sx = sLi + BNB * BPAD;                                 // [rhs][64]
@@ -628,7 +630,8 @@ __global__ void __launch_bounds__(BT) k_bsolve_chain(const BSys* __restrict__ sy
     double v = 0.0;
     if (row < nb && r8 + rr < nrhs) {
       unsigned long long b = BSOLVE_EMPTY;
-      for (long long it = 0; it < BSOLVE_WAIT; ++it) {
+      const long long limit = g_bsolve_wait;
+      for (long long it = 0; it < limit; ++it) {
         b = ld_relaxed_u64(OUT + col + kb + row);
         if (b != BSOLVE_EMPTY) break;
         if (it > 64) {
@@ -639,6 +642,7 @@ __global__ void __launch_bounds__(BT) k_bsolve_chain(const BSys* __restrict__ sy
       if (b == BSOLVE_EMPTY) {
         s_abort = 1;
         atomicExch(err, 1);
+        *(volatile int*)timed_out = 1;
       }
       v = __longlong_as_double((long long)b);
     }
@@ -1445,6 +1449,22 @@ static int batch_factor(BatchPlan* p, cudaStream_t s) {
   return MPDOK_OK;
 }
 
+int batch_debug_wait(long long limit) {
+  const long long v = limit > 0 ? limit : BSOLVE_WAIT;
+  MPDOK_CUDA_TRY(cudaMemcpyToSymbol(g_bsolve_wait, &v, sizeof(v)));
+  return MPDOK_OK;
+}
+
+// A solve does not synchronise, so a wait that ran out in one is reported by the
+// first later call on the plan that finds it (its blocks left X all NaN).
+int batch_timed_out(void* plan) {
+  BatchPlan* p = (BatchPlan*)plan;
+  if (*(volatile int*)p->timed_out == 0) return MPDOK_OK;
+  *(volatile int*)p->timed_out = 0;
+  set_error("batch triangular solve: a block's wait on its predecessor ran out in an earlier solve");
+  return MPDOK_ERR_TIMEOUT;
+}
+
 // V := A^{-1} V in place (V in the caller's packing), through the plan's R.
 static int batch_solve_inplace(BatchPlan* p, double* V, cudaStream_t s) {
   const size_t bytes = (size_t)p->total_x * sizeof(double);
@@ -1453,14 +1473,20 @@ static int batch_solve_inplace(BatchPlan* p, double* V, cudaStream_t s) {
   if (grid == 0) return MPDOK_OK;
   MPDOK_TRY(set_smem(k_bsolve_chain<false>, BSOLVE_SMEM));
   MPDOK_TRY(set_smem(k_bsolve_chain<true>, BSOLVE_SMEM));
-  MPDOK_CUDA_TRY(cudaMemsetAsync(p->d_ticket, 0, 2 * sizeof(int), s));
+  // (the error word too: a wait that ran out ends this solve's waits, not the next one's)
+  MPDOK_CUDA_TRY(cudaMemsetAsync(p->d_ticket, 0, 3 * sizeof(int), s));
+  if (const int t0 = debug_first_ticket()) {
+    MPDOK_CUDA_TRY(cudaMemcpyAsync(p->d_ticket, &t0, sizeof(int), cudaMemcpyHostToDevice, s));
+    MPDOK_CUDA_TRY(cudaStreamSynchronize(s));
+  }
   MPDOK_CUDA_TRY(cudaMemsetAsync(p->R, 0xff, bytes, s));
   launch(k_bsolve_chain<false>, dim3(grid), BT, BSOLVE_SMEM, s, (const BSys*)p->d_sys, preLvl_dev(p), p->maxblk,
-         p->nrhs, (const double*)p->A, (const double*)p->Linv, (const double*)V, p->R, p->d_ticket, p->d_ticket + 2);
+         p->nrhs, (const double*)p->A, (const double*)p->Linv, (const double*)V, p->R, p->d_ticket, p->d_ticket + 2,
+         p->timed_out);
   MPDOK_CUDA_TRY(cudaMemsetAsync(V, 0xff, bytes, s));
   launch(k_bsolve_chain<true>, dim3(grid), BT, BSOLVE_SMEM, s, (const BSys*)p->d_sys, preLvl_dev(p), p->maxblk,
          p->nrhs, (const double*)p->A, (const double*)p->Linv, (const double*)p->R, V, p->d_ticket + 1,
-         p->d_ticket + 2);
+         p->d_ticket + 2, p->timed_out);
   MPDOK_LAUNCH_CHECK("batch solve");
   return MPDOK_OK;
 }
@@ -1477,7 +1503,6 @@ static int batch_residual(BatchPlan* p, const double* B, const double* X, double
 static int batch_solve(BatchPlan* p, const double* B, double* X, int refine, cudaStream_t s) {
   const long long nx = p->total_x;
   if (nx == 0) return MPDOK_OK;
-  MPDOK_CUDA_TRY(cudaMemsetAsync(p->d_ticket + 2, 0, sizeof(int), s));
   MPDOK_CUDA_TRY(cudaMemcpyAsync(X, B, (size_t)nx * sizeof(double), cudaMemcpyDeviceToDevice, s));
   MPDOK_TRY(batch_solve_inplace(p, X, s));
   const unsigned g = (unsigned)std::min<long long>((nx + 255) / 256, (long long)num_sms() * 8);
@@ -1690,6 +1715,7 @@ static void plan_free(BatchPlan* p) {
   if (p->d_pre) cudaFree(p->d_pre);
   if (p->d_pert) cudaFree(p->d_pert);
   if (p->d_ticket) cudaFree(p->d_ticket);
+  if (p->timed_out) cudaFreeHost(p->timed_out);
   delete p;
 }
 
@@ -1797,6 +1823,9 @@ extern "C" int mpdok_batch_create(int nsys, const long long* n, int dim, int nrh
   if (e != cudaSuccess) return fail(e, "cudaMalloc (batch tickets)");
   e = cudaMemset(p->d_ticket, 0, 4 * sizeof(int));
   if (e != cudaSuccess) return fail(e, "cudaMemset (batch tickets)");
+  e = cudaHostAlloc((void**)&p->timed_out, sizeof(int), cudaHostAllocPortable);
+  if (e != cudaSuccess) return fail(e, "cudaHostAlloc (batch status)");
+  *p->timed_out = 0;
   const size_t nA = align_up((size_t)aA, 32), nL = align_up((size_t)aL, 32), nV = align_up((size_t)ax, 32),
                nR = align_up((size_t)aR, 32), nCo = align_up((size_t)ac, 32);
   p->bytes = (nA + nL + 2 * nV + nR + nCo) * sizeof(double);
@@ -1837,6 +1866,7 @@ extern "C" size_t mpdok_batch_bytes(void* plan) { return plan ? ((BatchPlan*)pla
 extern "C" int mpdok_batch_load(void* plan, const double* coords, const double* eps, const double* reg,
                                 cudaStream_t s) {
   MPDOK_ARG_CHECK(plan && coords && eps && reg, "null pointer");
+  MPDOK_TRY(batch_timed_out(plan));
   BatchPlan* p = (BatchPlan*)plan;
   for (auto& q : p->sys) {
     MPDOK_ARG_CHECK(std::isfinite(eps[q.user]) && std::isfinite(reg[q.user]) && reg[q.user] >= 0.0,
@@ -1856,6 +1886,7 @@ extern "C" int mpdok_batch_load(void* plan, const double* coords, const double* 
 
 extern "C" int mpdok_batch_factor(void* plan, cudaStream_t s) {
   MPDOK_ARG_CHECK(plan, "null plan");
+  MPDOK_TRY(batch_timed_out(plan));
   return batch_factor((BatchPlan*)plan, s);
 }
 
@@ -1863,11 +1894,13 @@ extern "C" int mpdok_batch_solve(void* plan, const double* B, double* X, int ref
   MPDOK_ARG_CHECK(plan && B && X, "null pointer");
   MPDOK_ARG_CHECK(refine >= 0 && refine <= 16, "refine must be in [0, 16]");
   MPDOK_ARG_CHECK(B != X, "B and X must not alias");
+  MPDOK_TRY(batch_timed_out(plan));
   return batch_solve((BatchPlan*)plan, B, X, refine, s);
 }
 
 extern "C" int mpdok_batch_relres(void* plan, const double* B, const double* X, double* relres, cudaStream_t s) {
   MPDOK_ARG_CHECK(plan && B && X && relres, "null pointer");
+  MPDOK_TRY(batch_timed_out(plan));
   BatchPlan* p = (BatchPlan*)plan;
   MPDOK_TRY(batch_residual(p, B, X, p->R, s));
   launch(k_brelres, dim3(p->nsys), BT, 0, s, (const BSys*)p->d_sys, p->nrhs, B, (const double*)p->R, relres);
@@ -1878,6 +1911,7 @@ extern "C" int mpdok_batch_relres(void* plan, const double* B, const double* X, 
 extern "C" int mpdok_batch_adjoint(void* plan, const double* X, const double* Lam, double* grad_coords,
                                    double* grad_eps, double* grad_reg, cudaStream_t s) {
   MPDOK_ARG_CHECK(plan && X && Lam && grad_coords && grad_eps && grad_reg, "null pointer");
+  MPDOK_TRY(batch_timed_out(plan));
   BatchPlan* p = (BatchPlan*)plan;
   const long long nt = p->preRow.back();
   if (nt > 0) {
@@ -1936,6 +1970,7 @@ extern "C" int mpdok_batch_perturbed(void* plan, cudaStream_t s) {
   int h = 0;
   MPDOK_CUDA_TRY(cudaMemcpyAsync(&h, p->d_pert, sizeof(int), cudaMemcpyDeviceToHost, s));
   MPDOK_CUDA_TRY(cudaStreamSynchronize(s));
+  MPDOK_TRY(batch_timed_out(plan));
   return h;
 }
 
@@ -1983,6 +2018,7 @@ extern "C" int mpdok_batch_graph_launch(void* plan, cudaStream_t s) {
     set_error("no graph: call mpdok_batch_graph_build first");
     return MPDOK_ERR_NOT_FACTORED;
   }
+  MPDOK_TRY(batch_timed_out(plan));
   MPDOK_CUDA_TRY(cudaGraphLaunch(p->exec, s));
   count_launch();
   return MPDOK_OK;
@@ -2002,6 +2038,7 @@ extern "C" int mpdok_batch_step(void* plan, const double* B, double* X, int refi
   MPDOK_ARG_CHECK(plan && B && X, "null pointer");
   MPDOK_ARG_CHECK(refine >= 0 && refine <= 16, "refine must be in [0, 16]");
   BatchPlan* p = (BatchPlan*)plan;
+  MPDOK_TRY(batch_timed_out(plan));
   if (p->schedule == 1) return batch_step_dag(p, B, X, refine, s);
   MPDOK_TRY(batch_factor(p, s));
   return batch_solve(p, B, X, refine, s);
@@ -2010,14 +2047,10 @@ extern "C" int mpdok_batch_step(void* plan, const double* B, double* X, int refi
 extern "C" int mpdok_batch_dag_status(void* plan, cudaStream_t s) {
   MPDOK_ARG_CHECK(plan, "null plan");
   BatchPlan* p = (BatchPlan*)plan;
-  int h = 0;
-  MPDOK_CUDA_TRY(cudaMemcpyAsync(&h, p->d_ticket + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
   MPDOK_CUDA_TRY(cudaStreamSynchronize(s));
-  if (h) {
-    set_error("batch triangular solve: a block's wait on its predecessor ran out");
-    return MPDOK_ERR_TIMEOUT;
-  }
+  MPDOK_TRY(batch_timed_out(plan));
   if (!p->d_dagstate) return MPDOK_OK;
+  int h = 0;
   const int* err = p->d_dagstate + p->dag_head_idx + 2;
   MPDOK_CUDA_TRY(cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, s));
   MPDOK_CUDA_TRY(cudaStreamSynchronize(s));

@@ -250,7 +250,7 @@ static int set_coef(const CholPcgWs& w, const double* host, int K, cudaStream_t 
   return MPDOK_OK;
 }
 
-static int chol_pcg_ir_core(void* plan, const Residual64& R, const Residual64& Ain, long long n, int K,
+static int chol_pcg_ir_body(void* plan, const Residual64& R, const Residual64& Ain, long long n, int K,
                             const double* B, long long ldb,
                             double* Xout, long long ldx, double tol, int maxiter_outer, double inner_tol,
                             int inner_maxiter, const CholPcgWs& w, mpdok_solve_info* info, cudaStream_t s) {
@@ -332,6 +332,17 @@ static int chol_pcg_ir_core(void* plan, const Residual64& R, const Residual64& A
   return MPDOK_OK;
 }
 
+// (a wait that ran out shows as NaN in the body)
+static int chol_pcg_ir_core(void* plan, const Residual64& R, const Residual64& Ain, long long n, int K,
+                            const double* B, long long ldb, double* Xout, long long ldx, double tol, int maxiter_outer,
+                            double inner_tol, int inner_maxiter, const CholPcgWs& w, mpdok_solve_info* info,
+                            cudaStream_t s) {
+  const int st = chol_pcg_ir_body(plan, R, Ain, n, K, B, ldb, Xout, ldx, tol, maxiter_outer, inner_tol, inner_maxiter, w,
+                                  info, s);
+  MPDOK_TRY(batch_timed_out(plan));
+  return st;
+}
+
 }  // namespace mpdok
 
 extern "C" size_t mpdok_chol_cg_ir_workspace_size(long long n, int nrhs, int mode) {
@@ -354,6 +365,7 @@ extern "C" int mpdok_chol_cg_ir(void* plan, const double* A64, long long lda, co
   MPDOK_ARG_CHECK(mode != 1 || opbuf != nullptr, "the split operator needs opbuf");
   MPDOK_ARG_CHECK(ldb >= n && ldx >= n && (mode == 2 || lda >= n), "leading dimension too small");
   MPDOK_ARG_CHECK(work_bytes >= mpdok_chol_cg_ir_workspace_size(n, nrhs, mode), "workspace too small");
+  MPDOK_TRY(batch_timed_out(plan));
   CholPcgWs w = chol_layout(n, nrhs, work);
   char* gw = (char*)work + align_up(w.total, 256);
   const size_t gbytes = work_bytes - align_up(w.total, 256);

@@ -112,6 +112,14 @@ int batch_precond(void* plan, long long n, int K, double* tmp, BatchPcCtx* ctx, 
 // (V: n x K column-major, ld n, K = the plan's nrhs).  Defined in batch.cu.
 int batch_apply_f64(void* plan, long long n, int K, double* V, cudaStream_t s);
 
+// MPDOK_ERR_TIMEOUT, once, when a wait of a finished solve of the plan ran out.
+int batch_timed_out(void* plan);
+
+// Test hooks (mpdok_debug_set): the batch solves' wait limit (<= 0: the default)
+// and the first ticket of every triangular solve (0: normal).
+int batch_debug_wait(long long limit);
+int debug_first_ticket();
+
 // One Arnoldi cycle (up to m steps) on the FP32 operator A32 with the
 // unnormalised start vector already in V[:,0] and ws.sc->nrm2 = ||V[:,0]||^2
 // set by cycle_setup.  reorth = 1 or 2 Gram-Schmidt passes.  Early stop when

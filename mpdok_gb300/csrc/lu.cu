@@ -2031,6 +2031,7 @@ __global__ void k_store_lower(const float* __restrict__ W, long long ldw, long l
 // First ticket of the next triangular solves; 0 except under a test hook
 // (mpdok_debug_set), which raises it so that no block ever solves block 0.
 static int g_first_ticket = 0;
+int debug_first_ticket() { return g_first_ticket; }
 
 // Outputs from `out` on start empty (TRSV_EMPTY in every word: the solves poll
 // them) and the two ticket counters, which follow them in the workspace, at -1:
@@ -2766,7 +2767,7 @@ extern "C" int mpdok_debug_set(int key, long long value) {
     case MPDOK_DEBUG_WAIT_LIMIT: {
       const long long v = value > 0 ? value : SPIN_LIMIT;
       MPDOK_CUDA_TRY(cudaMemcpyToSymbol(g_spin_limit, &v, sizeof(v)));
-      return MPDOK_OK;
+      return batch_debug_wait(value);
     }
     case MPDOK_DEBUG_TRSV_FIRST_TICKET:
       MPDOK_ARG_CHECK(value >= 0 && value < (1LL << 30), "first ticket out of range");
