@@ -275,7 +275,7 @@ static int chol_pcg_ir_body(void* plan, const Residual64& R, const Residual64& A
     MPDOK_TRY(R.apply(R.ctx, w.B, w.X, w.R, w.parts, K, n, s));
     MPDOK_TRY(cdots(w, w.R, w.R, n, K, rn.data(), s));
     double worst = 0.0;
-    for (int c = 0; c < K; ++c) worst = std::max(worst, bn[c] > 0 ? std::sqrt(rn[c]) / bn[c] : std::sqrt(rn[c]));
+    for (int c = 0; c < K; ++c) worst = worse_residual(worst, bn[c] > 0 ? std::sqrt(rn[c]) / bn[c] : std::sqrt(rn[c]));
     hist_push_info(info, outer, worst);
     if (!std::isfinite(worst)) { set_error("Cholesky-preconditioned CG-IR: non-finite residual"); return MPDOK_ERR_NONFINITE; }
     if (worst < tol) { converged = true; break; }

@@ -1372,7 +1372,7 @@ int cg_ir_core(const CgIrWs& w, const Operator32& A, const Residual64& R, const 
     double worst = 0.0;
     for (int j = 0; j < K; ++j) {
       const double rel = bn[j] > 0 ? std::sqrt(rn[j]) / bn[j] : 0.0;
-      worst = std::max(worst, rel);
+      worst = worse_residual(worst, rel);
     }
     hist_push(info, outer, worst);
     if (!std::isfinite(worst)) { set_error("CG-IR: non-finite residual"); return MPDOK_ERR_NONFINITE; }

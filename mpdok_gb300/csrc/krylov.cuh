@@ -2,6 +2,8 @@
 #pragma once
 #include "gemv.cuh"
 
+#include <cmath>
+
 namespace mpdok {
 
 // Device scalars of one solve (one cache line each group).
@@ -62,6 +64,9 @@ struct Operator32 {
   // workspace until its next product), which an Arnoldi step adds itself
   int (*partials)(const void* ctx, const float* x, cudaStream_t s, const int* skip, const float** P, int* S) = nullptr;
 };
+
+// The worse of two relative residuals, a NaN above all (std::max passes over it).
+inline double worse_residual(double a, double b) { return std::isfinite(a) && !(b <= a) ? b : a; }
 
 // FP64 residual r = b - A x (nrhs columns, leading dimension ld) with
 // per-column ||r||^2 into nrm2[0..nrhs).
