@@ -395,7 +395,9 @@ MPDOK_API int mpdok_batch_load(void* plan, const double* coords, const double* e
                                cudaStream_t stream);
 /* Assemble and factor every system (no host synchronisation). */
 MPDOK_API int mpdok_batch_factor(void* plan, cudaStream_t stream);
-/* X = A^{-1} B with `refine` FP64 refinement steps (no host synchronisation). */
+/* X = A^{-1} B with `refine` FP64 refinement steps (no host synchronisation).
+ * Solves of one plan may be issued on several streams and by several threads;
+ * they run one after the other. */
 MPDOK_API int mpdok_batch_solve(void* plan, const double* B, double* X, int refine, cudaStream_t stream);
 /* relres[s] = max over RHS of ||B - A X|| / ||B|| (device array, caller order). */
 MPDOK_API int mpdok_batch_relres(void* plan, const double* B, const double* X, double* relres, cudaStream_t stream);

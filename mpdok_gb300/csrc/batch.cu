@@ -40,6 +40,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <numeric>
 #include <vector>
 
@@ -73,10 +74,13 @@ struct BatchPlan {
   BSys* d_sys = nullptr;
   long long* d_pre = nullptr;         // preT | preS | preRow
   long long d_preS_base = 0, d_preRow_base = 0, d_preLvl_base = 0;
-  double* arena = nullptr;            // A | Linv | V | R | rowscratch
+  double* arena = nullptr;            // A | Linv | V | R | S | rowscratch | coordinates
   double *A = nullptr, *Linv = nullptr, *V = nullptr, *R = nullptr, *rows = nullptr, *coords = nullptr;
   int* d_pert = nullptr;
-  int* d_ticket = nullptr;            // the solves: forward and backward ticket, timed-out wait
+  double* S = nullptr;                // scratch of the solves (total_x), in the order of `solved`
+  int* d_ticket = nullptr;            // the same: forward and backward ticket, timed-out wait
+  cudaEvent_t solved = nullptr;       // the last use of S and d_ticket
+  std::mutex solve_mu;
   int* timed_out = nullptr;           // pinned: a wait of some solve ran out (kept until it is reported)
   size_t bytes = 0;
   int syrk_grid = 0;
@@ -1465,28 +1469,27 @@ int batch_timed_out(void* plan) {
   return MPDOK_ERR_TIMEOUT;
 }
 
-// V := A^{-1} V in place (V in the caller's packing), through the plan's R.
-static int batch_solve_inplace(BatchPlan* p, double* V, cudaStream_t s) {
+// V := A^{-1} V in place (V in the caller's packing) through R (as long); tk: two
+// tickets and the word that ends the waits of a solve once one of them ran out,
+// which the caller clears.
+static int batch_solve_inplace(BatchPlan* p, double* V, double* R, int* tk, cudaStream_t s) {
   const size_t bytes = (size_t)p->total_x * sizeof(double);
   const int groups = (p->nrhs + BSOLVE_RHS - 1) / BSOLVE_RHS;
   const unsigned grid = (unsigned)(p->preLvl.back() * groups);
   if (grid == 0) return MPDOK_OK;
   MPDOK_TRY(set_smem(k_bsolve_chain<false>, BSOLVE_SMEM));
   MPDOK_TRY(set_smem(k_bsolve_chain<true>, BSOLVE_SMEM));
-  // (the error word too: a wait that ran out ends this solve's waits, not the next one's)
-  MPDOK_CUDA_TRY(cudaMemsetAsync(p->d_ticket, 0, 3 * sizeof(int), s));
+  MPDOK_CUDA_TRY(cudaMemsetAsync(tk, 0, 2 * sizeof(int), s));
   if (const int t0 = debug_first_ticket()) {
-    MPDOK_CUDA_TRY(cudaMemcpyAsync(p->d_ticket, &t0, sizeof(int), cudaMemcpyHostToDevice, s));
+    MPDOK_CUDA_TRY(cudaMemcpyAsync(tk, &t0, sizeof(int), cudaMemcpyHostToDevice, s));
     MPDOK_CUDA_TRY(cudaStreamSynchronize(s));
   }
-  MPDOK_CUDA_TRY(cudaMemsetAsync(p->R, 0xff, bytes, s));
+  MPDOK_CUDA_TRY(cudaMemsetAsync(R, 0xff, bytes, s));
   launch(k_bsolve_chain<false>, dim3(grid), BT, BSOLVE_SMEM, s, (const BSys*)p->d_sys, preLvl_dev(p), p->maxblk,
-         p->nrhs, (const double*)p->A, (const double*)p->Linv, (const double*)V, p->R, p->d_ticket, p->d_ticket + 2,
-         p->timed_out);
+         p->nrhs, (const double*)p->A, (const double*)p->Linv, (const double*)V, R, tk, tk + 2, p->timed_out);
   MPDOK_CUDA_TRY(cudaMemsetAsync(V, 0xff, bytes, s));
   launch(k_bsolve_chain<true>, dim3(grid), BT, BSOLVE_SMEM, s, (const BSys*)p->d_sys, preLvl_dev(p), p->maxblk,
-         p->nrhs, (const double*)p->A, (const double*)p->Linv, (const double*)p->R, V, p->d_ticket + 1,
-         p->d_ticket + 2, p->timed_out);
+         p->nrhs, (const double*)p->A, (const double*)p->Linv, (const double*)R, V, tk + 1, tk + 2, p->timed_out);
   MPDOK_LAUNCH_CHECK("batch solve");
   return MPDOK_OK;
 }
@@ -1500,67 +1503,53 @@ static int batch_residual(BatchPlan* p, const double* B, const double* X, double
   return MPDOK_OK;
 }
 
-static int batch_solve(BatchPlan* p, const double* B, double* X, int refine, cudaStream_t s) {
+static int batch_solve_with(BatchPlan* p, const double* B, double* X, int refine, double* R, int* tk, cudaStream_t s) {
   const long long nx = p->total_x;
-  if (nx == 0) return MPDOK_OK;
+  MPDOK_CUDA_TRY(cudaMemsetAsync(tk + 2, 0, sizeof(int), s));
   MPDOK_CUDA_TRY(cudaMemcpyAsync(X, B, (size_t)nx * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  MPDOK_TRY(batch_solve_inplace(p, X, s));
+  MPDOK_TRY(batch_solve_inplace(p, X, R, tk, s));
   const unsigned g = (unsigned)std::min<long long>((nx + 255) / 256, (long long)num_sms() * 8);
   for (int it = 0; it < refine; ++it) {
     MPDOK_TRY(batch_residual(p, B, X, p->V, s));
-    MPDOK_TRY(batch_solve_inplace(p, p->V, s));
+    MPDOK_TRY(batch_solve_inplace(p, p->V, R, tk, s));
     launch(k_badd, dim3(g), 256, 0, s, X, (const double*)p->V, nx);
   }
   MPDOK_LAUNCH_CHECK("batch refine");
   return MPDOK_OK;
 }
 
-// FP32 columns (leading dimension ld) <-> the plan's FP64 packing (n x K, ld n).
-__global__ void k_cols_f32_to_f64(const float* __restrict__ v, long long ld, double* __restrict__ t, long long n,
-                                  int K) {
-  const long long total = n * K;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x)
-    t[e] = (double)v[(e / n) * ld + e % n];
-}
-__global__ void k_cols_f64_to_f32(const double* __restrict__ t, float* __restrict__ z, long long ld, long long n,
-                                  int K) {
-  const long long total = n * K;
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x)
-    z[(e / n) * ld + e % n] = (float)t[e];
-}
-
-static int bpc_apply_cols(void* ctx, const float* v, float* z, int K, long long ld, cudaStream_t s) {
-  BatchPcCtx* c = (BatchPcCtx*)ctx;
-  BatchPlan* p = (BatchPlan*)c->plan;
-  const long long total = c->n * K;
-  const unsigned g = (unsigned)std::max(1LL, std::min<long long>((total + 255) / 256, (long long)num_sms() * 8));
-  launch(k_cols_f32_to_f64, g, 256, 0, s, v, ld, c->tmp, c->n, K);
-  MPDOK_TRY(batch_solve_inplace(p, c->tmp, s));
-  launch(k_cols_f64_to_f32, g, 256, 0, s, (const double*)c->tmp, z, ld, c->n, K);
-  MPDOK_LAUNCH_CHECK("batch preconditioner");
-  return MPDOK_OK;
+// A caller may have several solves of one plan in flight on several streams.  They
+// share S and the tickets (V too, with refinement): each starts after the one
+// before it.  A solve that is being captured by the caller
+// may be replayed at any time and takes its own scratch into the graph.
+static int batch_solve(BatchPlan* p, const double* B, double* X, int refine, cudaStream_t s) {
+  if (p->total_x == 0) return MPDOK_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  MPDOK_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
+  if (cap != cudaStreamCaptureStatusNone) {
+    const size_t vec = align_up((size_t)p->total_x * sizeof(double), 256);
+    void* own = nullptr;
+    MPDOK_CUDA_TRY(cudaMallocAsync(&own, vec + 256, s));
+    const int st = batch_solve_with(p, B, X, refine, (double*)own, (int*)((char*)own + vec), s);
+    MPDOK_CUDA_TRY(cudaFreeAsync(own, s));
+    return st;
+  }
+  std::lock_guard<std::mutex> lk(p->solve_mu);
+  MPDOK_CUDA_TRY(cudaStreamWaitEvent(s, p->solved, 0));
+  const int st = batch_solve_with(p, B, X, refine, p->S, p->d_ticket, s);
+  MPDOK_CUDA_TRY(cudaEventRecord(p->solved, s));
+  return st;
 }
 
-int batch_apply_f64(void* plan, long long n, int K, double* V, cudaStream_t s) {
-  MPDOK_ARG_CHECK(plan && V, "null pointer");
+// V := A^{-1} V for the Cholesky-preconditioned CG-IR; R as long as V and tk (3
+// ints, tk[2] cleared by the caller) are the solve's own, since several of them
+// may share a plan.
+int batch_apply_f64(void* plan, long long n, int K, double* V, double* R, int* tk, cudaStream_t s) {
+  MPDOK_ARG_CHECK(plan && V && R && tk, "null pointer");
   BatchPlan* p = (BatchPlan*)plan;
   MPDOK_ARG_CHECK(p->nsys == 1 && p->sys[0].n == n, "the preconditioner plan must hold one system of size n");
   MPDOK_ARG_CHECK(p->nrhs == K, "the preconditioner plan's nrhs must equal the solve's nrhs");
-  return batch_solve_inplace(p, V, s);
-}
-
-int batch_precond(void* plan, long long n, int K, double* tmp, BatchPcCtx* ctx, Precond* pc) {
-  MPDOK_ARG_CHECK(plan && tmp && ctx && pc, "null pointer");
-  BatchPlan* p = (BatchPlan*)plan;
-  MPDOK_ARG_CHECK(p->nsys == 1 && p->sys[0].n == n, "the preconditioner plan must hold one system of size n");
-  MPDOK_ARG_CHECK(p->nrhs == K, "the preconditioner plan's nrhs must equal the solve's nrhs");
-  ctx->plan = plan;
-  ctx->tmp = tmp;
-  ctx->n = n;
-  pc->apply = nullptr;
-  pc->apply_cols = bpc_apply_cols;
-  pc->ctx = ctx;
-  return MPDOK_OK;
+  return batch_solve_inplace(p, V, R, tk, s);
 }
 
 static void dag_release(BatchPlan* p) {
@@ -1716,6 +1705,7 @@ static void plan_free(BatchPlan* p) {
   if (p->d_pert) cudaFree(p->d_pert);
   if (p->d_ticket) cudaFree(p->d_ticket);
   if (p->timed_out) cudaFreeHost(p->timed_out);
+  if (p->solved) cudaEventDestroy(p->solved);
   delete p;
 }
 
@@ -1826,16 +1816,19 @@ extern "C" int mpdok_batch_create(int nsys, const long long* n, int dim, int nrh
   e = cudaHostAlloc((void**)&p->timed_out, sizeof(int), cudaHostAllocPortable);
   if (e != cudaSuccess) return fail(e, "cudaHostAlloc (batch status)");
   *p->timed_out = 0;
+  e = cudaEventCreateWithFlags(&p->solved, cudaEventDisableTiming);
+  if (e != cudaSuccess) return fail(e, "cudaEventCreate (batch)");
   const size_t nA = align_up((size_t)aA, 32), nL = align_up((size_t)aL, 32), nV = align_up((size_t)ax, 32),
                nR = align_up((size_t)aR, 32), nCo = align_up((size_t)ac, 32);
-  p->bytes = (nA + nL + 2 * nV + nR + nCo) * sizeof(double);
+  p->bytes = (nA + nL + 3 * nV + nR + nCo) * sizeof(double);
   e = cudaMalloc(&p->arena, p->bytes);
   if (e != cudaSuccess) return fail(e, "cudaMalloc (batch arena)");
   p->A = p->arena;
   p->Linv = p->A + nA;
   p->V = p->Linv + nL;
   p->R = p->V + nV;
-  p->rows = p->R + nV;
+  p->S = p->R + nV;
+  p->rows = p->S + nV;
   p->coords = p->rows + nR;
   e = cudaMemset(p->Linv, 0, nL * sizeof(double));
   if (e != cudaSuccess) return fail(e, "cudaMemset (batch)");
@@ -1994,7 +1987,7 @@ extern "C" int mpdok_batch_graph_build(void* plan, const double* B, double* X, i
     st = batch_step_dag(p, B, X, refine, p->cap);
   } else {
     st = batch_factor(p, p->cap);
-    if (st == MPDOK_OK) st = batch_solve(p, B, X, refine, p->cap);
+    if (st == MPDOK_OK && p->total_x > 0) st = batch_solve_with(p, B, X, refine, p->S, p->d_ticket, p->cap);
   }
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(p->cap, &g);
@@ -2019,7 +2012,10 @@ extern "C" int mpdok_batch_graph_launch(void* plan, cudaStream_t s) {
     return MPDOK_ERR_NOT_FACTORED;
   }
   MPDOK_TRY(batch_timed_out(plan));
+  std::lock_guard<std::mutex> lk(p->solve_mu);
+  MPDOK_CUDA_TRY(cudaStreamWaitEvent(s, p->solved, 0));
   MPDOK_CUDA_TRY(cudaGraphLaunch(p->exec, s));
+  MPDOK_CUDA_TRY(cudaEventRecord(p->solved, s));
   count_launch();
   return MPDOK_OK;
 }

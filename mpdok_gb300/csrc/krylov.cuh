@@ -104,18 +104,11 @@ struct Precond {
   int (*apply_cols)(void* ctx, const float* v, float* z, int K, long long ld, cudaStream_t s) = nullptr;
 };
 
-// Preconditioner z = A^-1 v from the Cholesky factor held in a batch plan of
-// one system of size n with nrhs == K (double-float trailing update, FP64
-// diagonal blocks and solves); tmp holds n * K doubles.  Defined in batch.cu.
-struct BatchPcCtx {
-  void* plan = nullptr;
-  double* tmp = nullptr;
-  long long n = 0;
-};
-int batch_precond(void* plan, long long n, int K, double* tmp, BatchPcCtx* ctx, Precond* pc);
 // V := A^-1 V in FP64 with the Cholesky factor of a batch plan of one system
-// (V: n x K column-major, ld n, K = the plan's nrhs).  Defined in batch.cu.
-int batch_apply_f64(void* plan, long long n, int K, double* V, cudaStream_t s);
+// (V: n x K column-major, ld n, K = the plan's nrhs), through R (as long as V) and
+// tk (two tickets; tk[2] is set when a wait ran out, and the caller clears it).
+// Defined in batch.cu.
+int batch_apply_f64(void* plan, long long n, int K, double* V, double* R, int* tk, cudaStream_t s);
 
 // MPDOK_ERR_TIMEOUT, once, when a wait of a finished solve of the plan ran out.
 int batch_timed_out(void* plan);
