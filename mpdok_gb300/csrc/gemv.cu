@@ -222,16 +222,24 @@ gemv_finalize(const ACC* __restrict__ P, int S, int K, long long m, ACC alpha, A
   }
 }
 
-// FP64 y = alpha A x + beta bsrc of a small matrix in one launch, with the sum
-// of squares of y.  The products and their sums carry their rounding errors
-// along (two-product by FMA, two-sum), so y is the rounded exact result: the
-// residual of a refinement subtracts nearly equal vectors, and its own rounding
-// otherwise sets the residual that can be reached (n = 400, kappa 1e5: the
-// computed residual of the rounded solution is 1.7e-13 of ||b||, the true one
-// 0.7e-13).  Ten FP64 operations per entry instead of one, but a single launch
-// with every entry's load in flight at once.  Eight rows per block; 32 threads
-// per row take every 32nd column.
-constexpr long long GEMV_SMALL = 1LL << 19;  // entries: above, the FP64 pipe makes it slower than the two-pass form
+// FP64 y = alpha A x + beta bsrc of a small matrix, with the sum of squares of y.
+// The products and their sums carry their rounding errors along (two-product by
+// FMA, two-sum), so y is the rounded exact result: the residual of a refinement
+// subtracts nearly equal vectors, and its own rounding otherwise sets the residual
+// that can be reached (n = 400, kappa 1e5: the computed residual of the rounded
+// solution is 1.7e-13 of ||b||, the true one 0.7e-13).  Eleven FP64 operations per
+// entry instead of one: bound by that pipe (16 clocks an instruction), so all SMs
+// have to share the work.  Eight rows per block; 32 threads per row take every 32nd
+// column; of a matrix with few rows the columns are split over blocks, which leave
+// their sums in P for a second launch (PARTS).
+//
+// Taken up to 2^19 entries, above which the pipe makes it much slower than the
+// two-pass form, and up to 64 rows per column: below that the sums across the
+// threads of a row weigh more than its products (16384 x 32: 35 us against 8).
+// In us, two-pass form / one split / this rule: 1 x 5000 13.4 / 117 / 11.5,
+// 1 x 524288 163 / 11850 / 90, 64 x 8192 16.6 / 190 / 18.0, 600 x 600 12.8 / 18.3 /
+// 15.2, 724 x 724 13.2 / 21.1 / 21.2, 5000 x 104 11.3 / 22.3 / 22.3.
+constexpr long long GEMV_SMALL = 1LL << 19, GEMV_TALL = 64;
 
 struct DD {
   double s, c;
@@ -241,22 +249,28 @@ __device__ __forceinline__ DD dd_add(DD a, DD b) {
   return {t, ((a.s - (t - bb)) + (b.s - bb)) + (a.c + b.c)};
 }
 
+template <bool PARTS>
 __global__ void __launch_bounds__(GEMV_THREADS)
-gemv_n_small_f64(const double* __restrict__ A, long long lda, int m, int n, const double* __restrict__ x, double alpha,
-                 double beta, const double* bsrc, double* y, double* nrm_parts, unsigned* ticket, double* nrm2,
-                 const int* skip) {
+gemv_n_small_f64(const double* __restrict__ A, long long lda, int m, int n, int chunk, const double* __restrict__ x,
+                 double alpha, double beta, const double* bsrc, double* y, DD* P, double* nrm_parts, unsigned* ticket,
+                 double* nrm2, const int* skip) {
   __shared__ DD sp[8][8];
   __shared__ double red[32];
   if (skip != nullptr && *skip) return;
   const int rl = threadIdx.x & 7, g = threadIdx.x >> 3, warp = threadIdx.x >> 5;
   const int row = blockIdx.x * 8 + rl;
+  const int c0 = blockIdx.y * chunk, c1 = min(n, c0 + chunk);
   DD a = {0.0, 0.0};
   if (row < m) {
 #pragma unroll 4
-    for (int j = g; j < n; j += GEMV_THREADS / 8) {
-      const double av = __ldg(A + row + (long long)j * lda), xv = __ldg(x + j);
-      const double p = av * xv;
-      a = dd_add(a, {p, fma(av, xv, -p)});
+    for (int j = c0 + g; j < c1; j += GEMV_THREADS / 8) {  // (PARTS: n is the number of partial sums)
+      if constexpr (PARTS) {
+        a = dd_add(a, P[(long long)j * m + row]);
+      } else {
+        const double av = __ldg(A + row + (long long)j * lda), xv = __ldg(x + j);
+        const double p = av * xv;
+        a = dd_add(a, {p, fma(av, xv, -p)});
+      }
     }
   }
   auto across = [&](DD v) {  // over the lanes of one row: 8 and 16 apart
@@ -268,18 +282,18 @@ gemv_n_small_f64(const double* __restrict__ A, long long lda, int m, int n, cons
   a = across(a);
   if ((threadIdx.x & 31) < 8) sp[warp][rl] = a;
   __syncthreads();
+  if (warp == 0) a = across(dd_add(sp[g][rl], sp[g + 4][rl]));
   double sq = 0.0;
-  if (warp == 0) {
-    a = across(dd_add(sp[g][rl], sp[g + 4][rl]));
-    if (g == 0 && row < m) {
+  if (g == 0 && row < m) {
+    if (!PARTS && P != nullptr) {
+      P[(long long)blockIdx.y * m + row] = a;
+    } else {
       const double b = beta != 0.0 ? bsrc[row] : 0.0;
       const double p = alpha * a.s, q = beta * b;
       const DD r = dd_add({q, fma(beta, b, -q)}, {p, fma(alpha, a.s, -p) + alpha * a.c});
       double v = r.s + r.c;
-      if (!isfinite(v)) {  // infinities do not survive the error terms: the plain sum
-        double t = 0.0;
-        for (int j = 0; j < n; ++j) t = fma(A[row + (long long)j * lda], x[j], t);
-        v = alpha * t;
+      if (!isfinite(v)) {  // infinities do not survive the error terms; a.s is the plain sum
+        v = p;
         if (beta != 0.0) v = fma(beta, b, v);
       }
       y[row] = v;
@@ -290,6 +304,13 @@ gemv_n_small_f64(const double* __restrict__ A, long long lda, int m, int n, cons
     const double b = block_sum(sq, red);
     ordered_grid_sum(b, nrm_parts, ticket, nrm2);
   }
+}
+
+// Splits of the columns, S those of the two-pass form: as many as give every SM a
+// block, of at least 128 columns, and few enough that their sums and m norm parts
+// fit that form's S m doubles.
+static int small_splits(long long m, long long n, long long S) {
+  return (int)std::max(1LL, std::min({num_sms() / ((m + 7) / 8), n / 128, (S - 1) / 2}));
 }
 
 static unsigned finalize_blocks(long long total) {
@@ -390,12 +411,20 @@ int gemv_launch(int a_dtype, bool trans, const void* A, long long lda, long long
     const char* Xk = (const char*)X + (size_t)done * ldx * acc_bytes;
     char* Yk = (char*)Y + (size_t)done * ldy * acc_bytes;
     const char* Bk = Bsrc ? (const char*)Bsrc + (size_t)done * ldb * acc_bytes : nullptr;
-    if (a_dtype == MPDOK_F64 && !trans && K == 1 && red > 0 && m * n <= GEMV_SMALL) {
+    if (a_dtype == MPDOK_F64 && !trans && K == 1 && red > 0 && m * n <= GEMV_SMALL && m <= GEMV_TALL * n) {
       if (nrm2 && zero_ticket) MPDOK_CUDA_TRY(cudaMemsetAsync(ticket, 0, sizeof(unsigned), s));
       const int pslot = prof_start(MPDOK_PROF_GEMV_F64, s);
-      // (the blocks' norm parts, m / 8 of them, fit the partial-sum buffer of m doubles per split)
-      launch(gemv_n_small_f64, (unsigned)((m + 7) / 8), GEMV_THREADS, 0, s, (const double*)A, lda, (int)m, (int)n,
-             (const double*)Xk, alpha, beta, (const double*)Bk, (double*)Yk, (double*)P, ticket, nrm2, skip);
+      const int splits = small_splits(m, n, p.S);
+      DD* sums = splits > 1 ? (DD*)P : nullptr;
+      // the blocks' norm parts, behind the splits' sums
+      double* parts = (double*)P + (splits > 1 ? 2 * splits * m : 0);
+      const unsigned gx = (unsigned)((m + 7) / 8);
+      launch(gemv_n_small_f64<false>, dim3(gx, splits), GEMV_THREADS, 0, s, (const double*)A, lda, (int)m, (int)n,
+             ((int)n + splits - 1) / splits, (const double*)Xk, alpha, beta, (const double*)Bk, (double*)Yk, sums, parts,
+             ticket, splits > 1 ? (double*)nullptr : nrm2, skip);
+      if (splits > 1)
+        launch(gemv_n_small_f64<true>, gx, GEMV_THREADS, 0, s, (const double*)nullptr, 0LL, (int)m, splits, splits,
+               (const double*)nullptr, alpha, beta, (const double*)Bk, (double*)Yk, sums, parts, ticket, nrm2, skip);
       prof_stop(pslot, s, (double)m * (double)n * eb + (double)(m + n) * acc_bytes, skip);
       MPDOK_LAUNCH_CHECK("gemv small");
       done += K;
