@@ -182,7 +182,9 @@ gemv_t_stage1(const TA* __restrict__ A, long long lda, long long m, long long n,
 // block sums FIN_ROWS entries, four threads to an entry (every fourth split,
 // eight loads in flight): bound by the latency of the loads, so the splits are
 // spread rather than walked (n = 8192, 76 splits: 5.7 us; 10.2 us with one
-// thread to an entry).  The order of the sum is fixed.
+// thread to an entry).  Up to four splits, a thread takes an entry: the same order,
+// and three threads of four would have nothing to add (FP64, m = 524288, one
+// split: 8.7 us in all, 16.8 spread).  The order of the sum is fixed.
 constexpr int FIN_ROWS = GEMV_THREADS / 4;
 template <typename ACC>
 __global__ void __launch_bounds__(GEMV_THREADS)
@@ -195,7 +197,23 @@ gemv_finalize(const ACC* __restrict__ P, int S, int K, long long m, ACC alpha, A
   const long long total = m * K;
   const int r = threadIdx.x % FIN_ROWS, q = threadIdx.x / FIN_ROWS;
   double sq = 0.0;
-  for (long long b0 = (long long)blockIdx.x * FIN_ROWS; b0 < total; b0 += (long long)gridDim.x * FIN_ROWS) {
+  auto put = [&](long long idx, ACC sum) {
+    const long long i = idx % m;
+    const int k = (int)(idx / m);
+    ACC v = alpha * sum;
+    if (beta != ACC(0)) v = fma(beta, bsrc[i + k * ldb], v);
+    y[i + k * ldy] = v;
+    sq += (double)v * (double)v;
+  };
+  if (S <= 4) {
+    for (long long idx = (long long)blockIdx.x * GEMV_THREADS + threadIdx.x; idx < total;
+         idx += (long long)gridDim.x * GEMV_THREADS) {
+      ACC sum = ACC(0);
+      for (int s = 0; s < S; ++s) sum += P[s * total + idx];
+      put(idx, sum);
+    }
+  }
+  for (long long b0 = S <= 4 ? total : (long long)blockIdx.x * FIN_ROWS; b0 < total; b0 += (long long)gridDim.x * FIN_ROWS) {
     const long long idx = b0 + r;
     ACC sum = ACC(0);
     if (idx < total) {
@@ -205,15 +223,7 @@ gemv_finalize(const ACC* __restrict__ P, int S, int K, long long m, ACC alpha, A
     }
     part[q][r] = sum;
     __syncthreads();
-    if (q == 0 && idx < total) {
-      const long long i = idx % m;
-      const int k = (int)(idx / m);
-      sum = ((sum + part[1][r]) + part[2][r]) + part[3][r];
-      ACC v = alpha * sum;
-      if (beta != ACC(0)) v = fma(beta, bsrc[i + k * ldb], v);
-      y[i + k * ldy] = v;
-      sq += (double)v * (double)v;
-    }
+    if (q == 0 && idx < total) put(idx, ((sum + part[1][r]) + part[2][r]) + part[3][r]);
     __syncthreads();
   }
   if (nrm2 != nullptr) {

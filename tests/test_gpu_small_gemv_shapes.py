@@ -73,3 +73,25 @@ def test_residual_with_its_norm(n):
         N.check(lib.mpdok_residual(ptr(A), n, n, ptr(b), ptr(x), ptr(r), ptr(nrm), ptr(w), w.numel(), stream_handle()), "residual")
     assert abs(nrm.item() - (r * r).sum().item()) <= 2 * n * 2.0 ** -53 * nrm.item()
     assert (r - (b - A.t() @ x)).abs().max().item() <= 4 * n * 2.0 ** -53 * (A.abs().t() @ x.abs()).max().item()
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("m,n,k", [(200000, 3, 1), (70000, 200, 3), (40000, 300, 8), (3000, 260, 1)])
+def test_products_of_few_and_of_many_splits(m, n, k, dtype):
+    """One to four splits (a thread adds an entry) and more: n u of |A| |X|, with
+    rows that end inside a block."""
+    from mpdok_gb300 import _native as N
+    from mpdok_gb300._device import ptr, stream_handle
+    g = torch.Generator("cuda").manual_seed(m)
+    A = torch.randn(n, m, dtype=dtype, device="cuda", generator=g)
+    X = torch.randn(k, n, dtype=dtype, device="cuda", generator=g)
+    Y0 = torch.randn(k, m, dtype=dtype, device="cuda", generator=g)
+    Y = Y0.clone()
+    lib = N.load()
+    code = N.F64 if dtype == torch.float64 else N.F32
+    w = torch.empty(lib.mpdok_gemv_workspace_size(code, m, n, k, 0), dtype=torch.uint8, device="cuda")
+    N.check(lib.mpdok_gemv(code, 0, ptr(A), m, m, n, ptr(X), n, k, ptr(Y), m, 1.5, -0.5, ptr(w), w.numel(),
+                           stream_handle()), "gemv")
+    ref = 1.5 * (X.double() @ A.double()) - 0.5 * Y0.double()
+    bound = (n + 4) * torch.finfo(dtype).eps * (1.5 * (X.abs().double() @ A.abs().double()) + 0.5 * Y0.abs().double())
+    assert torch.all((Y.double() - ref).abs() <= bound)
