@@ -323,6 +323,11 @@ static int small_splits(long long m, long long n, long long S) {
   return (int)std::max(1LL, std::min({num_sms() / ((m + 7) / 8), n / 128, (S - 1) / 2}));
 }
 
+static bool overlap(const void* a, long long na, const void* b, long long nb) {  // of doubles
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+  return x < y + nb * sizeof(double) && y < x + na * sizeof(double);
+}
+
 static unsigned finalize_blocks(long long total) {
   long long b = (total + FIN_ROWS - 1) / FIN_ROWS;
   long long cap = (long long)num_sms() * 4;
@@ -421,7 +426,10 @@ int gemv_launch(int a_dtype, bool trans, const void* A, long long lda, long long
     const char* Xk = (const char*)X + (size_t)done * ldx * acc_bytes;
     char* Yk = (char*)Y + (size_t)done * ldy * acc_bytes;
     const char* Bk = Bsrc ? (const char*)Bsrc + (size_t)done * ldb * acc_bytes : nullptr;
-    if (a_dtype == MPDOK_F64 && !trans && K == 1 && red > 0 && m * n <= GEMV_SMALL && m <= GEMV_TALL * n) {
+    // (in one launch a block may write its y while another still reads x and A, so
+    // a product in place is the two-pass form's)
+    if (a_dtype == MPDOK_F64 && !trans && K == 1 && red > 0 && m * n <= GEMV_SMALL && m <= GEMV_TALL * n &&
+        !overlap(Yk, m, Xk, n) && !overlap(Yk, m, A, lda * (n - 1) + m)) {
       if (nrm2 && zero_ticket) MPDOK_CUDA_TRY(cudaMemsetAsync(ticket, 0, sizeof(unsigned), s));
       const int pslot = prof_start(MPDOK_PROF_GEMV_F64, s);
       const int splits = small_splits(m, n, p.S);

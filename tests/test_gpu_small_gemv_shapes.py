@@ -95,3 +95,17 @@ def test_products_of_few_and_of_many_splits(m, n, k, dtype):
     ref = 1.5 * (X.double() @ A.double()) - 0.5 * Y0.double()
     bound = (n + 4) * torch.finfo(dtype).eps * (1.5 * (X.abs().double() @ A.abs().double()) + 0.5 * Y0.abs().double())
     assert torch.all((Y.double() - ref).abs() <= bound)
+
+
+@pytest.mark.parametrize("n", [40, 300, 724])
+@pytest.mark.parametrize("where", ["x", "column"])
+def test_products_in_place(n, where):
+    """y = x, or y a column of A: every entry is read before y is written (n u of |A| |x|)."""
+    g = torch.Generator("cuda").manual_seed(n)
+    S = torch.randn(n, n, dtype=torch.float64, device="cuda", generator=g)
+    x = torch.randn(n, dtype=torch.float64, device="cuda", generator=g)
+    want, bound = S.t() @ x, n * 2.0 ** -52 * (S.abs().t() @ x.abs())
+    for _ in range(3):
+        A, v = S.clone().t(), x.clone()
+        y = _gemv(A, v, v if where == "x" else A[:, n // 2], 1.0, 0.0)
+        assert torch.all((y - want).abs() <= bound)
