@@ -15,8 +15,9 @@
 // S ways for occupancy; splits are combined in a fixed order (bitwise
 // reproducible).  Bound: the special-function pipe (one MUFU op per entry).
 //
-// FP64 kernel (residuals): the same loop in FP64 arithmetic with CUDA's exp /
-// sqrt, for r = b - K x accurate to FP64 rounding.
+// FP64 kernel (residuals): the same loop in FP64 arithmetic, for r = b - K x
+// accurate to FP64 rounding: the multiquadric with CUDA's sqrt, the Gaussian with
+// the integer-pipe exponential of phi64.cuh.
 #include "krylov.cuh"
 #include "matfree.cuh"
 #include "phi64.cuh"
@@ -179,8 +180,12 @@ k_matfree_f32(const __grid_constant__ CUtensorMap tmC, const __grid_constant__ C
 // operations for d^2 and K for the products; the exponential runs on the
 // integer pipe (phi64.cuh).  20000 centres x 16384 rows, D = 2, K = 3: 4.3 ms
 // (16.5 ms with CUDA's exp; the 7 FP64 operations per entry alone take 3.6 ms).
+// Six CTAs per SM, as the kernel had before D and K were compiled in: with 48
+// registers for K = 7 and 8 only five ran, and the few blocks of a short query
+// took a second wave (200000 centres, K = 8, multiquadric, 1 / 100 points: 590 /
+// 1590 us with five, 416 / 1248 with six, 478 / 1402 before).
 template <int KIND, int D, int K>
-__global__ void __launch_bounds__(MF_THREADS)
+__global__ void __launch_bounds__(MF_THREADS, 6)
 k_matfree_f64(const double* __restrict__ rows, const double* __restrict__ cols, long long nrows, long long ncols,
               long long chunk, GaussScale gs, const double* __restrict__ X, long long ldx, double* __restrict__ P) {
   __shared__ uint64_t sT[KIND == MPDOK_KERNEL_GAUSSIAN ? PHI_TAB : 1];
