@@ -77,8 +77,9 @@ MPDOK_API void mpdok_clear_error(void);
 
 /* Test hooks for the failure paths; no counterpart in the reference.
  * MPDOK_DEBUG_WAIT_LIMIT: iteration limit of the triangular solves' bounded
- *   waits on a predecessor block, of LU factors and of batches, on the current
- *   device (value <= 0 restores the default).
+ *   waits on a predecessor block, of LU factors, on the current device (value <= 0
+ *   restores the default); with a value below the default the batch solves
+ *   issued from then on wait 4096 iterations.
  * MPDOK_DEBUG_TRSV_FIRST_TICKET: first ticket that the next triangular solves
  *   of this process hand out (0 = normal).  With a value above 0 no block ever
  *   solves block 0, so the blocks that depend on it wait until their limit

@@ -77,9 +77,8 @@ struct BatchPlan {
   double* arena = nullptr;            // A | Linv | V | R | S | rowscratch | coordinates
   double *A = nullptr, *Linv = nullptr, *V = nullptr, *R = nullptr, *rows = nullptr, *coords = nullptr;
   int* d_pert = nullptr;
-  double* S = nullptr;                // scratch of the solves (total_x), in the order of `solved`
-  int* d_ticket = nullptr;            // the same: forward and backward ticket, timed-out wait
-  cudaEvent_t solved = nullptr;       // the last use of S and d_ticket
+  double* S = nullptr;                // scratch of the solves (total_x, then SOLVE_WORDS), in the order of `solved`
+  cudaEvent_t solved = nullptr;       // the last use of S
   std::mutex solve_mu;
   int* timed_out = nullptr;           // pinned: a wait of some solve ran out (kept until it is reported)
   size_t bytes = 0;
@@ -549,8 +548,8 @@ __device__ __forceinline__ double diag_dot(const double* sLi, const double* sx, 
 
 // Results start as this bit pattern; consumers poll the values themselves.
 constexpr unsigned long long BSOLVE_EMPTY = 0xffffffffffffffffull;
-constexpr long long BSOLVE_WAIT = 1LL << 24;
-__device__ long long g_bsolve_wait = BSOLVE_WAIT;  // (a device variable so that a test can shorten it)
+constexpr int BSOLVE_WAIT = 1 << 24, BSOLVE_WAIT_SHORT = 1 << 12;
+static bool g_short_wait = false;  // (a test hook)
 constexpr int BSOLVE_RHS = 4;    // right-hand sides of one CTA
 constexpr size_t BSOLVE_SMEM = (size_t)BNB * BPAD * (sizeof(double) + sizeof(DF)) +
                                (size_t)BNB * BSOLVE_RHS * (sizeof(double) + sizeof(DF));
@@ -575,10 +574,14 @@ __device__ __forceinline__ void st_relaxed_u64(double* p, unsigned long long v) 
 // inverse (3 us; four columns to a CTA, since FP64 is what an SM has least of),
 // publish.  32 systems of 300 .. 4000, 8 columns: 0.73 ms forward, 0.69 ms
 // backward; two launches per level took 2.2 and 2.1 ms.
-template <bool TRANS>
+// ALONE: every system is one block, nothing waits, and IN may be OUT (a CTA reads
+// its entries first).  BRIEF: short waits, for tests (the limit is compiled in: as
+// an argument it cost 6% of the kernel).
+enum BSolveMode { CHAIN, ALONE, BRIEF };
+template <bool TRANS, BSolveMode MODE>
 __global__ void __launch_bounds__(BT) k_bsolve_chain(const BSys* __restrict__ sys, const long long* __restrict__ lvl,
                                                      int maxblk, int nrhs, const double* __restrict__ A,
-                                                     const double* __restrict__ Linv, const double* __restrict__ IN,
+                                                     const double* __restrict__ Linv, const double* IN,
                                                      double* OUT, int* ticket, int* err, int* timed_out) {
   extern __shared__ double smem[];
   double* sLi = smem;                                            // [i][c]
@@ -588,7 +591,7 @@ __global__ void __launch_bounds__(BT) k_bsolve_chain(const BSys* __restrict__ sy
   __shared__ int s_t, s_abort;
   const int tid = threadIdx.x;
   if (tid == 0) {
-    s_t = atomicAdd(ticket, 1);
+    s_t = MODE == ALONE ? (int)blockIdx.x : atomicAdd(ticket, 1) + 1;  // (starts at -1)
     s_abort = 0;
   }
   __syncthreads();
@@ -634,24 +637,25 @@ __global__ void __launch_bounds__(BT) k_bsolve_chain(const BSys* __restrict__ sy
     double v = 0.0;
     if (row < nb && r8 + rr < nrhs) {
       unsigned long long b = BSOLVE_EMPTY;
-      const long long limit = g_bsolve_wait;
-      for (long long it = 0; it < limit; ++it) {
+      for (int it = 0; it < (MODE == BRIEF ? BSOLVE_WAIT_SHORT : BSOLVE_WAIT); ++it) {
         b = ld_relaxed_u64(OUT + col + kb + row);
         if (b != BSOLVE_EMPTY) break;
         if (it > 64) {
-          if ((it & 255) == 0 && *(volatile const int*)err) break;
+          if ((it & 255) == 0 && *(volatile const int*)err != -1) break;
           __nanosleep(32);
         }
       }
       if (b == BSOLVE_EMPTY) {
         s_abort = 1;
         atomicExch(err, 1);
-        *(volatile int*)timed_out = 1;
       }
       v = __longlong_as_double((long long)b);
     }
     __syncthreads();  // the previous tile has been used
-    if (s_abort) return;
+    if (s_abort) {
+      *(volatile int*)timed_out = 1;
+      return;
+    }
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
       const int i = tid & 63, c = (tid >> 6) + 4 * u;
@@ -1453,11 +1457,7 @@ static int batch_factor(BatchPlan* p, cudaStream_t s) {
   return MPDOK_OK;
 }
 
-int batch_debug_wait(long long limit) {
-  const long long v = limit > 0 ? limit : BSOLVE_WAIT;
-  MPDOK_CUDA_TRY(cudaMemcpyToSymbol(g_bsolve_wait, &v, sizeof(v)));
-  return MPDOK_OK;
-}
+void batch_debug_wait(bool brief) { g_short_wait = brief; }
 
 // A solve does not synchronise, so a wait that ran out in one is reported by the
 // first later call on the plan that finds it (its blocks left X all NaN).
@@ -1469,27 +1469,40 @@ int batch_timed_out(void* plan) {
   return MPDOK_ERR_TIMEOUT;
 }
 
-// V := A^{-1} V in place (V in the caller's packing) through R (as long); tk: two
-// tickets and the word that ends the waits of a solve once one of them ran out,
-// which the caller clears.
-static int batch_solve_inplace(BatchPlan* p, double* V, double* R, int* tk, cudaStream_t s) {
+// V := A^{-1} V in place (V in the caller's packing) through R (as long).  The words
+// behind R: two tickets and one that ends the solve's waits once one of them ran
+// out.  They start at -1, the bytes that mark R empty too, so one fill prepares all,
+// and systems of one block need none (ten systems of 64, one column, two
+// refinements: 114 us with the fills, 81 without; two launches per level 84).
+constexpr int SOLVE_WORDS = 4;
+static int batch_solve_inplace(BatchPlan* p, double* V, double* R, cudaStream_t s) {
   const size_t bytes = (size_t)p->total_x * sizeof(double);
+  int* tk = (int*)(R + p->total_x);
   const int groups = (p->nrhs + BSOLVE_RHS - 1) / BSOLVE_RHS;
   const unsigned grid = (unsigned)(p->preLvl.back() * groups);
   if (grid == 0) return MPDOK_OK;
-  MPDOK_TRY(set_smem(k_bsolve_chain<false>, BSOLVE_SMEM));
-  MPDOK_TRY(set_smem(k_bsolve_chain<true>, BSOLVE_SMEM));
-  MPDOK_CUDA_TRY(cudaMemsetAsync(tk, 0, 2 * sizeof(int), s));
-  if (const int t0 = debug_first_ticket()) {
+  auto pass = [&](auto* kern, const double* in, double* out, int* ticket) -> int {
+    MPDOK_TRY(set_smem(kern, BSOLVE_SMEM));
+    launch(kern, dim3(grid), BT, BSOLVE_SMEM, s, (const BSys*)p->d_sys, preLvl_dev(p), p->maxblk, p->nrhs,
+           (const double*)p->A, (const double*)p->Linv, in, out, ticket, tk + 2, p->timed_out);
+    return MPDOK_OK;
+  };
+  if (p->maxblk == 1) {  // nothing waits, nothing to prepare
+    MPDOK_TRY(pass(k_bsolve_chain<false, ALONE>, V, V, nullptr));
+    MPDOK_TRY(pass(k_bsolve_chain<true, ALONE>, V, V, nullptr));
+    MPDOK_LAUNCH_CHECK("batch solve");
+    return MPDOK_OK;
+  }
+  MPDOK_CUDA_TRY(cudaMemsetAsync(R, 0xff, bytes + 3 * sizeof(int), s));
+  if (const int t1 = debug_first_ticket()) {
+    const int t0 = t1 - 1;
     MPDOK_CUDA_TRY(cudaMemcpyAsync(tk, &t0, sizeof(int), cudaMemcpyHostToDevice, s));
     MPDOK_CUDA_TRY(cudaStreamSynchronize(s));
   }
-  MPDOK_CUDA_TRY(cudaMemsetAsync(R, 0xff, bytes, s));
-  launch(k_bsolve_chain<false>, dim3(grid), BT, BSOLVE_SMEM, s, (const BSys*)p->d_sys, preLvl_dev(p), p->maxblk,
-         p->nrhs, (const double*)p->A, (const double*)p->Linv, (const double*)V, R, tk, tk + 2, p->timed_out);
+  const bool brief = g_short_wait;
+  MPDOK_TRY(pass(brief ? k_bsolve_chain<false, BRIEF> : k_bsolve_chain<false, CHAIN>, V, R, tk));
   MPDOK_CUDA_TRY(cudaMemsetAsync(V, 0xff, bytes, s));
-  launch(k_bsolve_chain<true>, dim3(grid), BT, BSOLVE_SMEM, s, (const BSys*)p->d_sys, preLvl_dev(p), p->maxblk,
-         p->nrhs, (const double*)p->A, (const double*)p->Linv, (const double*)R, V, tk + 1, tk + 2, p->timed_out);
+  MPDOK_TRY(pass(brief ? k_bsolve_chain<true, BRIEF> : k_bsolve_chain<true, CHAIN>, R, V, tk + 1));
   MPDOK_LAUNCH_CHECK("batch solve");
   return MPDOK_OK;
 }
@@ -1503,15 +1516,14 @@ static int batch_residual(BatchPlan* p, const double* B, const double* X, double
   return MPDOK_OK;
 }
 
-static int batch_solve_with(BatchPlan* p, const double* B, double* X, int refine, double* R, int* tk, cudaStream_t s) {
+static int batch_solve_with(BatchPlan* p, const double* B, double* X, int refine, double* R, cudaStream_t s) {
   const long long nx = p->total_x;
-  MPDOK_CUDA_TRY(cudaMemsetAsync(tk + 2, 0, sizeof(int), s));
   MPDOK_CUDA_TRY(cudaMemcpyAsync(X, B, (size_t)nx * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  MPDOK_TRY(batch_solve_inplace(p, X, R, tk, s));
+  MPDOK_TRY(batch_solve_inplace(p, X, R, s));
   const unsigned g = (unsigned)std::min<long long>((nx + 255) / 256, (long long)num_sms() * 8);
   for (int it = 0; it < refine; ++it) {
     MPDOK_TRY(batch_residual(p, B, X, p->V, s));
-    MPDOK_TRY(batch_solve_inplace(p, p->V, R, tk, s));
+    MPDOK_TRY(batch_solve_inplace(p, p->V, R, s));
     launch(k_badd, dim3(g), 256, 0, s, X, (const double*)p->V, nx);
   }
   MPDOK_LAUNCH_CHECK("batch refine");
@@ -1519,7 +1531,7 @@ static int batch_solve_with(BatchPlan* p, const double* B, double* X, int refine
 }
 
 // A caller may have several solves of one plan in flight on several streams.  They
-// share S and the tickets (V too, with refinement): each starts after the one
+// share S (V too, with refinement): each starts after the one
 // before it.  A solve that is being captured by the caller
 // may be replayed at any time and takes its own scratch into the graph.
 static int batch_solve(BatchPlan* p, const double* B, double* X, int refine, cudaStream_t s) {
@@ -1527,29 +1539,27 @@ static int batch_solve(BatchPlan* p, const double* B, double* X, int refine, cud
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   MPDOK_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
   if (cap != cudaStreamCaptureStatusNone) {
-    const size_t vec = align_up((size_t)p->total_x * sizeof(double), 256);
     void* own = nullptr;
-    MPDOK_CUDA_TRY(cudaMallocAsync(&own, vec + 256, s));
-    const int st = batch_solve_with(p, B, X, refine, (double*)own, (int*)((char*)own + vec), s);
+    MPDOK_CUDA_TRY(cudaMallocAsync(&own, (size_t)p->total_x * sizeof(double) + SOLVE_WORDS * sizeof(int), s));
+    const int st = batch_solve_with(p, B, X, refine, (double*)own, s);
     MPDOK_CUDA_TRY(cudaFreeAsync(own, s));
     return st;
   }
   std::lock_guard<std::mutex> lk(p->solve_mu);
   MPDOK_CUDA_TRY(cudaStreamWaitEvent(s, p->solved, 0));
-  const int st = batch_solve_with(p, B, X, refine, p->S, p->d_ticket, s);
+  const int st = batch_solve_with(p, B, X, refine, p->S, s);
   MPDOK_CUDA_TRY(cudaEventRecord(p->solved, s));
   return st;
 }
 
-// V := A^{-1} V for the Cholesky-preconditioned CG-IR; R as long as V and tk (3
-// ints, tk[2] cleared by the caller) are the solve's own, since several of them
-// may share a plan.
-int batch_apply_f64(void* plan, long long n, int K, double* V, double* R, int* tk, cudaStream_t s) {
-  MPDOK_ARG_CHECK(plan && V && R && tk, "null pointer");
+// V := A^{-1} V for the Cholesky-preconditioned CG-IR, whose scratch R is its own,
+// since several of them may share a plan.
+int batch_apply_f64(void* plan, long long n, int K, double* V, double* R, cudaStream_t s) {
+  MPDOK_ARG_CHECK(plan && V && R, "null pointer");
   BatchPlan* p = (BatchPlan*)plan;
   MPDOK_ARG_CHECK(p->nsys == 1 && p->sys[0].n == n, "the preconditioner plan must hold one system of size n");
   MPDOK_ARG_CHECK(p->nrhs == K, "the preconditioner plan's nrhs must equal the solve's nrhs");
-  return batch_solve_inplace(p, V, R, tk, s);
+  return batch_solve_inplace(p, V, R, s);
 }
 
 static void dag_release(BatchPlan* p) {
@@ -1703,7 +1713,6 @@ static void plan_free(BatchPlan* p) {
   if (p->d_sys) cudaFree(p->d_sys);
   if (p->d_pre) cudaFree(p->d_pre);
   if (p->d_pert) cudaFree(p->d_pert);
-  if (p->d_ticket) cudaFree(p->d_ticket);
   if (p->timed_out) cudaFreeHost(p->timed_out);
   if (p->solved) cudaEventDestroy(p->solved);
   delete p;
@@ -1809,18 +1818,15 @@ extern "C" int mpdok_batch_create(int nsys, const long long* n, int dim, int nrh
   if (e != cudaSuccess) return fail(e, "cudaMalloc (batch systems)");
   e = cudaMalloc(&p->d_pert, sizeof(int));
   if (e != cudaSuccess) return fail(e, "cudaMalloc (batch counter)");
-  e = cudaMalloc(&p->d_ticket, 4 * sizeof(int));
-  if (e != cudaSuccess) return fail(e, "cudaMalloc (batch tickets)");
-  e = cudaMemset(p->d_ticket, 0, 4 * sizeof(int));
-  if (e != cudaSuccess) return fail(e, "cudaMemset (batch tickets)");
   e = cudaHostAlloc((void**)&p->timed_out, sizeof(int), cudaHostAllocPortable);
   if (e != cudaSuccess) return fail(e, "cudaHostAlloc (batch status)");
   *p->timed_out = 0;
   e = cudaEventCreateWithFlags(&p->solved, cudaEventDisableTiming);
   if (e != cudaSuccess) return fail(e, "cudaEventCreate (batch)");
   const size_t nA = align_up((size_t)aA, 32), nL = align_up((size_t)aL, 32), nV = align_up((size_t)ax, 32),
+               nS = align_up((size_t)ax + SOLVE_WORDS, 32),
                nR = align_up((size_t)aR, 32), nCo = align_up((size_t)ac, 32);
-  p->bytes = (nA + nL + 3 * nV + nR + nCo) * sizeof(double);
+  p->bytes = (nA + nL + 2 * nV + nS + nR + nCo) * sizeof(double);
   e = cudaMalloc(&p->arena, p->bytes);
   if (e != cudaSuccess) return fail(e, "cudaMalloc (batch arena)");
   p->A = p->arena;
@@ -1828,7 +1834,7 @@ extern "C" int mpdok_batch_create(int nsys, const long long* n, int dim, int nrh
   p->V = p->Linv + nL;
   p->R = p->V + nV;
   p->S = p->R + nV;
-  p->rows = p->S + nV;
+  p->rows = p->S + nS;
   p->coords = p->rows + nR;
   e = cudaMemset(p->Linv, 0, nL * sizeof(double));
   if (e != cudaSuccess) return fail(e, "cudaMemset (batch)");
@@ -1987,7 +1993,7 @@ extern "C" int mpdok_batch_graph_build(void* plan, const double* B, double* X, i
     st = batch_step_dag(p, B, X, refine, p->cap);
   } else {
     st = batch_factor(p, p->cap);
-    if (st == MPDOK_OK && p->total_x > 0) st = batch_solve_with(p, B, X, refine, p->S, p->d_ticket, p->cap);
+    if (st == MPDOK_OK && p->total_x > 0) st = batch_solve_with(p, B, X, refine, p->S, p->cap);
   }
   cudaGraph_t g = nullptr;
   cudaError_t e = cudaStreamEndCapture(p->cap, &g);

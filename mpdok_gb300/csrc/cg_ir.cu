@@ -194,7 +194,6 @@ __global__ void k_ccopy_out(const double* __restrict__ src, double* __restrict__
 
 struct CholPcgWs {
   double *B, *X, *R, *E, *r, *z, *p, *q, *zero, *parts, *coef, *dots;
-  int* tk;  // of the preconditioner's solves
   int nb;
   size_t total;
 };
@@ -215,8 +214,8 @@ static CholPcgWs chol_layout(long long n, int K, void* base) {
   auto take = [&](size_t b) { size_t o = off; off = align_up(off + b, 256); return o; };
   const size_t vec = (size_t)std::max(1LL, n) * K * sizeof(double);
   const size_t oB = take(vec), oX = take(vec), oR = take(vec), oE = take(vec), or_ = take(vec), oz = take(vec),
-               op = take(vec), oq = take(vec), o0 = take(vec), oparts = take((size_t)K * w.nb * sizeof(double)),
-               ocoef = take(8 * sizeof(double)), odots = take(8 * sizeof(double) + 4 * sizeof(int));
+               op = take(vec), oq = take(vec + 4 * sizeof(int)), o0 = take(vec), oparts = take((size_t)K * w.nb * sizeof(double)),
+               ocoef = take(8 * sizeof(double)), odots = take(8 * sizeof(double));
   w.total = off;
   if (base) {
     char* b = (char*)base;
@@ -224,7 +223,6 @@ static CholPcgWs chol_layout(long long n, int K, void* base) {
     w.r = (double*)(b + or_); w.z = (double*)(b + oz); w.p = (double*)(b + op); w.q = (double*)(b + oq);
     w.zero = (double*)(b + o0); w.parts = (double*)(b + oparts); w.coef = (double*)(b + ocoef);
     w.dots = (double*)(b + odots);
-    w.tk = (int*)(w.dots + 8);
   }
   return w;
 }
@@ -258,7 +256,6 @@ static int chol_pcg_ir_body(void* plan, const Residual64& R, const Residual64& A
                             int inner_maxiter, const CholPcgWs& w, mpdok_solve_info* info, cudaStream_t s) {
   const unsigned g = (unsigned)std::max(1LL, std::min<long long>((n * K + 255) / 256, (long long)num_sms() * 8));
   launch(k_ccopy_in, g, 256, 0, s, B, ldb, w.B, n, K);
-  MPDOK_CUDA_TRY(cudaMemsetAsync(w.tk, 0, 4 * sizeof(int), s));
   MPDOK_CUDA_TRY(cudaMemsetAsync(w.X, 0, sizeof(double) * n * K, s));
   MPDOK_CUDA_TRY(cudaMemsetAsync(w.zero, 0, sizeof(double) * n * K, s));
   std::vector<double> bn(K), rn(K), rz(K), rz1(K), pq(K), cf(K);
@@ -288,7 +285,7 @@ static int chol_pcg_ir_body(void* plan, const Residual64& R, const Residual64& A
     MPDOK_CUDA_TRY(cudaMemsetAsync(w.E, 0, sizeof(double) * n * K, s));
     MPDOK_CUDA_TRY(cudaMemcpyAsync(w.r, w.R, sizeof(double) * n * K, cudaMemcpyDeviceToDevice, s));
     MPDOK_CUDA_TRY(cudaMemcpyAsync(w.z, w.r, sizeof(double) * n * K, cudaMemcpyDeviceToDevice, s));
-    MPDOK_TRY(batch_apply_f64(plan, n, K, w.z, w.q, w.tk, s));
+    MPDOK_TRY(batch_apply_f64(plan, n, K, w.z, w.q, s));
     MPDOK_CUDA_TRY(cudaMemcpyAsync(w.p, w.z, sizeof(double) * n * K, cudaMemcpyDeviceToDevice, s));
     MPDOK_TRY(cdots(w, w.r, w.z, n, K, rz.data(), s));
     std::vector<double> r0(rn);
@@ -311,7 +308,7 @@ static int chol_pcg_ir_body(void* plan, const Residual64& R, const Residual64& A
       }
       if (!any) break;
       MPDOK_CUDA_TRY(cudaMemcpyAsync(w.z, w.r, sizeof(double) * n * K, cudaMemcpyDeviceToDevice, s));
-      MPDOK_TRY(batch_apply_f64(plan, n, K, w.z, w.q, w.tk, s));
+      MPDOK_TRY(batch_apply_f64(plan, n, K, w.z, w.q, s));
       MPDOK_TRY(cdots(w, w.r, w.z, n, K, rz1.data(), s));
       for (int c = 0; c < K; ++c) {
         cf[c] = (live[c] && rz[c] != 0.0) ? rz1[c] / rz[c] : 0.0;
@@ -336,22 +333,15 @@ static int chol_pcg_ir_body(void* plan, const Residual64& R, const Residual64& A
   return MPDOK_OK;
 }
 
-// (a wait that ran out shows as NaN in the body; the plan may be another solve's
-// too, so the word of this one says whose it was)
+// (a wait of the preconditioner that ran out shows as NaN in the body)
 static int chol_pcg_ir_core(void* plan, const Residual64& R, const Residual64& Ain, long long n, int K,
                             const double* B, long long ldb, double* Xout, long long ldx, double tol, int maxiter_outer,
                             double inner_tol, int inner_maxiter, const CholPcgWs& w, mpdok_solve_info* info,
                             cudaStream_t s) {
   const int st = chol_pcg_ir_body(plan, R, Ain, n, K, B, ldb, Xout, ldx, tol, maxiter_outer, inner_tol, inner_maxiter, w,
                                   info, s);
-  if (st != MPDOK_ERR_NONFINITE) return st;
-  int ran_out = 0;
-  MPDOK_CUDA_TRY(cudaMemcpyAsync(&ran_out, w.tk + 2, sizeof(int), cudaMemcpyDeviceToHost, s));
-  MPDOK_CUDA_TRY(cudaStreamSynchronize(s));
-  if (!ran_out) return st;
-  batch_timed_out(plan);  // (reported here)
-  set_error("Cholesky preconditioner: a block's wait on its predecessor ran out");
-  return MPDOK_ERR_TIMEOUT;
+  if (st == MPDOK_ERR_NONFINITE) MPDOK_TRY(batch_timed_out(plan));
+  return st;
 }
 
 }  // namespace mpdok

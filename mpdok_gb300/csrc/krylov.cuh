@@ -105,17 +105,16 @@ struct Precond {
 };
 
 // V := A^-1 V in FP64 with the Cholesky factor of a batch plan of one system
-// (V: n x K column-major, ld n, K = the plan's nrhs), through R (as long as V) and
-// tk (two tickets; tk[2] is set when a wait ran out, and the caller clears it).
-// Defined in batch.cu.
-int batch_apply_f64(void* plan, long long n, int K, double* V, double* R, int* tk, cudaStream_t s);
+// (V: n x K column-major, ld n, K = the plan's nrhs), through R: as long as V and
+// 16 bytes.  Defined in batch.cu.
+int batch_apply_f64(void* plan, long long n, int K, double* V, double* R, cudaStream_t s);
 
 // MPDOK_ERR_TIMEOUT, once, when a wait of a finished solve of the plan ran out.
 int batch_timed_out(void* plan);
 
-// Test hooks (mpdok_debug_set): the batch solves' wait limit (<= 0: the default)
-// and the first ticket of every triangular solve (0: normal).
-int batch_debug_wait(long long limit);
+// Test hooks (mpdok_debug_set): short waits in the batch solves, and the first
+// ticket of every triangular solve (0: normal).
+void batch_debug_wait(bool brief);
 int debug_first_ticket();
 
 // One Arnoldi cycle (up to m steps) on the FP32 operator A32 with the

@@ -2767,7 +2767,8 @@ extern "C" int mpdok_debug_set(int key, long long value) {
     case MPDOK_DEBUG_WAIT_LIMIT: {
       const long long v = value > 0 ? value : SPIN_LIMIT;
       MPDOK_CUDA_TRY(cudaMemcpyToSymbol(g_spin_limit, &v, sizeof(v)));
-      return batch_debug_wait(value);
+      batch_debug_wait(v < SPIN_LIMIT);
+      return MPDOK_OK;
     }
     case MPDOK_DEBUG_TRSV_FIRST_TICKET:
       MPDOK_ARG_CHECK(value >= 0 && value < (1LL << 30), "first ticket out of range");
