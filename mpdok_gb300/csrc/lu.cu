@@ -2787,7 +2787,8 @@ extern "C" size_t mpdok_lu_factor_size(long long n, int fdtype) {
 
 extern "C" size_t mpdok_lu_work_size(long long n, int fdtype) {
   if (n < 0) return 0;
-  return lu_work_layout(n, fdtype).total;
+  // (FP32: room to align a work buffer that is not, see mpdok_lu_factor_copy)
+  return lu_work_layout(n, fdtype).total + (fdtype == MPDOK_F32 ? 16 : 0);
 }
 
 extern "C" size_t mpdok_lu_apply_work_size(long long n) {
@@ -2828,6 +2829,13 @@ extern "C" int mpdok_lu_factor_copy(const double* A, long long lda, long long n,
   MPDOK_ARG_CHECK(A && factors && work, "null pointer");
   MPDOK_ARG_CHECK(lda >= n, "lda < n");
   MPDOK_ARG_CHECK(factor_bytes >= lu_layout(n, fdtype).total, "factor buffer too small");
+  // the trailing update reads its operands and W in 16-byte units (TMA); FP32
+  // factors with pivoting take any work buffer of aligned doubles
+  if (fdtype == MPDOK_F32 && !aligned16(work)) {
+    const size_t pad = 16 - (reinterpret_cast<uintptr_t>(work) & 15u);
+    work = (char*)work + pad;
+    work_bytes -= std::min(work_bytes, pad);
+  }
   MPDOK_ARG_CHECK(work_bytes >= lu_work_layout(n, fdtype).total, "work buffer too small");
   MPDOK_ARG_CHECK(n < (1LL << 31), "n too large");
   MPDOK_ARG_CHECK(A32 == nullptr || lda32 >= n, "lda32 < n");
@@ -3158,7 +3166,8 @@ static int lu_ir_groups(const double* A, long long lda, long long n, const void*
     // with a column that the digits would lose more of than an FP64 product does
     // (residual64.cu) takes that product, from its first such step on.
     void* rw = wb + mw.off_q;
-    std::vector<char> digits(ng, residual64_pays(n, K));
+    // (they want an aligned workspace)
+    std::vector<char> digits(ng, residual64_pays(n, K) && aligned16(work));
     if (digits[0]) MPDOK_TRY(residual64_prepare(A, lda, n, rw, s));
     auto fp64_residual = [&](int q) -> int {
       const long long c = (long long)q * K;
