@@ -1535,7 +1535,7 @@ __device__ void piv_moves(const int* s_piv, long long jp, int nb, int* plan) {
 // Up to 16 CTAs (384 rows each, one thread to a row) hold the panel in shared
 // memory and meet at one hardware cluster barrier per column; candidates and
 // rows travel through distributed shared memory.  Panels of up to 6144 rows
-// take it: a column costs about 1.6 us against 4.7 us behind a grid barrier in
+// take it: a column costs about 1.7 us against 4.7 us behind a grid barrier in
 // global memory (n = 5000: 8.8 against 24.2 ms for the 40 panels, 220 against
 // 604 us each).  Of its 3700 cycles the barrier takes 1500 (800 with four CTAs),
 // the rows' copies 430, the argmax 370, the elimination 560, the columns right

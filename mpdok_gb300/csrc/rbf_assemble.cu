@@ -133,7 +133,7 @@ rbf_assemble_kernel(const double* __restrict__ R, long long nr,
 // memory, its mirror image (x_i - x_j and x_j - x_i have the same squares, so
 // both triangles hold the bits of the full evaluation).  A symmetric matrix
 // reads the same in row- and column-major order.  Bound by the FP64 pipe: 2 D
-// operations per pair (D = 3, n = 20000: 1.9 ms on that pipe, 0.47 ms for the
+// operations per pair (D = 3, n = 20000: 2.1 ms on that pipe, 0.47 ms for the
 // 3.2 GB of writes).  Measured there: 2.83 ms, against 17.24 ms with CUDA's exp
 // over all pairs; the general kernel below takes 5.16 ms.  Multiquadric: 5.98
 // against 11.62 ms.

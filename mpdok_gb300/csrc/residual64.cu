@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(1024) k_row_weights(const int* __restrict__ E,
 
 // W[j] = (S_j, P_j) of the rule above with w_i = 2^-E_i, then with w_i = 1 (in units
 // of the matrix's largest exponent).  A warp to a column: one more read of A
-// (n = 8192: 0.1 ms a solve).
+// (n = 8192: 0.12 ms a solve).
 __global__ void __launch_bounds__(256)
 k_column_weights(const double* __restrict__ A, long long lda, long long n, const int* __restrict__ E,
                  const float* __restrict__ rel, float4* __restrict__ W) {
@@ -300,12 +300,12 @@ k_column_digits(const double* __restrict__ X, long long ldx, long long n, int nc
 }
 
 // One CTA: rows [128 bx, ..), columns [32 by, ..), K chunks [bz per, ..).  Warp 0
-// loads the digits of X (TMA), warps 2 .. 9 convert A (coalesced FP64 loads, 35
+// loads the digits of X (TMA), warps 2 .. 9 convert A (coalesced FP64 loads, 39
 // integer instructions per entry, 16-byte stores into the swizzled layout) and
 // drain, warp 1 issues the MMAs: per 16-deep step 36 of 128 x 32, bound by the
 // reads of A's digits from shared memory.  Two stages and two sets of
 // accumulators, so converting, multiplying and draining overlap.
-// n = 8192, 72 columns: 0.93 ms (FP64 pipe: nine passes of 0.89 ms).
+// n = 8192, 72 columns: 0.95 ms (FP64 pipe: nine passes of 0.89 ms).
 __global__ void __launch_bounds__(THREADS, 1)
 k_residual64(const double* __restrict__ A, long long lda, int n, const int* __restrict__ E,
              const __grid_constant__ CUtensorMap tmX, int nc, int nchunk, int per, long long* __restrict__ P, int* err) {
