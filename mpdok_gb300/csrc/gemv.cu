@@ -184,9 +184,9 @@ gemv_t_stage1(const TA* __restrict__ A, long long lda, long long m, long long n,
 // spread rather than walked (n = 8192, 76 splits: 5.7 us; 10.2 us with one
 // thread to an entry).  Up to four splits, a thread takes an entry: the same order,
 // and three threads of four would have nothing to add (FP64, m = 524288, one
-// split: 8.7 us in all, 16.8 spread).  The order of the sum is fixed.
+// split: 8.7 us in all, 16.8 spread; FEW).  The order of the sum is fixed.
 constexpr int FIN_ROWS = GEMV_THREADS / 4;
-template <typename ACC>
+template <typename ACC, bool FEW>
 __global__ void __launch_bounds__(GEMV_THREADS)
 gemv_finalize(const ACC* __restrict__ P, int S, int K, long long m, ACC alpha, ACC beta,
               const ACC* bsrc, long long ldb, ACC* y, long long ldy,
@@ -205,7 +205,7 @@ gemv_finalize(const ACC* __restrict__ P, int S, int K, long long m, ACC alpha, A
     y[i + k * ldy] = v;
     sq += (double)v * (double)v;
   };
-  if (S <= 4) {
+  if constexpr (FEW) {
     for (long long idx = (long long)blockIdx.x * GEMV_THREADS + threadIdx.x; idx < total;
          idx += (long long)gridDim.x * GEMV_THREADS) {
       ACC sum = ACC(0);
@@ -213,7 +213,7 @@ gemv_finalize(const ACC* __restrict__ P, int S, int K, long long m, ACC alpha, A
       put(idx, sum);
     }
   }
-  for (long long b0 = S <= 4 ? total : (long long)blockIdx.x * FIN_ROWS; b0 < total; b0 += (long long)gridDim.x * FIN_ROWS) {
+  for (long long b0 = (long long)blockIdx.x * FIN_ROWS; !FEW && b0 < total; b0 += (long long)gridDim.x * FIN_ROWS) {
     const long long idx = b0 + r;
     ACC sum = ACC(0);
     if (idx < total) {
@@ -465,14 +465,13 @@ int gemv_launch(int a_dtype, bool trans, const void* A, long long lda, long long
     }
     if (nrm2 && zero_ticket) MPDOK_CUDA_TRY(cudaMemsetAsync(ticket, 0, sizeof(unsigned), s));
     const unsigned fb = finalize_blocks(out * K);
+    const bool few = p.S <= 4;
     if (a_dtype == MPDOK_F64)
-      launch(gemv_finalize<double>, fb, GEMV_THREADS, 0, s, (const double*)P, p.S, K, out, alpha, beta,
-                                                       (const double*)Bk, ldb, (double*)Yk, ldy, fin_parts,
-                                                       ticket, nrm2, skip);
+      launch(few ? gemv_finalize<double, true> : gemv_finalize<double, false>, fb, GEMV_THREADS, 0, s, (const double*)P,
+             p.S, K, out, alpha, beta, (const double*)Bk, ldb, (double*)Yk, ldy, fin_parts, ticket, nrm2, skip);
     else
-      launch(gemv_finalize<float>, fb, GEMV_THREADS, 0, s, (const float*)P, p.S, K, out, (float)alpha, (float)beta,
-                                                      (const float*)Bk, ldb, (float*)Yk, ldy, fin_parts, ticket,
-                                                      nrm2, skip);
+      launch(few ? gemv_finalize<float, true> : gemv_finalize<float, false>, fb, GEMV_THREADS, 0, s, (const float*)P,
+             p.S, K, out, (float)alpha, (float)beta, (const float*)Bk, ldb, (float*)Yk, ldy, fin_parts, ticket, nrm2, skip);
     MPDOK_LAUNCH_CHECK("gemv finalize");
     done += K;
   }
